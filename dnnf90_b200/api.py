@@ -198,8 +198,8 @@ def profile_enable(on: bool = True):
 
 
 # names of the Bell kernel variants by id (the forward's, the adjoint's)
-FWD_VARIANTS = {0: "v5-global", 1: "v5-shared", 2: "v8", 3: "tiled"}
-ADJ_VARIANTS = {0: "v5-global", 1: "v5-shared", 2: "v7", 3: "tiled"}
+FWD_VARIANTS = {0: "v5-global", 1: "v5-shared", 2: "v8", 3: "tiled", 4: "column"}
+ADJ_VARIANTS = {0: "v5-global", 1: "v5-shared", 2: "v7", 3: "tiled", 4: "column"}
 
 
 def tune_report() -> list:

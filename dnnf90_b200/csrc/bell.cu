@@ -59,6 +59,7 @@ void DevBellPlan::release() {
   for (void *p : ps)
     if (p) cudaFree(p);
   tile.release();
+  col.release();
   *this = DevBellPlan();
 }
 
@@ -184,6 +185,7 @@ int upload_bell_plan(const TableSet &t, DevBellPlan &d) {
   d.nrows = P.nrows;
   d.dt_off = P.dt_off;
   if ((rc = upload_tile_plan(t, d.tile))) return rc;
+  if ((rc = upload_col(t, d.col))) return rc;
   d.ready = true;
   return RC_OK;
 }
@@ -1483,6 +1485,13 @@ int tune_force(int which, int variant) {
   return RC_OK;
 }
 
+// the column kernels (bell_col.cu) run wherever they apply unless another
+// variant is pinned
+static bool use_col(int which) {
+  const int f = g_force[which];
+  return f < 0 || f >= 4;
+}
+
 template <typename L>
 static int tuned_launch(const TuneKey &key, int nvar, int dflt, long items, cudaStream_t st,
                         L launch) {
@@ -1685,6 +1694,8 @@ static int fwd2_k(const DevBellPlan &bp, const DevTables &t, int n, int npts, co
 int bell_fwd2(const DevBellPlan &bp, const DevTables &t, int n, int npts, const void *S,
               void *T, void *h, bool train, int prec, cudaStream_t st) {
   if (!bp.ready) return RC_UNSUPPORTED;
+  if (use_col(0) && !(t.iact == 0 && bp.f9.ok && g_series_fwd) && col_applies(bp.col, n, npts, prec))
+    return bell_fwd_col(bp.col, t, n, npts, S, T, h, train, prec, st);
   return prec == PREC_F64 ? fwd2_k<double>(bp, t, n, npts, S, T, h, train, st)
                           : fwd2_k<float>(bp, t, n, npts, S, T, h, train, st);
 }
@@ -1777,6 +1788,8 @@ int bell_adj2(const DevBellPlan &bp, const DevTables &t, int n, int npts, const 
               const void *h, void *Sb, double *gbias, int gstride, int prec,
               cudaStream_t st) {
   if (!bp.ready) return RC_UNSUPPORTED;
+  if (use_col(1) && col_applies(bp.col, n, npts, prec))
+    return bell_adj_col(bp.col, t, n, npts, Tb, h, Sb, gbias, gstride, prec, st);
   return prec == PREC_F64 ? adj2_t<double>(bp, t, n, npts, Tb, h, Sb, gbias, gstride, st)
                           : adj2_t<float>(bp, t, n, npts, Tb, h, Sb, gbias, gstride, st);
 }
@@ -1785,19 +1798,11 @@ int bell_adj2(const DevBellPlan &bp, const DevTables &t, int n, int npts, const 
 struct AdjL2sArgs {
   int n, na, npts, gy;
   const int *up;           // [na][D0]: slot of g + e_i | (g_i + 1) << 16, or -1
-  const void *Tb, *h;      // [P][na][n] (h unused when h is formed in the kernel)
+  const void *Tb, *h;      // [P][na][n]
   const double *X;         // [P][D0]
   double *g;               // dW_2 [n][D0 + 1], accumulated (null in row mode)
   double *rows;            // [P][nw] (row mode)
   size_t nw, woff;
-  // h formed in the kernel (graded slots): the layer's weights [n][D0 + 1],
-  // s^(q)(S^0) [P][k + 2][n] kept by the forward, the order, the first slot
-  // of each degree and a - e_i | i << 16 per slot (k_layer2v's monomials)
-  const double *W;
-  const void *sig;
-  const int *par;
-  int k;
-  int ds[KMAX + 2];
 };
 
 // The first hidden layer's Bell adjoint fused with dW_2 (the k_adj_l2v sums)
@@ -1819,16 +1824,13 @@ struct AdjL2sArgs {
 // steps its multiplier at each degree boundary.  (Summing each degree with
 // W^g and multiplying by s^(p+1) once was measured slower: the degree runs
 // are short, 1 to 4 slots per warp.)
-template <typename R, int D0, int NPB, bool AN>
+template <typename R, int D0, int NPB>
 __global__ void __launch_bounds__(1024) k_adj_l2s(AdjL2sArgs a) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   unsigned char *sm = smem_raw;
   const int na = a.na, n = a.n;
-  // one buffer: Tb rows, then h rows (AN: the k + 2 rows of s^(q))
-  const uint32_t bsz = (AN ? (uint32_t)(na + KMAX + 2) : 2u * na) * 128;
-  // AN: the tile's monomials [na] rows, the degree starts
-  const uint32_t moff = 2 * bsz, dsoff = moff + (AN ? (uint32_t)na * 128 : 0u);
-  const uint32_t upoff = dsoff + (AN ? 128u : 0u);
+  // one buffer: Tb rows, then h rows
+  const uint32_t bsz = 2u * na * 128, upoff = 2 * bsz;
   const uint32_t redoff = upoff + ((uint32_t)na * D0 * 8 + 127) / 128 * 128;
   // (byte offset of the Tb row of g + e_i, multiplier g_i + 1) per (g, i);
   // a missing child reads row 0 with multiplier 0
@@ -1850,39 +1852,10 @@ __global__ void __launch_bounds__(1024) k_adj_l2s(AdjL2sArgs a) {
     const size_t pofs = (size_t)(it % a.npts) * plane;
     const int j0 = (int)(it / a.npts) * NPB;
     stage_rows<NPB, R>(sm + dst, (const R *)a.Tb + pofs, na, n, j0, 1024);
-    if (AN)
-      stage_rows<NPB, R>(sm + dst + na * 128,
-                         (const R *)a.sig + (size_t)(it % a.npts) * (a.k + 2) * n, a.k + 2, n,
-                         j0, 1024);
-    else
-      stage_rows<NPB, R>(sm + dst + na * 128, (const R *)a.h + pofs, na, n, j0, 1024);
+    stage_rows<NPB, R>(sm + dst + na * 128, (const R *)a.h + pofs, na, n, j0, 1024);
   };
   if (it0 < it1) stage(it0, 0);
   cp_async_commit();
-  // AN: the monomials W^g of tile tl's neurons (every thread; barriers inside)
-  const int *sds = (const int *)(sm + dsoff);
-  auto build_m = [&](int tl) {
-    const int j = tl * NPB + ln;
-    const double *wr = a.W + (size_t)(j < n ? j : n - 1) * (D0 + 1);
-    if (warp == 0 && lact) srow<R>(sm, moff + lo) = (R)1;
-    __syncthreads();
-    for (int p = 1; p <= a.k; ++p) {
-      for (int ia = sds[p] + warp; ia < sds[p + 1]; ia += 32) {
-        const int pk = __ldg(a.par + ia);
-        if (lact)
-          srow<R>(sm, moff + ia * 128 + lo) =
-              (R)((double)srow<R>(sm, moff + (pk & 0xffff) * 128 + lo) * wr[1 + (pk >> 16)]);
-      }
-      __syncthreads();
-    }
-  };
-  int mtile = -1;
-  if (AN && it0 < it1) {
-    if (threadIdx.x < KMAX + 2) ((int *)(sm + dsoff))[threadIdx.x] = a.ds[threadIdx.x];
-    __syncthreads();
-    mtile = (int)(it0 / a.npts);
-    build_m(mtile);
-  }
   double acc[D0 + 1];
 #pragma unroll
   for (int o = 0; o <= D0; ++o) acc[o] = 0.0;
@@ -1910,42 +1883,17 @@ __global__ void __launch_bounds__(1024) k_adj_l2s(AdjL2sArgs a) {
       flush(tile);
       tile = tl;
     }
-    if (AN && tl != mtile) {  // block-uniform: every warp is past the last item
-      build_m(tl);
-      mtile = tl;
-    }
     const uint32_t tb = buf + lo, hb = tb + na * 128;
     R s[D0 + 1];
 #pragma unroll
     for (int o = 0; o <= D0; ++o) s[o] = (R)0;
-    if (AN) {
-      // h^g = (R)s^(p+1) * W^g, p = |g|: the slots of a warp rise in degree,
-      // so its multiplier steps at each degree boundary
-      int p = 0, pend = sds[1];
-      R dq = srow<R>(sm, hb + 128);  // this item's s^(1) row
-      for (int g = warp; g < na; g += 32) {
-        while (g >= pend) {
-          ++p;
-          pend = sds[p + 1];
-          dq = srow<R>(sm, hb + (p + 1) * 128);
-        }
-        const R hg = dq * srow<R>(sm, moff + g * 128 + lo);
-        s[0] += srow<R>(sm, tb + g * 128) * hg;
+    for (int g = warp; g < na; g += 32) {
+      const R hg = srow<R>(sm, hb + g * 128);
+      s[0] += srow<R>(sm, tb + g * 128) * hg;
 #pragma unroll
-        for (int i = 0; i < D0; ++i) {
-          const uint2 u = up[g * D0 + i];
-          s[1 + i] += (R)__uint_as_float(u.y) * srow<R>(sm, tb + u.x) * hg;
-        }
-      }
-    } else {
-      for (int g = warp; g < na; g += 32) {
-        const R hg = srow<R>(sm, hb + g * 128);
-        s[0] += srow<R>(sm, tb + g * 128) * hg;
-#pragma unroll
-        for (int i = 0; i < D0; ++i) {
-          const uint2 u = up[g * D0 + i];
-          s[1 + i] += (R)__uint_as_float(u.y) * srow<R>(sm, tb + u.x) * hg;
-        }
+      for (int i = 0; i < D0; ++i) {
+        const uint2 u = up[g * D0 + i];
+        s[1 + i] += (R)__uint_as_float(u.y) * srow<R>(sm, tb + u.x) * hg;
       }
     }
     const double *x = a.X + (size_t)pt * D0;
@@ -1978,30 +1926,21 @@ __global__ void __launch_bounds__(1024) k_adj_l2s(AdjL2sArgs a) {
   if (it0 < it1) flush(tile);
 }
 
-// shared memory of k_adj_l2s: two item buffers (Tb rows, then h rows, or
-// with h formed in the kernel the item's s^(q) rows), then (an) the
-// monomials and the degree starts, the (g, i) table and the per-warp row sums
-static size_t l2s_smem(int na, int d0, bool an) {
-  return (an ? (size_t)2 * (na + KMAX + 2) * 128 + (size_t)na * 128 + 128
-             : (size_t)4 * na * 128) +
-         ((size_t)na * d0 * 8 + 127) / 128 * 128 + (size_t)32 * (d0 + 1) * 128;
-}
-
-bool bell_adj_l2s_analytic(int d0, int na, int n, int prec) {
-  const int rsz = prec == PREC_F64 ? 8 : 4;
-  return d0 >= 1 && d0 <= 8 && na <= 65535 && n % (16 / rsz) == 0 &&
-         l2s_smem(na, d0, true) <= 227 * 1024;
+// shared memory of k_adj_l2s: two item buffers (Tb rows, then h rows), the
+// (g, i) table and the per-warp row sums
+static size_t l2s_smem(int na, int d0) {
+  return (size_t)4 * na * 128 + ((size_t)na * d0 * 8 + 127) / 128 * 128 +
+         (size_t)32 * (d0 + 1) * 128;
 }
 
 template <typename R, int D0>
 static int adj_l2s_k(const AdjL2sArgs &a, cudaStream_t st) {
   constexpr int NPB = sizeof(R) == 8 ? 16 : 32;
-  const bool an = a.W != nullptr;
-  const size_t smem = l2s_smem(a.na, D0, an);
+  const size_t smem = l2s_smem(a.na, D0);
   if (smem > 227 * 1024 || a.na > 65535 || a.n % (16 / (int)sizeof(R))) return RC_UNSUPPORTED;
   AdjL2sArgs b = a;
   b.gy = (a.n + NPB - 1) / NPB;
-  auto k = an ? k_adj_l2s<R, D0, NPB, true> : k_adj_l2s<R, D0, NPB, false>;
+  auto k = k_adj_l2s<R, D0, NPB>;
   CKB(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   const int grid = persistent_grid((const void *)k, 1024, smem, (long)a.npts * b.gy);
   LAUNCH("k_bell_adj_l2", st, k<<<grid, 1024, smem, st>>>(b));
@@ -2026,18 +1965,11 @@ static int adj_l2s_t(int d0, const AdjL2sArgs &a, cudaStream_t st) {
 
 int bell_adj_l2s(int d0, int n, int na, int npts, const int *up, const void *Tb, const void *h,
                  const double *X, double *g, double *rows, size_t nw, size_t woff, int prec,
-                 cudaStream_t st, const L2Analytic *an) {
+                 cudaStream_t st) {
   if (npts <= 0) return RC_OK;
   AdjL2sArgs a;
   a.n = n; a.na = na; a.npts = npts; a.gy = 0; a.up = up; a.Tb = Tb; a.h = h; a.X = X;
   a.g = g; a.rows = rows; a.nw = nw; a.woff = woff;
-  a.W = nullptr; a.sig = nullptr; a.par = nullptr; a.k = 0;
-  for (int p = 0; p < KMAX + 2; ++p) a.ds[p] = na;
-  if (an) {
-    if (an->k < 1 || an->k > KMAX) return RC_UNSUPPORTED;
-    a.W = an->W; a.sig = an->sig; a.par = an->par; a.k = an->k;
-    for (int p = 0; p <= an->k + 1; ++p) a.ds[p] = an->dstart[p];
-  }
   return prec == PREC_F64 ? adj_l2s_t<double>(d0, a, st) : adj_l2s_t<float>(d0, a, st);
 }
 

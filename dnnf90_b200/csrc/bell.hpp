@@ -4,6 +4,7 @@
 
 #include <string>
 
+#include "bell_col.hpp"
 #include "bell_plan.hpp"
 
 namespace dnnf90 {
@@ -83,6 +84,7 @@ struct DevBellPlan {
     bool ok = false;
   } f9;
   TileDev tile;            // register-tiled kernels (dense sets, FP32)
+  ColDev col;              // column kernels (small sets)
   double *sc64 = nullptr;  // [3][na]: a!, 1/a!, 1/a! (Tb, h, Sb scales)
   float *sc32 = nullptr;
   void release();
@@ -115,8 +117,8 @@ int bell_fwd_tile(const TileDev &d, const DevTables &t, int n, int npts, const v
 int bell_adj_tile(const TileDev &d, int n, int npts, const void *Tb, const void *h, void *Sb,
                   double *gbias, int gstride, cudaStream_t st);
 // The first hidden layer is analytic: h^g = s^(|g|+1)(S^0) W^g.  With these
-// inputs the adjoint forms h itself (graded slots) from the s^(q) the
-// forward kept, and reads no h plane.
+// inputs the adjoint (bell_adj_l2a) forms h itself (graded slots) from the
+// s^(q) the forward kept, and reads no h plane.
 struct L2Analytic {
   const double *W;         // the layer's weights [n][d0 + 1]
   const void *sig;         // [P][k + 2][n]: s^(q)(S^0), kept by the forward
@@ -124,13 +126,10 @@ struct L2Analytic {
   int k;
   const int *dstart;       // host [k + 2]: first slot of each degree
 };
-// whether the adjoint can form h itself for these sizes (its shared memory)
-bool bell_adj_l2s_analytic(int d0, int na, int n, int prec);
-// the first hidden layer's adjoint fused with dW_2, staged through shared
-// memory (RC_UNSUPPORTED when an item's rows do not fit); an: h formed in
-// the kernel (null: read from the h plane)
+// the first hidden layer's adjoint fused with dW_2 from the h plane, staged
+// through shared memory (RC_UNSUPPORTED when an item's rows do not fit)
 int bell_adj_l2s(int d0, int n, int na, int npts, const int *up, const void *Tb, const void *h,
                  const double *X, double *g, double *rows, size_t nw, size_t woff, int prec,
-                 cudaStream_t st, const L2Analytic *an = nullptr);
+                 cudaStream_t st);
 
 }  // namespace dnnf90

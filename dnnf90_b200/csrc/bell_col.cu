@@ -1,0 +1,609 @@
+// bell_col.cu - Bell kernels with one thread per (point, neuron).
+//
+// Column kernels (small carried sets).  A set of a few tens of slots has too
+// little work per neuron to share between warps: the block-per-point kernels
+// of bell.cu spend such items in barriers (one per degree) and idle warps.
+// Here every thread owns one neuron of one point and keeps its slots in its
+// own column of shared memory ([slot][thread], so that a warp's access is
+// one conflict-free row); no thread reads another's column, so the items
+// need no barrier at all.  The pair lists are warp-uniform broadcasts.
+// Forward: the Horner form of the Bell sum over factorial-normalised series
+// (see tile_plan.hpp), with D and E side by side and updated in place: an
+// output only reads slots of lower degree, so the slots are taken in
+// descending order of degree.
+//
+// First-layer adjoint (every graded set).  The first hidden layer is
+// analytic, h^g = s^(|g|+1)(S^0) W^g, so its adjoint needs the Tb plane once
+// and per neuron tile a table of monomials.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <map>
+#include <string>
+
+#include "bell.hpp"
+#include "bell_col.hpp"
+#include "engine.hpp"
+#include "kernels.cuh"
+
+namespace dnnf90 {
+
+#define CKC(x)                                                        \
+  do {                                                                \
+    cudaError_t e_ = (x);                                             \
+    if (e_ != cudaSuccess) {                                          \
+      set_error(std::string("bell_col: ") + cudaGetErrorString(e_));  \
+      return e_ == cudaErrorMemoryAllocation ? RC_NOMEM : RC_DEVICE;  \
+    }                                                                 \
+  } while (0)
+
+// ------------------------------------------------------------ the program
+ColProg build_col_prog(const TableSet &t) {
+  ColProg P;
+  const int na = t.na, d0 = t.d0;
+  for (int a = 0; a < na; ++a) P.kt = std::max(P.kt, t.deg[a]);
+  std::map<std::vector<int>, int> at;
+  std::vector<std::vector<int>> al(na);
+  for (int a = 0; a < na; ++a) {
+    al[a].assign(t.alpha.begin() + (size_t)a * d0, t.alpha.begin() + (size_t)(a + 1) * d0);
+    at[al[a]] = a;
+  }
+  std::vector<std::vector<uint32_t>> f(na), adj(na);
+  std::vector<int> g(d0);
+  for (int a = 0; a < na; ++a)
+    for (int b = 0; b < na; ++b) {
+      bool le = true;
+      for (int i = 0; i < d0; ++i) {
+        g[i] = al[a][i] - al[b][i];
+        if (g[i] < 0) le = false;
+      }
+      if (!le) continue;
+      const int ig = at.at(g);  // the set is downward closed
+      if (b != 0) f[a].push_back((uint32_t)b | ((uint32_t)ig << 16));
+      adj[b].push_back((uint32_t)a | ((uint32_t)ig << 16));
+    }
+  auto flat = [&](const std::vector<std::vector<uint32_t>> &v, std::vector<int> &hdr,
+                  std::vector<uint32_t> &rec) {
+    for (int a = 0; a < na; ++a) {
+      if (rec.size() & 1) rec.push_back(0);
+      hdr.push_back((int)rec.size());
+      hdr.push_back((int)v[a].size());
+      rec.insert(rec.end(), v[a].begin(), v[a].end());
+    }
+    if (rec.size() & 1) rec.push_back(0);
+  };
+  flat(f, P.fhdr, P.frec);
+  flat(adj, P.ahdr, P.arec);
+  P.dstart.assign(P.kt + 2, na);
+  for (int a = na - 1; a >= 0; --a) P.dstart[t.deg[a]] = a;
+  for (int p = P.kt; p >= 0; --p) P.dstart[p] = std::min(P.dstart[p], P.dstart[p + 1]);
+  return P;
+}
+
+namespace {
+
+constexpr int NT = 64;        // threads per block of the column kernels
+
+template <typename R> struct Vec2;
+template <> struct Vec2<float> { typedef float2 T; };
+template <> struct Vec2<double> { typedef double2 T; };
+
+struct ColArgs {
+  int n, na, npts, k, kt, iact, nrec, gstride;
+  const int *hdr;
+  const uint32_t *rec;
+  const int *dstart;
+  const double *sc;        // [3][na]: a!, 1/a!, 1/a!
+  const double *tpc;
+  const void *A, *B;       // forward: S; adjoint: Tb, h
+  void *C, *D;             // forward: T, h; adjoint: Sb
+  double *gbias;
+};
+
+size_t col_tables(int na, int nrec, size_t rsz) {
+  return (size_t)na * 8 + (size_t)nrec * 4 + (KMAX + 3) * 4 + 2 * (size_t)na * rsz + 64;
+}
+// columns: s~ and the (D, E) pairs (forward) or Tb and h (adjoint), the
+// s^(q) rows
+size_t col_fwd_smem(int na, int kt, int nrec, size_t rsz) {
+  return (size_t)(3 * na + kt + 2) * NT * rsz + col_tables(na, nrec, rsz);
+}
+size_t col_adj_smem(int na, int nrec, size_t rsz) {
+  return (size_t)2 * na * NT * rsz + col_tables(na, nrec, rsz);
+}
+
+// shared copies of the tables; the pointers are set by the caller's layout
+template <typename R>
+struct ColTab {
+  int2 *hdr;
+  uint32_t *rec;
+  R *fact, *ifact;
+  int *ds;
+  __device__ void load(unsigned char *p, const ColArgs &a) {
+    // records first: they are read as 8-byte pairs
+    rec = (uint32_t *)p;
+    hdr = (int2 *)(rec + (a.nrec + 1) / 2 * 2);
+    fact = (R *)(hdr + a.na);
+    ifact = fact + a.na;
+    ds = (int *)(ifact + a.na);
+    for (int i = threadIdx.x; i < a.nrec; i += NT) rec[i] = __ldg(a.rec + i);
+    for (int i = threadIdx.x; i < a.na; i += NT) {
+      hdr[i] = make_int2(__ldg(a.hdr + 2 * i), __ldg(a.hdr + 2 * i + 1));
+      fact[i] = (R)__ldg(a.sc + i);
+      ifact[i] = (R)__ldg(a.sc + a.na + i);
+    }
+    for (int i = threadIdx.x; i < a.kt + 2; i += NT) ds[i] = __ldg(a.dstart + i);
+  }
+};
+
+__device__ __forceinline__ float2 madd2(float s, float2 d, float2 acc) {
+  return __ffma2_rn(make_float2(s, s), d, acc);
+}
+__device__ __forceinline__ double2 madd2(double s, double2 d, double2 acc) {
+  return make_double2(fma(s, d.x, acc.x), fma(s, d.y, acc.y));
+}
+
+// Bound: the loads and stores of the planes while the set is small (5 slots,
+// 16384 points x 64 in FP64: 1020 us in the block-per-point kernels, 53 here,
+// 126 MB at 2.4 TB/s), the shared-memory loads of the pairs beyond about 15
+// slots.  NT = 64: small blocks, so that as many columns as fit are resident.
+template <typename R, bool TRAIN>
+__global__ void __launch_bounds__(NT) k_bell_fwd_col(ColArgs a) {
+  typedef typename Vec2<R>::T R2;
+  extern __shared__ __align__(16) unsigned char smc[];
+  const int n = a.n, na = a.na, kt = a.kt;
+  R2 *de = (R2 *)smc + threadIdx.x;                       // [na]
+  R *s = (R *)((R2 *)smc + (size_t)na * NT) + threadIdx.x;  // [na]
+  R *sig = s + (size_t)na * NT;                           // [kt + 2]
+  ColTab<R> t;
+  t.load((unsigned char *)((R *)((R2 *)smc + (size_t)na * NT) + (size_t)(na + kt + 2) * NT), a);
+  __syncthreads();
+  const long total = (long)a.npts * n, stride = (long)gridDim.x * NT;
+  const size_t plane = (size_t)na * n;
+  for (long e = (long)blockIdx.x * NT + threadIdx.x; e < total; e += stride) {
+    const long pt = e / n;
+    const size_t base = (size_t)pt * plane + (size_t)(e - pt * n);
+    const R *S = (const R *)a.A + base;
+    R s0 = S[0];
+#pragma unroll 4
+    for (int i = 1; i < na; ++i) s[i * NT] = S[(size_t)i * n] * t.ifact[i];
+    if (a.iact == 0) {
+      const double th = tanh((double)s0);
+      const int ld = a.k + 3;
+      for (int q = 0; q <= kt + 1; ++q) {
+        double v = __ldg(a.tpc + q * ld + q + 1);
+        for (int i = q; i >= 0; --i) v = v * th + __ldg(a.tpc + q * ld + i);
+        sig[q * NT] = (R)v;
+      }
+    } else {
+      double d[KMAX + 2];
+      sigma_derivs(a.iact, a.tpc, a.k, (double)s0, d);
+      for (int q = 0; q <= kt + 1; ++q) sig[q * NT] = (R)d[q];
+    }
+    R *T = (R *)a.C + base, *H = (R *)a.D + base;
+    R2 top;
+    top.x = sig[kt * NT];
+    top.y = sig[(kt + 1) * NT];
+    de[0] = top;
+    for (int q = kt - 1; q >= 0; --q) {
+      const R inv = (R)1 / (R)(q + 1);
+      for (int i = t.ds[kt - q + 1] - 1; i >= 1; --i) {
+        const int2 h = t.hdr[i];
+        R2 acc, bcc;
+        acc.x = acc.y = bcc.x = bcc.y = (R)0;
+        const uint32_t *r = t.rec + h.x;
+        int c = 0;
+        for (; c + 1 < h.y; c += 2) {
+          const uint2 u = *(const uint2 *)(r + c);
+          acc = madd2(s[(u.x & 0xffffu) * NT], de[(u.x >> 16) * NT], acc);
+          bcc = madd2(s[(u.y & 0xffffu) * NT], de[(u.y >> 16) * NT], bcc);
+        }
+        if (c < h.y) {
+          const uint32_t u = r[c];
+          acc = madd2(s[(u & 0xffffu) * NT], de[(u >> 16) * NT], acc);
+        }
+        acc.x = (acc.x + bcc.x) * inv;
+        acc.y = (acc.y + bcc.y) * inv;
+        if (q > 0) {
+          de[i * NT] = acc;
+        } else {
+          T[(size_t)i * n] = t.fact[i] * acc.x;
+          if (TRAIN) H[(size_t)i * n] = t.fact[i] * acc.y;
+        }
+      }
+      if (q > 0) {
+        R2 o;
+        o.x = sig[q * NT];
+        o.y = sig[(q + 1) * NT];
+        de[0] = o;
+      }
+    }
+    T[0] = sig[0];
+    if (TRAIN) H[0] = sig[NT];
+  }
+}
+
+// Sb_b b! = sum_g (a! Tb_a)(h_g / g!), a = b + g.  The threads stride over
+// the (point, neuron) pairs by a multiple of n, so a thread's neuron is
+// fixed and its share of the bias gradient stays in a register.  (5 slots,
+// 16384 points x 64 in FP64: 550 us before, 40 here.)
+template <typename R>
+__global__ void __launch_bounds__(NT) k_bell_adj_col(ColArgs a) {
+  extern __shared__ __align__(16) unsigned char smc[];
+  __shared__ double red[NT];
+  const int n = a.n, na = a.na;
+  R *tb = (R *)smc + threadIdx.x, *hh = tb + (size_t)na * NT;
+  ColTab<R> t;
+  t.load((unsigned char *)((R *)smc + (size_t)2 * na * NT), a);
+  __syncthreads();
+  const long total = (long)a.npts * n;
+  const long stride = (long)gridDim.x * NT / n * n;
+  const size_t plane = (size_t)na * n;
+  const long e0 = (long)blockIdx.x * NT + threadIdx.x;
+  double gb = 0.0;
+  for (long e = e0 < stride ? e0 : total; e < total; e += stride) {
+    const long pt = e / n;
+    const size_t base = (size_t)pt * plane + (size_t)(e - pt * n);
+    const R *Tb = (const R *)a.A + base, *H = (const R *)a.B + base;
+#pragma unroll 4
+    for (int i = 0; i < na; ++i) {
+      tb[i * NT] = Tb[(size_t)i * n] * t.fact[i];
+      hh[i * NT] = H[(size_t)i * n] * t.ifact[i];
+    }
+    R *Sb = (R *)a.C + base;
+    for (int i = na - 1; i >= 0; --i) {
+      const int2 h = t.hdr[i];
+      const uint32_t *r = t.rec + h.x;
+      R acc = (R)0, bcc = (R)0;
+      int c = 0;
+      for (; c + 1 < h.y; c += 2) {
+        const uint2 u = *(const uint2 *)(r + c);
+        acc = fma(tb[(u.x & 0xffffu) * NT], hh[(u.x >> 16) * NT], acc);
+        bcc = fma(tb[(u.y & 0xffffu) * NT], hh[(u.y >> 16) * NT], bcc);
+      }
+      if (c < h.y) {
+        const uint32_t u = r[c];
+        acc = fma(tb[(u & 0xffffu) * NT], hh[(u >> 16) * NT], acc);
+      }
+      const R v = (acc + bcc) * t.ifact[i];
+      Sb[(size_t)i * n] = v;
+      if (i == 0) gb += (double)v;
+    }
+  }
+  if (!a.gbias) return;
+  red[threadIdx.x] = gb;
+  __syncthreads();
+  // threads n apart share a neuron
+  if (threadIdx.x < n) {
+    double v = 0.0;
+    for (int i = threadIdx.x; i < NT; i += n) v += red[i];
+    if (v != 0.0) atomicAdd(a.gbias + (size_t)(e0 % n) * a.gstride, v);
+  }
+}
+
+int resident_grid(const void *k, int threads, size_t smem) {
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess ||
+      per_sm < 1)
+    per_sm = 1;
+  return grid_sms() * per_sm;
+}
+
+// ------------------------------------------------------------ first layer
+struct L2aArgs {
+  int n, na, npts, k, nt, ppw, zsplit;
+  const int *up;           // [na][D0]: slot of g + e_i | (g_i + 1) << 16, or -1
+  const int *par;          // [na]: slot of a - e_i | i << 16, i the first nonzero dimension
+  const double *sc;        // [3][na]: a!, 1/a!, 1/a!
+  const void *Tb, *sig;    // [P][na][n], [P][k + 2][n]
+  const double *X, *W;     // [P][D0], [n][D0 + 1]
+  double *g, *rows;
+  size_t nw, woff;
+  int ds[KMAX + 2];
+};
+
+constexpr int L2T = 256;   // threads per block
+
+// Sb^0 = sum_a Tb^a h^a and Sb^{e_i} = sum_a a_i Tb^a h^{a - e_i} with
+// h^g = s^(|g|+1) W^g.  With M_a = W^a / a! and x_a = a! Tb^a both read
+// x_a M_a and x_a M_{a - e_i}, and s depends on the degree alone, so each
+// degree is summed first:
+//   Sb^0 = sum_p s^(p+1) sum_{|a| = p} x_a M_a,
+//   Sb^{e_i} = sum_p s^(p) sum_{|a| = p} x_a M_{a - e_i}.
+// One lane per neuron of a tile (lanes beyond a narrow layer's neurons take
+// further points) and PT points at a time per thread: the tile's M rows sit
+// in shared memory and one read of a row serves PT points, so the kernel
+// streams Tb (65536 points x 128 at K = 7, D0 = 4 in FP32: 11 GB in 2.76 ms,
+// 4.0 TB/s; the kernel that staged every item through shared memory and
+// summed it over 32 warps took 6.44).  Gradient mode keeps FP64 sums over a
+// thread's points and may split the slots over blockIdx.z (dW_2 is linear
+// in each slot's share) when there are few points; row mode writes each
+// point's sums.
+template <typename R, int D0, int PT>
+__global__ void __launch_bounds__(L2T) k_adj_l2a(L2aArgs a) {
+  extern __shared__ __align__(16) unsigned char sm2[];
+  const int na = a.na, n = a.n, nt = a.nt;
+  R *M = (R *)sm2;                              // [na + 1][nt], row na zero
+  R *fact = M + (size_t)(na + 1) * nt;          // [na]
+  int *off = (int *)(fact + (na + (na & 1)));   // [na][D0]: word offset of row a - e_i
+  const int j0 = blockIdx.y * nt;
+  for (int e = threadIdx.x; e < na * D0; e += L2T) off[e] = na * nt;
+  for (int e = threadIdx.x; e < na; e += L2T) fact[e] = (R)__ldg(a.sc + e);
+  for (int e = threadIdx.x; e < nt; e += L2T) {
+    M[e] = (R)1;
+    M[(size_t)na * nt + e] = (R)0;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < na * D0; e += L2T) {
+    const int g = e / D0, i = e - g * D0, u = __ldg(a.up + e);
+    if (u >= 0) off[(u & 0xffff) * D0 + i] = g * nt;
+  }
+  for (int p = 1; p <= a.k; ++p) {
+    const int r0 = a.ds[p], nr = a.ds[p + 1] - r0;
+    for (int e = threadIdx.x; e < nr * nt; e += L2T) {
+      const int r = r0 + e / nt, jl = e % nt, j = min(j0 + jl, n - 1);
+      const int pk = __ldg(a.par + r), ps = pk & 0xffff, i = pk >> 16;
+      // the exponent of dimension i: a! over (a - e_i)!
+      const double f = __ldg(a.sc + ps) * __ldg(a.sc + na + r);
+      M[(size_t)r * nt + jl] =
+          (R)((double)M[(size_t)ps * nt + jl] * (__ldg(a.W + (size_t)j * (D0 + 1) + 1 + i) * f));
+    }
+    __syncthreads();
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int jl = lane % nt, sub = lane / nt, j = j0 + jl;
+  const bool act = sub < a.ppw && j < n;
+  const R *Ml = M + jl;
+  // the slots of this block
+  const int a0 = (int)((long)na * blockIdx.z / a.zsplit);
+  const int a1 = (int)((long)na * (blockIdx.z + 1) / a.zsplit);
+  double acc[D0 + 1];
+#pragma unroll
+  for (int o = 0; o <= D0; ++o) acc[o] = 0.0;
+  const long nwarp = (long)gridDim.x * (L2T / 32);
+  const int step = a.ppw;
+  for (long w = (long)blockIdx.x * (L2T / 32) + warp; w * step * PT < a.npts; w += nwarp) {
+    if (!act) continue;
+    long pt[PT];
+    const R *Tb[PT], *sg[PT];
+    R s[PT][D0 + 1];
+#pragma unroll
+    for (int k = 0; k < PT; ++k) {
+      pt[k] = (w * PT + k) * step + sub;
+      const long q = pt[k] < a.npts ? pt[k] : (long)a.npts - 1;  // read twice, dropped below
+      Tb[k] = (const R *)a.Tb + (size_t)q * na * n + j;
+      sg[k] = (const R *)a.sig + (size_t)q * (a.k + 2) * n + j;
+#pragma unroll
+      for (int o = 0; o <= D0; ++o) s[k][o] = (R)0;
+    }
+    for (int p = 0; p <= a.k; ++p) {
+      const int r0 = max(a.ds[p], a0), r1 = min(a.ds[p + 1], a1);
+      if (r0 >= r1) continue;
+      R b[PT][D0 + 1];
+#pragma unroll
+      for (int k = 0; k < PT; ++k)
+#pragma unroll
+        for (int o = 0; o <= D0; ++o) b[k][o] = (R)0;
+#pragma unroll 4
+      for (int r = r0; r < r1; ++r) {
+        R x[PT];
+#pragma unroll
+        for (int k = 0; k < PT; ++k) x[k] = __ldcs(Tb[k] + (size_t)r * n);
+        const R f = fact[r], m0 = Ml[r * nt];
+#pragma unroll
+        for (int k = 0; k < PT; ++k) {
+          x[k] *= f;
+          b[k][0] = fma(x[k], m0, b[k][0]);
+        }
+#pragma unroll
+        for (int i = 0; i < D0; ++i) {
+          const R m = Ml[off[r * D0 + i]];
+#pragma unroll
+          for (int k = 0; k < PT; ++k) b[k][1 + i] = fma(x[k], m, b[k][1 + i]);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < PT; ++k) {
+        const R s1 = sg[k][(size_t)(p + 1) * n], sp = sg[k][(size_t)p * n];
+        s[k][0] = fma(s1, b[k][0], s[k][0]);
+#pragma unroll
+        for (int i = 0; i < D0; ++i) s[k][1 + i] = fma(sp, b[k][1 + i], s[k][1 + i]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < PT; ++k) {
+      if (pt[k] >= a.npts) continue;
+      const double *x = a.X + (size_t)pt[k] * D0;
+      if (a.rows) {
+        double *row = a.rows + (size_t)pt[k] * a.nw + a.woff + (size_t)j * (D0 + 1);
+        row[0] = (double)s[k][0];
+#pragma unroll
+        for (int i = 0; i < D0; ++i) row[1 + i] = (double)s[k][0] * __ldg(x + i) + (double)s[k][1 + i];
+      } else {
+        acc[0] += (double)s[k][0];
+#pragma unroll
+        for (int i = 0; i < D0; ++i)
+          acc[1 + i] += (double)s[k][0] * __ldg(x + i) + (double)s[k][1 + i];
+      }
+    }
+  }
+  if (!a.g) return;
+  // the block's sums: warps, then the lanes that share a neuron, then one
+  // atomic per weight
+  __syncthreads();  // the monomials are done with
+  double *red = (double *)sm2;                  // [D0 + 1][L2T]
+#pragma unroll
+  for (int o = 0; o <= D0; ++o) red[o * L2T + threadIdx.x] = act ? acc[o] : 0.0;
+  __syncthreads();
+  for (int e = threadIdx.x; e < nt * (D0 + 1); e += L2T) {
+    const int o = e / nt, l = e - o * nt;
+    if (j0 + l >= n) continue;
+    double v = 0.0;
+    for (int w = 0; w < L2T / 32; ++w)
+      for (int u = 0; u < a.ppw; ++u) v += red[o * L2T + w * 32 + u * nt + l];
+    if (v != 0.0) atomicAdd(a.g + (size_t)(j0 + l) * (D0 + 1) + o, v);
+  }
+}
+
+// neurons of a tile: the layer cut into equal tiles of at most 32
+int l2a_tile(int n) { return (n + (n + 31) / 32 - 1) / ((n + 31) / 32); }
+
+size_t l2a_smem(int na, int nt, int d0, size_t rsz) {
+  const size_t tab = (size_t)(na + 1) * nt * rsz + (size_t)(na + 1) * rsz + (size_t)na * d0 * 4 + 16;
+  return std::max(tab, (size_t)(d0 + 1) * L2T * 8);
+}
+
+template <typename R, int D0>
+int l2a_k(L2aArgs a, cudaStream_t st) {
+  constexpr int PT = sizeof(R) == 8 ? 2 : 4;
+  const size_t smem = l2a_smem(a.na, a.nt, D0, sizeof(R));
+  const void *k = (const void *)k_adj_l2a<R, D0, PT>;
+  CKC(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int gy = (a.n + a.nt - 1) / a.nt;
+  const long per = (long)(L2T / 32) * a.ppw * PT;  // points per block and pass
+  const int full = resident_grid(k, L2T, smem);
+  const int gx = (int)std::max(1L, std::min((a.npts + per - 1) / per, (long)std::max(1, full / gy)));
+  // few points: the slots are split over blocks too, at least 8 to a block
+  // (300 points of 8 neurons, 330 slots: 113 us before, 19 here)
+  a.zsplit = a.rows ? 1 : std::max(1, std::min(a.na / 8, full / std::max(1, gx * gy)));
+  LAUNCH("k_bell_adj_l2", st, (k_adj_l2a<R, D0, PT><<<dim3(gx, gy, a.zsplit), L2T, smem, st>>>(a)));
+  CKC(cudaGetLastError());
+  return RC_OK;
+}
+
+template <typename R>
+int l2a_t(int d0, const L2aArgs &a, cudaStream_t st) {
+  switch (d0) {
+    case 1: return l2a_k<R, 1>(a, st);
+    case 2: return l2a_k<R, 2>(a, st);
+    case 3: return l2a_k<R, 3>(a, st);
+    case 4: return l2a_k<R, 4>(a, st);
+    case 5: return l2a_k<R, 5>(a, st);
+    case 6: return l2a_k<R, 6>(a, st);
+    case 7: return l2a_k<R, 7>(a, st);
+    case 8: return l2a_k<R, 8>(a, st);
+    default: return RC_UNSUPPORTED;
+  }
+}
+
+template <typename T>
+int put_col(T **d, const std::vector<T> &h) {
+  CKC(cudaMalloc(d, std::max<size_t>(1, h.size()) * sizeof(T)));
+  if (!h.empty()) CKC(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
+  return RC_OK;
+}
+
+template <typename R>
+int fwd_col_t(const ColDev &d, const ColArgs &a, bool train, cudaStream_t st) {
+  const size_t smem = col_fwd_smem(d.na, d.kt, d.nfrec, sizeof(R));
+  const void *k = train ? (const void *)k_bell_fwd_col<R, true> : (const void *)k_bell_fwd_col<R, false>;
+  CKC(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const long total = (long)a.npts * a.n;
+  const int grid = (int)std::max(1L, std::min((total + NT - 1) / NT, (long)resident_grid(k, NT, smem)));
+  if (train) { LAUNCH("k_bell_fwd", st, (k_bell_fwd_col<R, true><<<grid, NT, smem, st>>>(a))); }
+  else { LAUNCH("k_bell_fwd", st, (k_bell_fwd_col<R, false><<<grid, NT, smem, st>>>(a))); }
+  CKC(cudaGetLastError());
+  return RC_OK;
+}
+
+template <typename R>
+int adj_col_t(const ColDev &d, const ColArgs &a, cudaStream_t st) {
+  const size_t smem = col_adj_smem(d.na, d.narec, sizeof(R));
+  const void *k = (const void *)k_bell_adj_col<R>;
+  CKC(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  // at least one neuron row of threads, so that the stride is not zero
+  const long total = (long)a.npts * a.n;
+  long grid = std::max(1L, std::min((total + NT - 1) / NT, (long)resident_grid(k, NT, smem)));
+  grid = std::max(grid, (long)(a.n + NT - 1) / NT);
+  LAUNCH("k_bell_adj", st, (k_bell_adj_col<R><<<(int)grid, NT, smem, st>>>(a)));
+  CKC(cudaGetLastError());
+  return RC_OK;
+}
+
+}  // namespace
+
+// ------------------------------------------------------------ host side
+void ColDev::release() {
+  for (void *p : {(void *)fhdr, (void *)ahdr, (void *)frec, (void *)arec, (void *)dstart})
+    if (p) cudaFree(p);
+  *this = ColDev();
+}
+
+// The rule, by the forward and adjoint measured against the best of the
+// block-per-point kernels (us, 8192 points, layers of 64; FP64):
+//   |A|   10: 39 + 41 against 436 + 306     35: 352 + 284 against 660 + 482
+//         21: 200 + 123 against 904 + 404   56: 1145 + 704 against 1150 + 706
+// and in FP32 33 + 31 against 201 + 150 (10), 164 + 133 against 287 + 220
+// (35), 558 + 288 against 465 + 293 (56): the columns win while the state
+// leaves several warps per SM, up to 36 slots.  Below COL_THREADS neurons
+// there are too few threads to hide a long column's serial chain (2400
+// neurons: 11.5 against 12.8 us at 10 slots, 17 against 15 at 20, 44 against
+// 29 at 36), where only the shortest columns pay.
+constexpr int COL_MAX = 36, COL_SHORT = 16;
+constexpr long COL_THREADS = 8192;
+
+int upload_col(const TableSet &t, ColDev &d) {
+  d.release();
+  if (t.na > COL_MAX) return RC_OK;
+  const ColProg P = build_col_prog(t);
+  int rc;
+  if ((rc = put_col(&d.fhdr, P.fhdr)) || (rc = put_col(&d.ahdr, P.ahdr)) ||
+      (rc = put_col(&d.frec, P.frec)) || (rc = put_col(&d.arec, P.arec)) ||
+      (rc = put_col(&d.dstart, P.dstart))) {
+    d.release();
+    return rc;
+  }
+  d.na = t.na;
+  d.kt = P.kt;
+  d.nfrec = (int)P.frec.size();
+  d.narec = (int)P.arec.size();
+  d.ok = true;
+  return RC_OK;
+}
+
+bool col_applies(const ColDev &d, int n, int npts, int prec) {
+  const size_t rsz = prec == PREC_F64 ? 8 : 4;
+  return d.ok && n >= 1 && (d.na <= COL_SHORT || (long)npts * n >= COL_THREADS) &&
+         col_fwd_smem(d.na, d.kt, d.nfrec, rsz) <= 227 * 1024 &&
+         col_adj_smem(d.na, d.narec, rsz) <= 226 * 1024;
+}
+
+int bell_fwd_col(const ColDev &d, const DevTables &t, int n, int npts, const void *S, void *T,
+                 void *h, bool train, int prec, cudaStream_t st) {
+  ColArgs a{};
+  a.n = n; a.na = d.na; a.npts = npts; a.k = t.k; a.kt = d.kt; a.iact = t.iact;
+  a.nrec = d.nfrec; a.hdr = d.fhdr; a.rec = d.frec; a.dstart = d.dstart; a.sc = t.bp.sc64;
+  a.tpc = t.tpc; a.A = S; a.C = T; a.D = h;
+  return prec == PREC_F64 ? fwd_col_t<double>(d, a, train, st) : fwd_col_t<float>(d, a, train, st);
+}
+
+int bell_adj_col(const ColDev &d, const DevTables &t, int n, int npts, const void *Tb,
+                 const void *h, void *Sb, double *gbias, int gstride, int prec,
+                 cudaStream_t st) {
+  ColArgs a{};
+  a.n = n; a.na = d.na; a.npts = npts; a.k = t.k; a.kt = d.kt; a.iact = t.iact;
+  a.nrec = d.narec; a.hdr = d.ahdr; a.rec = d.arec; a.dstart = d.dstart; a.sc = t.bp.sc64;
+  a.A = Tb; a.B = h; a.C = Sb; a.gbias = gbias; a.gstride = gstride;
+  return prec == PREC_F64 ? adj_col_t<double>(d, a, st) : adj_col_t<float>(d, a, st);
+}
+
+bool l2a_applies(int d0, int na, int n, int prec) {
+  const size_t rsz = prec == PREC_F64 ? 8 : 4;
+  return d0 >= 1 && d0 <= 8 && n >= 1 && na <= 65535 &&
+         l2a_smem(na, l2a_tile(n), d0, rsz) <= 227 * 1024;
+}
+
+int bell_adj_l2a(const DevTables &t, int n, int npts, const void *Tb, const double *X, double *g,
+                 double *rows, size_t nw, size_t woff, int prec, const L2Analytic &an,
+                 cudaStream_t st) {
+  if (npts <= 0) return RC_OK;
+  L2aArgs a{};
+  a.n = n; a.na = t.na; a.npts = npts; a.k = t.k; a.nt = l2a_tile(n);
+  a.ppw = std::max(1, 32 / a.nt); a.zsplit = 1; a.up = t.l2up; a.par = an.par; a.sc = t.bp.sc64;
+  a.Tb = Tb; a.sig = an.sig; a.X = X; a.W = an.W; a.g = g; a.rows = rows; a.nw = nw;
+  a.woff = woff;
+  for (int p = 0; p < KMAX + 2; ++p) a.ds[p] = p <= an.k + 1 ? an.dstart[p] : t.na;
+  return prec == PREC_F64 ? l2a_t<double>(t.d0, a, st) : l2a_t<float>(t.d0, a, st);
+}
+
+}  // namespace dnnf90

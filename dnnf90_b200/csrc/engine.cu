@@ -1399,7 +1399,7 @@ template <typename R>
 static bool l2_analytic(const DevTables &t, int n) {
   return t.graded && t.k >= 1 && t.k <= 8 && (size_t)t.na * 32 * sizeof(R) <= 200 * 1024 &&
          (int)t.dstart.size() >= t.k + 2 &&
-         bell_adj_l2s_analytic(t.d0, t.na, n, sizeof(R) == 8 ? PREC_F64 : PREC_SPLIT);
+         l2a_applies(t.d0, t.na, n, sizeof(R) == 8 ? PREC_F64 : PREC_SPLIT);
 }
 
 // streaming first hidden layer; RC_UNSUPPORTED when the shape is outside it
@@ -1657,15 +1657,19 @@ static int adj_chunk(Chunk<R> &c, const double *X, const double *seed,
   a2.Tb = p.Tb; a2.h = p.h[1]; a2.X = X;
   a2.g = rows || !grad ? nullptr : grad + net.woff[1];
   a2.rows = rows; a2.nw = net.nw; a2.woff = net.woff[1];
-  L2Analytic an{c.W64(2), p.sig, t.l2par, t.k, t.dstart.data()};
-  rc = bell_adj_l2s(t.d0, a2.n, na, np, t.l2up, p.Tb, p.h[1], X, a2.g, rows, net.nw,
-                    net.woff[1], split ? PREC_SPLIT : PREC_F64, c.st,
-                    l2_analytic<R>(t, a2.n) ? &an : nullptr);
-  if (rc == RC_UNSUPPORTED && l2_analytic<R>(t, a2.n)) {
+  const int pr = split ? PREC_SPLIT : PREC_F64;
+  if (l2_analytic<R>(t, a2.n)) {
     // the forward wrote no h plane for this layer, so no other kernel may run
-    set_error("first-layer adjoint: the analytic kernel refused a shape it was chosen for");
-    return RC_DEVICE;
+    const L2Analytic an{c.W64(2), p.sig, t.l2par, t.k, t.dstart.data()};
+    rc = bell_adj_l2a(t, a2.n, np, p.Tb, X, a2.g, rows, net.nw, net.woff[1], pr, an, c.st);
+    if (rc == RC_UNSUPPORTED) {
+      set_error("first-layer adjoint: the analytic kernel refused a shape it was chosen for");
+      return RC_DEVICE;
+    }
+    return rc;
   }
+  rc = bell_adj_l2s(t.d0, a2.n, na, np, t.l2up, p.Tb, p.h[1], X, a2.g, rows, net.nw,
+                    net.woff[1], pr, c.st);
   if (rc != RC_UNSUPPORTED) return rc;
   {
     AdjL2vArgs v;
