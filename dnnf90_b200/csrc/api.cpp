@@ -24,6 +24,7 @@
 #include "../../include/dnnf90_b200.h"
 #include "engine.hpp"
 #include "gemm_tc.hpp"
+#include "scratch.hpp"
 
 using namespace dnnf90;
 
@@ -765,6 +766,7 @@ int dnnf90_net_free(int nid) {
   NetH &n = g_net[nid];
   n.dt.release();
   n.dn.release();
+  scratch_trim();  // the scratch kept for calls on it goes back too
   n = NetH();
   g_gen[nid]++;
   return RC_OK;
@@ -1169,21 +1171,19 @@ static int ngd_host(int nid, int nrow, const double *rows, const double *b, int 
   int rc = device_ready();
   if (rc) return rc;
   const int nw = (int)g_net[nid].w.size();
-  double *dr = nullptr, *db = nullptr, *du = nullptr;
-  if ((rc = ck(cudaMalloc(&dr, sizeof(double) * (size_t)nrow * nw), "cudaMalloc"))) return rc;
-  if ((rc = ck(cudaMalloc(&db, sizeof(double) * nw * 2), "cudaMalloc"))) {
-    cudaFree(dr);
+  DevScratch rs, vs;
+  if ((rc = ck(rs.take(sizeof(double) * (size_t)nrow * nw, nullptr), "scratch")) ||
+      (rc = ck(vs.take(sizeof(double) * nw * 2, nullptr), "scratch")))
     return rc;
-  }
-  du = db + nw;
-  rc = ck(cudaMemcpy(dr, rows, sizeof(double) * (size_t)nrow * nw, cudaMemcpyHostToDevice), "H2D");
-  if (!rc) rc = ck(cudaMemcpy(db, b, sizeof(double) * nw, cudaMemcpyHostToDevice), "H2D");
+  double *dr = rs.as<double>(), *db = vs.as<double>(), *du = db + nw;
+  rc = ck(cudaMemcpyAsync(dr, rows, sizeof(double) * (size_t)nrow * nw, cudaMemcpyHostToDevice,
+                          nullptr), "H2D");
+  if (!rc)
+    rc = ck(cudaMemcpyAsync(db, b, sizeof(double) * nw, cudaMemcpyHostToDevice, nullptr), "H2D");
   if (!rc)
     rc = dual ? ngd_device_dual(dr, nrow, nw, db, nb, mu, du, prec, nullptr)
               : ngd_device(dr, nrow, nw, db, nb, mu, du, prec, nullptr);
   if (!rc) rc = ck(cudaMemcpy(u, du, sizeof(double) * nw, cudaMemcpyDeviceToHost), "D2H");
-  cudaFree(dr);
-  cudaFree(db);
   return rc;
 }
 

@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "engine.hpp"
+#include "scratch.hpp"
 #include "gemm_f64.hpp"
 #include "gemm_tc.hpp"
 #include "kernels.cuh"
@@ -123,6 +124,44 @@ std::string profile_read() {
       return e_ == cudaErrorMemoryAllocation ? RC_NOMEM : RC_DEVICE;    \
     }                                                                   \
   } while (0)
+
+// ------------------------------------------------------------- scratch pool
+static cudaMemPool_t scratch_pool(bool create) {
+  static std::mutex mu;
+  static cudaMemPool_t pool[64] = {};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
+  std::lock_guard<std::mutex> lk(mu);
+  if (!pool[dev] && create) {
+    cudaMemPoolProps pr{};
+    pr.allocType = cudaMemAllocationTypePinned;
+    pr.location.type = cudaMemLocationTypeDevice;
+    pr.location.id = dev;
+    cudaMemPool_t p = nullptr;
+    unsigned long long keep = POOL_KEEP;
+    if (cudaMemPoolCreate(&p, &pr) != cudaSuccess) return nullptr;
+    cudaMemPoolSetAttribute(p, cudaMemPoolAttrReleaseThreshold, &keep);
+    pool[dev] = p;
+  }
+  return pool[dev];
+}
+cudaError_t DevScratch::take(size_t bytes, cudaStream_t st) {
+  release();
+  cudaMemPool_t pool = scratch_pool(true);
+  if (!pool) return cudaErrorMemoryAllocation;
+  st_ = st;
+  const cudaError_t e = cudaMallocFromPoolAsync(&p_, bytes, pool, st);
+  if (e != cudaSuccess) p_ = nullptr;
+  return e;
+}
+void DevScratch::release() {
+  if (p_) cudaFreeAsync(p_, st_);
+  p_ = nullptr;
+}
+void scratch_trim() {
+  cudaMemPool_t pool = scratch_pool(false);
+  if (pool) cudaMemPoolTrimTo(pool, 0);
+}
 
 int device_ready() {
   static int state = 0;  // 0 unknown, 1 ok, -1 none

@@ -1,0 +1,41 @@
+// scratch.hpp - device scratch of one call, from a stream-ordered pool.
+//
+// A call that needs device memory only while it runs takes it from one pool
+// per device, private to the library (cudaMallocAsync), instead of
+// cudaMalloc / cudaFree, which wait for the whole device and map fresh pages
+// on every call (0.75 ms for a 7 MB operand).  The pool is bounded: at each
+// synchronisation CUDA returns what it holds beyond POOL_KEEP bytes, and
+// scratch_trim (called when a network is freed) returns the rest.  The
+// allocations are ordered on the caller's stream, so calls of several
+// threads and streams share the pool safely.
+#pragma once
+#include <cuda_runtime.h>
+
+#include <cstddef>
+
+namespace dnnf90 {
+
+constexpr size_t POOL_KEEP = (size_t)512 << 20;
+
+// device memory for work enqueued on st, released (in stream order) when the
+// object goes out of scope; null after a failure
+class DevScratch {
+ public:
+  DevScratch() = default;
+  ~DevScratch() { release(); }
+  DevScratch(const DevScratch &) = delete;
+  DevScratch &operator=(const DevScratch &) = delete;
+  cudaError_t take(size_t bytes, cudaStream_t st);
+  void release();
+  template <typename T>
+  T *as() const { return (T *)p_; }
+
+ private:
+  void *p_ = nullptr;
+  cudaStream_t st_ = nullptr;
+};
+
+// returns what the current device's pool holds unused
+void scratch_trim();
+
+}  // namespace dnnf90
