@@ -10,7 +10,10 @@
 // Forward: the Horner form of the Bell sum over factorial-normalised series
 // (see tile_plan.hpp), with D and E side by side and updated in place: an
 // output only reads slots of lower degree, so the slots are taken in
-// descending order of degree.
+// descending order of degree.  Every sum is one chain that starts with the
+// pair (a, 0), and the adjoint's sums keep the chains of the block-per-point
+// kernels: up to K = 2 both then round exactly as those do (a natural-gradient step divides by a small damping what the
+// rounding of its rows leaves).
 //
 // First-layer adjoint (every graded set).  The first hidden layer is
 // analytic, h^g = s^(|g|+1)(S^0) W^g, so its adjoint needs the Tb plane once
@@ -59,7 +62,8 @@ ColProg build_col_prog(const TableSet &t) {
       }
       if (!le) continue;
       const int ig = at.at(g);  // the set is downward closed
-      if (b != 0) f[a].push_back((uint32_t)b | ((uint32_t)ig << 16));
+      if (b != 0 && b == a) f[a].insert(f[a].begin(), (uint32_t)b);
+      else if (b != 0) f[a].push_back((uint32_t)b | ((uint32_t)ig << 16));
       adj[b].push_back((uint32_t)a | ((uint32_t)ig << 16));
     }
   auto flat = [&](const std::vector<std::vector<uint32_t>> &v, std::vector<int> &hdr,
@@ -189,21 +193,21 @@ __global__ void __launch_bounds__(NT) k_bell_fwd_col(ColArgs a) {
       const R inv = (R)1 / (R)(q + 1);
       for (int i = t.ds[kt - q + 1] - 1; i >= 1; --i) {
         const int2 h = t.hdr[i];
-        R2 acc, bcc;
-        acc.x = acc.y = bcc.x = bcc.y = (R)0;
+        R2 acc;
+        acc.x = acc.y = (R)0;
         const uint32_t *r = t.rec + h.x;
         int c = 0;
         for (; c + 1 < h.y; c += 2) {
           const uint2 u = *(const uint2 *)(r + c);
           acc = madd2(s[(u.x & 0xffffu) * NT], de[(u.x >> 16) * NT], acc);
-          bcc = madd2(s[(u.y & 0xffffu) * NT], de[(u.y >> 16) * NT], bcc);
+          acc = madd2(s[(u.y & 0xffffu) * NT], de[(u.y >> 16) * NT], acc);
         }
         if (c < h.y) {
           const uint32_t u = r[c];
           acc = madd2(s[(u & 0xffffu) * NT], de[(u >> 16) * NT], acc);
         }
-        acc.x = (acc.x + bcc.x) * inv;
-        acc.y = (acc.y + bcc.y) * inv;
+        acc.x *= inv;
+        acc.y *= inv;
         if (q > 0) {
           de[i * NT] = acc;
         } else {
@@ -227,7 +231,7 @@ __global__ void __launch_bounds__(NT) k_bell_fwd_col(ColArgs a) {
 // the (point, neuron) pairs by a multiple of n, so a thread's neuron is
 // fixed and its share of the bias gradient stays in a register.  (5 slots,
 // 16384 points x 64 in FP64: 550 us before, 40 here.)
-template <typename R>
+template <typename R, int CHAINS>
 __global__ void __launch_bounds__(NT) k_bell_adj_col(ColArgs a) {
   extern __shared__ __align__(16) unsigned char smc[];
   __shared__ double red[NT];
@@ -259,13 +263,14 @@ __global__ void __launch_bounds__(NT) k_bell_adj_col(ColArgs a) {
       for (; c + 1 < h.y; c += 2) {
         const uint2 u = *(const uint2 *)(r + c);
         acc = fma(tb[(u.x & 0xffffu) * NT], hh[(u.x >> 16) * NT], acc);
-        bcc = fma(tb[(u.y & 0xffffu) * NT], hh[(u.y >> 16) * NT], bcc);
+        R &second = CHAINS == 2 ? bcc : acc;
+        second = fma(tb[(u.y & 0xffffu) * NT], hh[(u.y >> 16) * NT], second);
       }
       if (c < h.y) {
         const uint32_t u = r[c];
         acc = fma(tb[(u & 0xffffu) * NT], hh[(u >> 16) * NT], acc);
       }
-      const R v = (acc + bcc) * t.ifact[i];
+      const R v = (CHAINS == 2 ? acc + bcc : acc) * t.ifact[i];
       Sb[(size_t)i * n] = v;
       if (i == 0) gb += (double)v;
     }
@@ -303,6 +308,25 @@ struct L2aArgs {
 };
 
 constexpr int L2T = 256;   // threads per block
+
+// a block's dW_2 sums, one set acc per thread: over the warps, then over the
+// lanes that share a neuron, then one atomic per weight
+template <int D0, int NTHR>
+__device__ __forceinline__ void l2_reduce(const L2aArgs &a, double *red, const double (&acc)[D0 + 1],
+                                          bool act, int j0) {
+  __syncthreads();  // the tables are done with; red: [D0 + 1][NTHR]
+#pragma unroll
+  for (int o = 0; o <= D0; ++o) red[o * NTHR + threadIdx.x] = act ? acc[o] : 0.0;
+  __syncthreads();
+  for (int e = threadIdx.x; e < a.nt * (D0 + 1); e += NTHR) {
+    const int o = e / a.nt, l = e - o * a.nt;
+    if (j0 + l >= a.n) continue;
+    double v = 0.0;
+    for (int w = 0; w < NTHR / 32; ++w)
+      for (int u = 0; u < a.ppw; ++u) v += red[o * NTHR + w * 32 + u * a.nt + l];
+    if (v != 0.0) atomicAdd(a.g + (size_t)(j0 + l) * (D0 + 1) + o, v);
+  }
+}
 
 // Sb^0 = sum_a Tb^a h^a and Sb^{e_i} = sum_a a_i Tb^a h^{a - e_i} with
 // h^g = s^(|g|+1) W^g.  With M_a = W^a / a! and x_a = a! Tb^a both read
@@ -427,22 +451,89 @@ __global__ void __launch_bounds__(L2T) k_adj_l2a(L2aArgs a) {
       }
     }
   }
-  if (!a.g) return;
-  // the block's sums: warps, then the lanes that share a neuron, then one
-  // atomic per weight
-  __syncthreads();  // the monomials are done with
-  double *red = (double *)sm2;                  // [D0 + 1][L2T]
-#pragma unroll
-  for (int o = 0; o <= D0; ++o) red[o * L2T + threadIdx.x] = act ? acc[o] : 0.0;
+  if (a.g) l2_reduce<D0, L2T>(a, (double *)sm2, acc, act, j0);
+}
+
+// The first-layer adjoint of a small set in the order of k_adj_l2s: slot g's
+// products are formed as (g_i + 1) Tb^{g + e_i} h^g, h^g = s^(|g|+1) W^g, and
+// summed over g = w, w + 32, ...; the sums of the 32 w are added in R in row
+// mode and in FP64 (with the sums over the points) in gradient mode, so that
+// a row or a gradient rounds as it does there.  Tb and h of a thread's
+// (point, neuron) sit in its own columns of shared memory.  Bound: the rows
+// written, or Tb read.
+constexpr int L2RT = 128;
+template <typename R, int D0>
+__global__ void __launch_bounds__(L2RT) k_adj_l2r(L2aArgs a) {
+  extern __shared__ __align__(16) unsigned char sm2[];
+  const int na = a.na, n = a.n, nt = a.nt, j0 = blockIdx.y * nt;
+  R *tb = (R *)sm2 + threadIdx.x, *hh = tb + (size_t)na * L2RT;
+  R *M = (R *)sm2 + (size_t)2 * na * L2RT;      // [na][nt]
+  int *up = (int *)(M + ((size_t)na * nt + 1) / 2 * 2);  // [na][D0]
+  for (int e = threadIdx.x; e < na * D0; e += L2RT) up[e] = __ldg(a.up + e);
+  for (int e = threadIdx.x; e < nt; e += L2RT) M[e] = (R)1;
   __syncthreads();
-  for (int e = threadIdx.x; e < nt * (D0 + 1); e += L2T) {
-    const int o = e / nt, l = e - o * nt;
-    if (j0 + l >= n) continue;
-    double v = 0.0;
-    for (int w = 0; w < L2T / 32; ++w)
-      for (int u = 0; u < a.ppw; ++u) v += red[o * L2T + w * 32 + u * nt + l];
-    if (v != 0.0) atomicAdd(a.g + (size_t)(j0 + l) * (D0 + 1) + o, v);
+  for (int p = 1; p <= a.k; ++p) {
+    const int r0 = a.ds[p], nr = a.ds[p + 1] - r0;
+    for (int e = threadIdx.x; e < nr * nt; e += L2RT) {
+      const int r = r0 + e / nt, jl = e % nt, j = min(j0 + jl, n - 1), pk = __ldg(a.par + r);
+      M[(size_t)r * nt + jl] = (R)((double)M[(size_t)(pk & 0xffff) * nt + jl] *
+                                   __ldg(a.W + (size_t)j * (D0 + 1) + 1 + (pk >> 16)));
+    }
+    __syncthreads();
   }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int jl = lane % nt, sub = lane / nt, j = j0 + jl;
+  const bool act = sub < a.ppw && j < n;
+  double acc[D0 + 1];
+#pragma unroll
+  for (int o = 0; o <= D0; ++o) acc[o] = 0.0;
+  const long nwarp = (long)gridDim.x * (L2RT / 32);
+  for (long w0 = (long)blockIdx.x * (L2RT / 32) + warp; w0 * a.ppw < a.npts; w0 += nwarp) {
+    const long pt = w0 * a.ppw + sub;
+    if (!act || pt >= a.npts) continue;
+    const double *x = a.X + (size_t)pt * D0;
+    const R *Tb = (const R *)a.Tb + (size_t)pt * na * n + j;
+    const R *sg = (const R *)a.sig + (size_t)pt * (a.k + 2) * n + j;
+    for (int p = 0; p <= a.k; ++p) {
+      if (a.ds[p] >= a.ds[p + 1]) continue;
+      const R dq = sg[(size_t)(p + 1) * n];
+      for (int g = a.ds[p]; g < a.ds[p + 1]; ++g) {
+        tb[g * L2RT] = __ldcs(Tb + (size_t)g * n);
+        hh[g * L2RT] = dq * M[(size_t)g * nt + jl];
+      }
+    }
+    R v[D0 + 1];
+#pragma unroll
+    for (int o = 0; o <= D0; ++o) v[o] = (R)0;
+    for (int w = 0; w < min(32, na); ++w) {
+      R s[D0 + 1];
+#pragma unroll
+      for (int o = 0; o <= D0; ++o) s[o] = (R)0;
+      for (int g = w; g < na; g += 32) {
+        const R hg = hh[g * L2RT];
+        s[0] += tb[g * L2RT] * hg;
+#pragma unroll
+        for (int i = 0; i < D0; ++i) {
+          const int u = up[g * D0 + i];
+          if (u >= 0) s[1 + i] += (R)(u >> 16) * tb[(u & 0xffff) * L2RT] * hg;
+        }
+      }
+      if (a.rows) {
+#pragma unroll
+        for (int o = 0; o <= D0; ++o) v[o] += s[o];
+      } else {
+        acc[0] += (double)s[0];
+#pragma unroll
+        for (int i = 0; i < D0; ++i) acc[1 + i] += (double)s[0] * __ldg(x + i) + (double)s[1 + i];
+      }
+    }
+    if (!a.rows) continue;
+    double *row = a.rows + (size_t)pt * a.nw + a.woff + (size_t)j * (D0 + 1);
+    row[0] = (double)v[0];
+#pragma unroll
+    for (int i = 0; i < D0; ++i) row[1 + i] = (double)v[0] * __ldg(x + i) + (double)v[1 + i];
+  }
+  if (a.g) l2_reduce<D0, L2RT>(a, (double *)sm2, acc, act, j0);
 }
 
 // neurons of a tile: the layer cut into equal tiles of at most 32
@@ -453,8 +544,29 @@ size_t l2a_smem(int na, int nt, int d0, size_t rsz) {
   return std::max(tab, (size_t)(d0 + 1) * L2T * 8);
 }
 
+size_t l2r_smem(int na, int nt, int d0, size_t rsz) {
+  return std::max(((size_t)2 * na * L2RT + (size_t)na * nt + 1) * rsz + (size_t)na * d0 * 4 + 16,
+                  (size_t)(d0 + 1) * L2RT * 8);
+}
+// the sets k_adj_l2r takes: rows while the columns fit, and gradients on the
+// split path while its conversions to FP64, one set per slot, cost less than
+// the Tb plane's traffic (in FP64 both orders agree to rounding)
+constexpr int L2R_ROWS = 36, L2R_GRAD = 16;
+
 template <typename R, int D0>
 int l2a_k(L2aArgs a, cudaStream_t st) {
+  if (a.na <= (a.rows ? L2R_ROWS : sizeof(R) == 4 ? L2R_GRAD : 0)) {
+    const size_t smem = l2r_smem(a.na, a.nt, D0, sizeof(R));
+    const void *k = (const void *)k_adj_l2r<R, D0>;
+    CKC(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int gy = (a.n + a.nt - 1) / a.nt;
+    const long per = (long)(L2RT / 32) * a.ppw;
+    const int gx = (int)std::max(1L, std::min((a.npts + per - 1) / per,
+                                              (long)std::max(1, resident_grid(k, L2RT, smem) / gy)));
+    LAUNCH("k_bell_adj_l2", st, (k_adj_l2r<R, D0><<<dim3(gx, gy), L2RT, smem, st>>>(a)));
+    CKC(cudaGetLastError());
+    return RC_OK;
+  }
   constexpr int PT = sizeof(R) == 8 ? 2 : 4;
   const size_t smem = l2a_smem(a.na, a.nt, D0, sizeof(R));
   const void *k = (const void *)k_adj_l2a<R, D0, PT>;
@@ -509,13 +621,19 @@ int fwd_col_t(const ColDev &d, const ColArgs &a, bool train, cudaStream_t st) {
 template <typename R>
 int adj_col_t(const ColDev &d, const ColArgs &a, cudaStream_t st) {
   const size_t smem = col_adj_smem(d.na, d.narec, sizeof(R));
-  const void *k = (const void *)k_bell_adj_col<R>;
+  // one chain per sum, as in k_bell_adj7, for launches too small for the
+  // block-per-point kernels to have been timed on, where that one ran; two,
+  // as in k_bell_adj5, beyond
+  const bool one = (long)a.npts * ((a.n + 128 / (int)sizeof(R) - 1) / (128 / (int)sizeof(R))) <
+                   8L * grid_sms();
+  const void *k = one ? (const void *)k_bell_adj_col<R, 1> : (const void *)k_bell_adj_col<R, 2>;
   CKC(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // at least one neuron row of threads, so that the stride is not zero
   const long total = (long)a.npts * a.n;
   long grid = std::max(1L, std::min((total + NT - 1) / NT, (long)resident_grid(k, NT, smem)));
   grid = std::max(grid, (long)(a.n + NT - 1) / NT);
-  LAUNCH("k_bell_adj", st, (k_bell_adj_col<R><<<(int)grid, NT, smem, st>>>(a)));
+  if (one) { LAUNCH("k_bell_adj", st, (k_bell_adj_col<R, 1><<<(int)grid, NT, smem, st>>>(a))); }
+  else { LAUNCH("k_bell_adj", st, (k_bell_adj_col<R, 2><<<(int)grid, NT, smem, st>>>(a))); }
   CKC(cudaGetLastError());
   return RC_OK;
 }

@@ -1056,8 +1056,7 @@ int gemm_tc_dw(const DevNet *net, int l, int M, int n, int m, const void *Sb, co
 
 // G[i][j] += sum_r J[r][i] J[r][j] (j <= i) over an FP32 copy J[nrow][ldj]
 // (ldj a multiple of 16, zero past nw): k_tc_dw with both operands J over
-// the lower triangle of 128 x 128 output tiles, the rows split across blocks
-// only while there are fewer tiles than SMs.  (4096 rows of 4481:
+// the lower triangle of 128 x 128 output tiles.  (4096 rows of 4481:
 // 0.70 ms, 118 useful TFLOP/s; tiles of 128 x 64 over the whole square through
 // the plain-load kernel took 2.25 ms.)
 int gemm_tc_syrk(const float *J, int nrow, int nw, int ldj, double *G, cudaStream_t st) {
@@ -1070,19 +1069,25 @@ int gemm_tc_syrk(const float *J, int nrow, int nw, int ldj, double *G, cudaStrea
     CKT(cudaMalloc(&flag, sizeof(int)));
     CKT(cudaMemset(flag, 0, sizeof(int)));
   }
-  const int nkb_all = (nrow + tc::DW_RB - 1) / tc::DW_RB;
-  const int ctas_k = (int)std::max<long>(1, std::min<long>(nkb_all, grid_sms() / low));
+  // rows per block: whole 64-row blocks, split over as many blocks as two
+  // waves of 128 x 64 tiles of the full square leave room for.  The split
+  // sets the runs of rows (at most 512) summed in FP32, so the rounding of a
+  // metric depends on nothing else.
+  const int nkb64 = (nrow + 63) / 64;
+  const long tiles = (long)((nw + 63) / 64) * nt;
+  const int ctas_k = (int)std::max<long>(1, std::min<long>(nkb64, 2 * grid_sms() / tiles));
   tc::DwArgs a;
   std::memset(&a, 0, sizeof a);
   a.Mdw = nw; a.Ndw = nw; a.K = nrow;
   a.bwa = a.bwb = std::min(128, ldj);
-  a.kb_per_cta = (nkb_all + ctas_k - 1) / ctas_k;
+  a.kb_per_cta = (nkb64 + ctas_k - 1) / ctas_k * (64 / tc::DW_RB);
   a.G = G; a.gld = nw; a.gcol0 = 0; a.flag = flag; a.low = 1;
   CUtensorMap map;
   std::memset(&map, 0, sizeof map);
   int rc = f32_box_map(&map, J, nrow, ldj, ldj, a.bwa);
   if (rc) return rc;
-  const dim3 grid((nkb_all + a.kb_per_cta - 1) / a.kb_per_cta, (unsigned)low, 1);
+  const int rows_cta = a.kb_per_cta * tc::DW_RB;
+  const dim3 grid((nrow + rows_cta - 1) / rows_cta, (unsigned)low, 1);
   CKT(cudaFuncSetAttribute(tc::k_tc_dw, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)tc::DW_SMEM));
   LAUNCH("k_tc_syrk", st, tc::k_tc_dw<<<grid, tc::DW_NTH, tc::DW_SMEM, st>>>(a, map, map));
