@@ -238,6 +238,13 @@ struct KfDev {
   KfState *st = nullptr;
   KfBar *bar = nullptr;
   int seq_grid = 0;          // CTAs of the one-launch sequence (0: no cooperative launch)
+  // grouped updates (null gbuf: the filter is small): one allocation
+  void *gbuf = nullptr;
+  int nitem = 0;
+  int4 *gitems = nullptr, *grt = nullptr;
+  double *gU = nullptr, *gY = nullptr, *gJ[2] = {nullptr, nullptr};
+  double *grpart = nullptr, *gcpart = nullptr, *gdots = nullptr;
+  void *grp = nullptr;
   double *wprior = nullptr;  // [nw] iterated EKF: the prior weights
   bool prior = false;        // set by an IEKF begin
   double *stage = nullptr;   // host-call staging (rows, innovations, scales, weights)

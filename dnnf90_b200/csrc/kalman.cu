@@ -29,6 +29,9 @@
 // advances lambda.  A call therefore reads and writes the covariance once
 // per observation, plus one read-only pass for the first row.
 //
+// Calls of several observations on a dense filter that is not small apply
+// eight of them per pass (grouped updates, below).
+//
 // Small filters run a whole call as one cooperative launch (k_kf_seq): the
 // same tile code, reduce and scalar step as phases between bounded grid
 // barriers, with the same summation orders, so both paths give the same
@@ -538,6 +541,416 @@ __global__ void __launch_bounds__(256) k_kf_seq(const int4 *__restrict__ tiles, 
   }
 }
 
+// ---------------------------------------------------- grouped updates
+// A call hands over all its rows at once, so up to GM = 8 observations share
+// one pass over the covariance.  With P the covariance before the group and
+// Y_k = P j_k (jf_k = scale_k j_k, written j below), the covariance before
+// observation k of the group is
+//     P_k = a_k P + c_k I - sum_{i<k} b_i p_i p_i^T,   p_i = s_i P_i j_i
+// (s_i the gate's scale), because each update is P <- (P - p p^T / denom) /
+// lambda + q I: a <- a / lambda, c <- c / lambda + q, b_i <- b_i / lambda and
+// b_k = 1 / (lambda denom).  Every p_i is therefore a combination of the Y_l
+// and j_l, l <= i, whose coefficients, denominators and gates follow from the
+// 8 x 8 products j_l . Y_k and j_l . j_k alone.  Per group three launches:
+//   k_kf_greduce  sums the partial products into Y, forms the 8 x 8
+//                 products, and its last CTA runs the recursion over k
+//   k_kf_gvec     U_i = sqrt(b_i) p_i, w += sum_k p_k xi_k / denom_k, and the
+//                 next group's rows packed as [weight][8]
+//   k_kf_gtiles   P <- a P + c I - U U^T and, in the same read, the products
+//                 of the new P with the next group's rows
+// The covariance is read and written once per eight observations instead of
+// once per observation.  A sum of squares -U U^T rounds alike on both sides
+// of the diagonal, so P stays exactly symmetric.  A denominator that is not
+// positive ends the group there: the observations before it are applied.
+
+constexpr int GM = 8;            // observations per group
+constexpr int GW = 8;            // warps of k_kf_gtiles: tile rows of a row block
+constexpr int GVS = 12;          // row stride of the staged column vectors (doubles)
+
+struct KfGroup {
+  int m;                         // observations to apply (0: none)
+  double a, c;
+  double ua[GM][GM], ub[GM][GM]; // U_i = sum_l ua[i][l] Y_l + ub[i][l] j_l
+  double wa[GM], wb[GM];         // w += sum_l wa[l] Y_l + wb[l] j_l
+};
+
+__device__ __forceinline__ void kf_dmma(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+__device__ __forceinline__ void kf_cp16(void *dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (uint32_t)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+// 16-byte chunk of (row, column pair c2) in a staged tile: the exclusive or
+// spreads the rows so that both the fragment reads of 16 bytes (8 rows x 4
+// pairs) and the transposed ones of 8 bytes (4 rows x 4 columns per half
+// warp) meet each bank once
+__device__ __forceinline__ int kf_chunk(int row, int c2) {
+  return row * 16 + (c2 ^ (((row & 1) << 2) | (row & 2)));
+}
+
+// One CTA per item: a row block of eight tile rows I0 .. I0 + 7, one per
+// warp, over the column tiles J0 .. J0 + Jn - 1.  A warp holds its 32 x 32
+// tile as 4 x 4 fragments of the FP64 tensor cores (mma.sync m8n8k4, 32
+// products each for the update and the two products with the next rows); the
+// fragment of the updated tile is itself the left operand of the row
+// products, with column 8 j + 2 c4 + e as the product's k; the column
+// products read the tile transposed from shared memory.  The next column's
+// tiles and vectors stream in by cp.async meanwhile.  Row products stay in
+// registers along the item, column products are summed over the eight warps,
+// so the partial sums are a tenth of the covariance's traffic.
+// Bound: HBM; at nw = 17025 one pass takes 450 us for 2.32 GB (5.1 TB/s), 69 us
+// per observation with the two small launches, against 569 for single updates.
+template <int MODE>
+__global__ void __launch_bounds__(GW * 32, 1)
+    k_kf_gtiles(const int4 *__restrict__ items, int n, double *__restrict__ P,
+                const double *__restrict__ U, const double *__restrict__ Jn,
+                const KfGroup *__restrict__ grp, const KfState *__restrict__ st,
+                double *__restrict__ rpart, double *__restrict__ cpart) {
+  extern __shared__ __align__(16) double gsm[];
+  double *tiles = gsm;                          // [2][GW][KTE]
+  double *vec = tiles + 2 * GW * KTE;           // [2][2][KT * GVS]: U, J of the column tile
+  double *colb = vec + 2 * 2 * KT * GVS;        // [GW][KT * GM]
+  double ga = 1.0, gc = 0.0;
+  if (MODE == KM_PJ) {
+    if (st->status) return;
+  } else {
+    if (grp->m == 0) return;
+    ga = grp->a;
+    gc = grp->c;
+  }
+  const int4 ia = items[2 * blockIdx.x], ib = items[2 * blockIdx.x + 1];
+  const int I0 = ia.x, J0 = ia.y, nJ = ia.z, rp = ib.x, cp = ib.y;
+  const int tb = (n + KT - 1) / KT;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31, r8 = lane >> 2, c4 = lane & 3;
+  const int I = I0 + warp;
+  // first tile of this warp's row: (I, J) sits at row0 + J
+  double *row0 = P + ((size_t)I * tb - (size_t)I * (I - 1) / 2 - I) * KTE;
+  auto stage = [&](int jj) {
+    const int J = J0 + jj, buf = jj & 1;
+    if (I < tb && I <= J) {
+      double *dst = tiles + (buf * GW + warp) * KTE;
+      const double *src = row0 + (size_t)J * KTE;
+#pragma unroll
+      for (int q = 0; q < KTE / 2 / 32; ++q) {
+        const int e = q * 32 + lane;  // 16-byte chunk: row e / 16, pair e % 16
+        kf_cp16(dst + 2 * kf_chunk(e >> 4, e & 15), src + 2 * e);
+      }
+    }
+    // the vectors of the column tile: 32 rows of 8 doubles each
+    {
+      const int which = t >> 7, e = t & 127, r = e >> 2, c = (e & 3) * 2, R = J * KT + r;
+      double *dst = vec + (buf * 2 + which) * KT * GVS + r * GVS + c;
+      const double *src = which ? Jn : U;
+      if (which ? MODE != KM_UPD : MODE != KM_PJ) {
+        if (R < n) kf_cp16(dst, src + (size_t)R * GM + c);
+        else *(double2 *)dst = make_double2(0.0, 0.0);
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  stage(0);
+  double ur[4][2], jr[4][2], yr[4][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+      const int Ru = I * KT + 8 * i + r8, Rj = I * KT + 8 * i + c4 + 4 * s;
+      ur[i][s] = MODE != KM_PJ && Ru < n ? -U[(size_t)Ru * GM + c4 + 4 * s] : 0.0;
+      jr[i][s] = MODE != KM_UPD && Rj < n ? Jn[(size_t)Rj * GM + r8] : 0.0;
+      yr[i][s] = 0.0;
+    }
+  for (int jj = 0; jj < nJ; ++jj) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // this column's vectors are in; every warp is done with the last column
+    if (jj + 1 < nJ) stage(jj + 1);
+    const int J = J0 + jj, buf = jj & 1;
+    const bool act = I < tb && I <= J;
+    double *tile = tiles + (buf * GW + warp) * KTE;
+    const double *uc = vec + (buf * 2) * KT * GVS, *jc = uc + KT * GVS;
+    double yc[4][2];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) yc[j][0] = yc[j][1] = 0.0;
+    if (act) {
+      __syncwarp();  // this warp's copies of the tile
+      double *gp = row0 + (size_t)J * KTE;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        double v[4][2];
+        const int row = 8 * i + r8;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double2 x = *(const double2 *)(tile + 2 * kf_chunk(row, 4 * j + c4));
+          v[j][0] = x.x;
+          v[j][1] = x.y;
+        }
+        if (MODE != KM_PJ) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            v[j][0] *= ga;
+            v[j][1] *= ga;
+#pragma unroll
+            for (int s = 0; s < 2; ++s)
+              kf_dmma(v[j], ur[i][s], uc[(8 * j + r8) * GVS + c4 + 4 * s]);
+            if (I == J && i == j && I * KT + row < n) {
+              if (r8 == 2 * c4) v[j][0] += gc;
+              if (r8 == 2 * c4 + 1) v[j][1] += gc;
+            }
+            const double2 x = make_double2(v[j][0], v[j][1]);
+            if (MODE != KM_UPD) *(double2 *)(tile + 2 * kf_chunk(row, 4 * j + c4)) = x;
+            __stcs((double2 *)(gp + row * KT + 8 * j + 2 * c4), x);
+          }
+        }
+        if (MODE != KM_UPD)
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+              kf_dmma(yr[i], v[j][e], jc[(8 * j + 2 * c4 + e) * GVS + r8]);
+      }
+      if (MODE != KM_UPD && I != J) {
+        __syncwarp();  // the updated tile is in shared memory
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+#pragma unroll
+            for (int s = 0; s < 2; ++s) {
+              const int row = 8 * i + c4 + 4 * s, col = 8 * j + r8;
+              kf_dmma(yc[j], tile[2 * kf_chunk(row, col >> 1) + (col & 1)], jr[i][s]);
+            }
+      }
+    }
+    if (MODE != KM_UPD) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        *(double2 *)(colb + warp * KT * GM + (8 * j + r8) * GM + 2 * c4) =
+            make_double2(yc[j][0], yc[j][1]);
+      __syncthreads();
+      double v = 0.0;
+#pragma unroll
+      for (int w = 0; w < GW; ++w) v += colb[w * KT * GM + t];
+      cpart[(size_t)(cp + jj) * KT * GM + t] = v;
+    }
+  }
+  if (MODE != KM_UPD)
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      *(double2 *)(rpart + (size_t)(rp + warp) * KT * GM + (8 * i + r8) * GM + 2 * c4) =
+          make_double2(yr[i][0], yr[i][1]);
+}
+
+// Y of one row tile from the partial sums (column partials of the row blocks
+// 0 .. K / 8, then the row block's own segments, in that order), the tile's
+// shares of j_l . Y_k and j_l . j_k, and in the last CTA (a counter, no
+// waiting) their totals and the recursion over the group's observations.
+constexpr int GRT = 512;
+__global__ void __launch_bounds__(GRT)
+    k_kf_greduce(int nw, const int4 *__restrict__ grt,
+                 const double *__restrict__ rpart, const double *__restrict__ cpart,
+                 const double *__restrict__ J, double *__restrict__ Y, KfRowArgs ra, int k0, int m,
+                 int kbase, double *__restrict__ dots, unsigned *__restrict__ ctr,
+                 KfGroup *__restrict__ grp, KfState *__restrict__ st) {
+  __shared__ double ys[KT * GM], js[KT * GM], half[KT * GM];
+  __shared__ double tot[4][2 * GM * GM];
+  __shared__ double al[GM][GM], be[GM][GM], bb[GM], dd[GM], wc[GM];
+  __shared__ bool s_last;
+  const int t = threadIdx.x;
+  if (st->status) {  // an earlier group failed: nothing is applied from there on
+    if (blockIdx.x == 0 && t == 0) grp->m = 0;
+    return;
+  }
+  const int K = blockIdx.x, tb = gridDim.x, nb = K / GW;  // row tile, tiles per side
+  const int4 gr = grt[K];            // x: its first row partial, y: segments of its row block
+  {
+    const int e = t & 255, h = t >> 8;  // even terms, odd terms
+    const int terms = nb + 1 + gr.y;
+    double v = 0.0;
+#pragma unroll 8
+    for (int q = h; q < terms; q += 2) {
+      const double *src =
+          q <= nb ? cpart + (size_t)(q * tb - GW / 2 * q * (q - 1) + K - GW * q) * KT * GM
+                  : rpart + (size_t)(gr.x + (q - nb - 1) * GW) * KT * GM;
+      v += __ldcg(src + e);
+    }
+    if (h) half[e] = v;
+    __syncthreads();
+    if (!h) {
+      v += half[e];
+      const bool ok = K * KT + (e >> 3) < nw;
+      ys[e] = ok ? v : 0.0;
+      js[e] = ok ? J[(size_t)K * KT * GM + e] : 0.0;
+      if (ok) Y[(size_t)K * KT * GM + e] = v;
+    }
+  }
+  __syncthreads();
+  if (t < 2 * GM * GM) {  // j_l . Y_k, then j_l . j_k
+    const int l = (t >> 3) & 7, k = t & 7;
+    const double *b = t < GM * GM ? ys : js;
+    double v = 0.0;
+#pragma unroll 8
+    for (int r = 0; r < KT; ++r) v = fma(js[r * GM + l], b[r * GM + k], v);
+    dots[(size_t)blockIdx.x * 2 * GM * GM + t] = v;
+  }
+  __threadfence();
+  __syncthreads();
+  if (t == 0) s_last = atomicAdd(ctr, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  {
+    const int e = t & 127, h = t >> 7;
+    double v = 0.0;
+#pragma unroll 16
+    for (int b = h; b < (int)gridDim.x; b += 4) v += __ldcg(dots + (size_t)b * 2 * GM * GM + e);
+    tot[h][e] = v;
+  }
+  __syncthreads();
+  if (t < 128) tot[0][t] += tot[1][t] + (tot[2][t] + tot[3][t]);
+  __syncthreads();
+  if (t >= 32) return;
+  // one warp: lane l the coefficients of Y_l and j_l
+  const double *g = tot[0], *nn = tot[0] + GM * GM;
+  const int l = t & 7;
+  const double q = st->q, gate = st->gate, lam0 = st->lam0;
+  double lam = st->lam, a = 1.0, c = 0.0;
+  int k = 0, ng = 0, fail = 0;
+  double lamk = lam, denomk = 0.0, sgk = 1.0, xik = 0.0;
+  for (; k < m; ++k) {
+    if (t < GM) {  // lane i: d_ik = p_i . j_k
+      double d = 0.0;
+      if (t < k)
+        for (int x = 0; x <= t; ++x)
+          d = fma(al[t][x], g[x * GM + k], fma(be[t][x], nn[x * GM + k], d));
+      dd[t] = d;
+    }
+    __syncwarp();
+    double jpj = fma(a, g[k * GM + k], c * nn[k * GM + k]);
+    double av = l == k ? a : 0.0, bv = l == k ? c : 0.0;
+    for (int i = 0; i < k; ++i) {
+      const double bd = bb[i] * dd[i];
+      jpj = fma(-bd, dd[i], jpj);
+      av = fma(-bd, al[i][l], av);
+      bv = fma(-bd, be[i][l], bv);
+    }
+    double denom = lam + jpj;
+    if (!(denom > 0.0)) {
+      fail = kbase + k0 + k + 1;
+      break;
+    }
+    double xi = row_scale(ra, k0 + k) * ra.xi[k0 + k], sg = 1.0;
+    if (gate > 0.0 && xi * xi > gate * gate * denom) {
+      const double s2 = gate * gate * lam / (xi * xi - gate * gate * jpj);
+      sg = sqrt(s2);
+      xi = sg * xi;
+      denom = lam + s2 * jpj;
+      ++ng;
+    }
+    __syncwarp();
+    if (t < GM) {
+      al[k][l] = sg * av;
+      be[k][l] = sg * bv;
+      if (t < k) bb[t] /= lam;
+      if (t == k) {
+        bb[k] = 1.0 / (lam * denom);
+        wc[k] = xi / denom;
+      }
+    }
+    a /= lam;
+    c = c / lam + (q > 0.0 ? q : 0.0);
+    lamk = lam;
+    denomk = denom;
+    sgk = sg;
+    xik = xi;
+    lam = __dadd_rn(__dmul_rn(lam0, lam), 1.0) - lam0;
+    __syncwarp();
+  }
+  if (t < GM) {
+    double wa = 0.0, wb = 0.0;
+    for (int i = 0; i < k; ++i) {
+      const double s = sqrt(bb[i]);
+      grp->ua[i][l] = s * al[i][l];
+      grp->ub[i][l] = s * be[i][l];
+      wa = fma(wc[i], al[i][l], wa);
+      wb = fma(wc[i], be[i][l], wb);
+    }
+    for (int i = k; i < GM; ++i) grp->ua[i][l] = grp->ub[i][l] = 0.0;
+    grp->wa[l] = wa;
+    grp->wb[l] = wb;
+  }
+  if (t == 0) {
+    *ctr = 0;
+    grp->m = k;
+    grp->a = a;
+    grp->c = c;
+    st->lam = lam;
+    st->ngated += ng;
+    if (k > 0) {
+      st->lamk = lamk;
+      st->denom = denomk;
+      st->sg = sgk;
+      st->xi = xik;
+    }
+    if (fail) st->status = fail;
+  }
+}
+
+// U, the weights and the next group's packed rows (grp null: only the rows);
+// one thread per weight
+__global__ void __launch_bounds__(128)
+    k_kf_gvec(int nw, const KfGroup *__restrict__ grp, const double *__restrict__ Y,
+              const double *J, double *__restrict__ U, double *__restrict__ w,
+              KfRowArgs ra, int knext, int mnext, double *Jnext) {
+  __shared__ KfGroup g;
+  const int R = blockIdx.x * 128 + threadIdx.x;
+  if (grp) {
+    for (int e = threadIdx.x; e < (int)(sizeof(KfGroup) / 4); e += 128)
+      ((int *)&g)[e] = ((const int *)grp)[e];
+    __syncthreads();
+    if (g.m == 0) return;
+  }
+  if (R >= nw) return;
+  if (grp) {
+    double y[GM], j[GM], dw = 0.0;
+#pragma unroll
+    for (int l = 0; l < GM; l += 2) {
+      const double2 a = *(const double2 *)(Y + (size_t)R * GM + l);
+      const double2 b = *(const double2 *)(J + (size_t)R * GM + l);
+      // rows from a failed observation on take no part (they may hold NaN)
+      y[l] = l < g.m ? a.x : 0.0;
+      y[l + 1] = l + 1 < g.m ? a.y : 0.0;
+      j[l] = l < g.m ? b.x : 0.0;
+      j[l + 1] = l + 1 < g.m ? b.y : 0.0;
+    }
+#pragma unroll
+    for (int l = 0; l < GM; ++l) dw = fma(g.wa[l], y[l], fma(g.wb[l], j[l], dw));
+    w[R] += dw;
+#pragma unroll
+    for (int i = 0; i < GM; i += 2) {
+      double u[2] = {0.0, 0.0};
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int l = 0; l <= i + h; ++l)
+          u[h] = fma(g.ua[i + h][l], y[l], fma(g.ub[i + h][l], j[l], u[h]));
+      *(double2 *)(U + (size_t)R * GM + i) = make_double2(u[0], u[1]);
+    }
+  }
+  if (mnext > 0) {
+    double v[GM];
+#pragma unroll
+    for (int k = 0; k < GM; ++k)
+      v[k] = k < mnext ? row_scale(ra, knext + k) * ra.rows[(size_t)(knext + k) * ra.ld + R] : 0.0;
+#pragma unroll
+    for (int k = 0; k < GM; k += 2)
+      *(double2 *)(Jnext + (size_t)R * GM + k) = make_double2(v[k], v[k + 1]);
+  }
+}
+
 __global__ void k_kf_init_tiles(const int4 *__restrict__ tiles, double *__restrict__ P, double p0) {
   const int4 t = tiles[blockIdx.x];
   double *tp = P + (size_t)blockIdx.x * KTE;
@@ -560,7 +973,113 @@ void KfDev::release() {
   cudaFree(bar);
   cudaFree(stage);
   cudaFree(wprior);
+  cudaFree(gbuf);
   *this = KfDev();
+}
+
+// Dense filters of at least this many tiles group the observations of a call
+// (of at least KF_GROUP_OBS); smaller ones keep the one-launch sequence, whose
+// bits do not depend on how a sequence is split into calls.
+// The decoupled filter keeps single updates: its blocks share the denominators
+// but each has products j_l . P j_k of its own, so that the recursion would
+// run per block.
+// Measured per observation, 64 (3) to a call, against the faster of the
+// single-update paths: nw = 1217 5.5 (21) us against 14.3 (25.5), 4481 9.4 (31)
+// against 48 (64), 17025 69 (220) against 569 (645).
+constexpr int KF_GROUP_TILES = 512, KF_GROUP_OBS = 3;
+constexpr size_t GT_SMEM =
+    (size_t)(2 * GW * KTE + 2 * 2 * KT * GVS + GW * KT * GM) * sizeof(double);
+
+// buffers and work items of the grouped updates: one allocation
+static int group_create(KfDev &d) {
+  std::vector<int4> items, grt;
+  const int tb = (d.nw + KT - 1) / KT;
+  long steps = 0;
+  for (int I0 = 0; I0 < tb; I0 += GW) steps += tb - I0;
+  // column tiles per item: about 12, so that its start-up is small beside
+  // it, and a whole number of waves of one CTA per SM
+  const long waves = std::max(1L, (steps + 6L * grid_sms()) / (12L * grid_sms()));
+  const int seg = (int)std::max(2L, (steps + waves * grid_sms() - 1) / (waves * grid_sms()));
+  int cp = 0, rp = 0;
+  for (int I0 = 0; I0 < tb; I0 += GW) {
+    const int rblock = rp, ns = (tb - I0 + seg - 1) / seg;
+    for (int s = 0; s < ns; ++s) {
+      const int J0 = I0 + s * seg, nJ = std::min(seg, tb - J0);
+      items.push_back(make_int4(I0, J0, nJ, 0));
+      items.push_back(make_int4(rp, cp, 0, 0));
+      rp += GW;
+      cp += nJ;
+    }
+    for (int K = I0; K < std::min(tb, I0 + GW); ++K) {
+      grt.push_back(make_int4(rblock + K - I0, ns, 0, 0));
+    }
+  }
+  size_t cur = 0;
+  auto take = [&](size_t bytes) {
+    const size_t at = cur;
+    cur = (cur + bytes + 255) / 256 * 256;
+    return at;
+  };
+  const size_t vb = (size_t)d.nw * GM * sizeof(double);
+  const size_t oi = take(items.size() * sizeof(int4)), og = take(grt.size() * sizeof(int4));
+  const size_t oU = take(vb), oY = take(vb), oJ0 = take(vb), oJ1 = take(vb);
+  const size_t orp = take((size_t)rp * KT * GM * 8), ocp = take((size_t)cp * KT * GM * 8);
+  const size_t od = take((size_t)d.nred * 2 * GM * GM * 8), ogr = take(sizeof(KfGroup));
+  if (cudaMalloc(&d.gbuf, cur) != cudaSuccess) {
+    cudaGetLastError();  // the two-launch path needs none of it
+    d.gbuf = nullptr;
+    return RC_OK;
+  }
+  char *p = (char *)d.gbuf;
+  CKK(cudaMemcpy(p + oi, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  CKK(cudaMemcpy(p + og, grt.data(), grt.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  d.nitem = (int)items.size() / 2;
+  d.gitems = (int4 *)(p + oi);
+  d.grt = (int4 *)(p + og);
+  d.gU = (double *)(p + oU);
+  d.gY = (double *)(p + oY);
+  d.gJ[0] = (double *)(p + oJ0);
+  d.gJ[1] = (double *)(p + oJ1);
+  d.grpart = (double *)(p + orp);
+  d.gcpart = (double *)(p + ocp);
+  d.gdots = (double *)(p + od);
+  d.grp = p + ogr;
+  return RC_OK;
+}
+
+template <int MODE>
+static int launch_gtiles(const KfDev &d, const double *Jn, cudaStream_t s) {
+  CKK(cudaFuncSetAttribute(k_kf_gtiles<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)GT_SMEM));
+  LAUNCH("k_kf_gtiles", s,
+         (k_kf_gtiles<MODE><<<d.nitem, GW * 32, GT_SMEM, s>>>(
+             d.gitems, d.nw, d.P, d.gU, Jn, (const KfGroup *)d.grp, d.st, d.grpart, d.gcpart)));
+  CKK(cudaGetLastError());
+  return RC_OK;
+}
+
+// the observations of one call, eight to a pass over the covariance
+static int run_groups(KfDev &d, int nobs, const KfRowArgs &ra, double *w, cudaStream_t s,
+                      int kbase) {
+  KfGroup *grp = (KfGroup *)d.grp;
+  const int gv = (d.nw + 127) / 128;
+  int rc;
+  LAUNCH("k_kf_gvec", s, (k_kf_gvec<<<gv, 128, 0, s>>>(d.nw, nullptr, d.gY, d.gJ[0], d.gU, w, ra, 0,
+                                                       std::min(GM, nobs), d.gJ[0])));
+  if ((rc = launch_gtiles<KM_PJ>(d, d.gJ[0], s))) return rc;
+  for (int k0 = 0, b = 0; k0 < nobs; k0 += GM, b ^= 1) {
+    const int m = std::min(GM, nobs - k0), mn = std::max(0, std::min(GM, nobs - k0 - GM));
+    LAUNCH("k_kf_greduce", s,
+           (k_kf_greduce<<<d.nred, GRT, 0, s>>>(d.nw, d.grt, d.grpart, d.gcpart, d.gJ[b], d.gY, ra,
+                                                k0, m, kbase, d.gdots, d.ctr, grp, d.st)));
+    LAUNCH("k_kf_gvec", s, (k_kf_gvec<<<gv, 128, 0, s>>>(d.nw, grp, d.gY, d.gJ[b], d.gU, w, ra,
+                                                         k0 + GM, mn, d.gJ[b ^ 1])));
+    if ((rc = mn ? launch_gtiles<KM_UPD_PJ>(d, d.gJ[b ^ 1], s)
+                 : launch_gtiles<KM_UPD>(d, d.gJ[b ^ 1], s)))
+      return rc;
+  }
+  CKK(cudaGetLastError());
+  return RC_OK;
 }
 
 int kf_create(KfDev &d, const std::vector<int> &bsz, const std::vector<int> &boff, double p0,
@@ -613,6 +1132,10 @@ int kf_create(KfDev &d, const std::vector<int> &bsz, const std::vector<int> &bof
     d.seq_grid = coop && per_sm > 0 ? std::min(grid_sms() * per_sm, std::max(d.ntile, d.nred))
                                     : 0;
   }
+  if (d.dense && d.ntile >= KF_GROUP_TILES) {
+    const int rc = group_create(d);
+    if (rc) return rc;
+  }
   CKK(cudaMemcpy(d.tiles, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice));
   CKK(cudaMemcpy(d.rtl, rtl.data(), rtl.size() * sizeof(int4), cudaMemcpyHostToDevice));
   CKK(cudaMemset(d.ctr, 0, sizeof(unsigned)));
@@ -634,6 +1157,18 @@ int kf_run(KfDev &d, int nobs, const double *rows, size_t ld, const double *xi,
   if (nobs <= 0) return RC_OK;
   KfRowArgs ra{rows, ld, xi, scale};
   int path = g_kf_path.load();
+  // a call of several observations on a larger filter: every call of a
+  // sequence comes here, so each forms its own first products
+  if (path < 0 && d.gbuf && nobs >= KF_GROUP_OBS) {
+    if (kbase == 0) CKK(cudaMemsetAsync(&d.st->status, 0, sizeof(int), s));
+    return run_groups(d, nobs, ra, w, s, kbase);
+  }
+  // one or two observations of a grouping filter: the call before, grouped,
+  // formed no products for this one
+  if (path < 0 && d.gbuf) {
+    first = true;
+    has_next = false;
+  }
   // a stream being captured into a graph takes the two-launch path, whose
   // kernels are plain launches
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;

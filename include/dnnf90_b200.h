@@ -267,8 +267,10 @@ int dnnf90_tune_report(char *buf, int len);
  * recurrence measured faster).  The two forwards agree to rounding.  which 3
  * picks the Kalman update path: 0 two launches per update, 1 one
  * cooperative launch per call, -1 by size (the default: one launch for
- * small filters); the two give identical bits.  For reproducible timing and
- * for tests; new */
+ * small filters); the two give identical bits.  By size, a call of several
+ * observations on a dense filter of about 1000 weights or more applies eight
+ * of them per pass over the covariance, equal to the single updates to
+ * rounding.  For reproducible timing and for tests; new */
 int dnnf90_tune_force(int which, int variant);
 /* policy (0 work, 1 square root, 2 none) and timed replay ms of the graph
  * the last committee step used; new */
