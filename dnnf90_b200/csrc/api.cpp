@@ -39,7 +39,14 @@ struct NetH {
   int nlayer = 0;
   std::vector<int> dims;
   std::vector<double> w;  // flat layer layout
-  uint64_t wver = 1;      // bumped on every host-side weight change
+  uint64_t wver = 1;      // bumped on every weight change
+  // w64 on the device is newer than w (host_weights fetches it)
+  bool host_stale = false;
+  // recorded after the last write of w64, on wst: a call on another stream
+  // waits for it
+  cudaEvent_t wev = nullptr;
+  cudaStream_t wst = nullptr;
+  bool wev_set = false;
   int prec = PREC_F64;
   bool dt_ok = false;
   DevTables dt;
@@ -151,7 +158,49 @@ size_t layer_off(const NetH &n, int l) {  // 1-based l in 2..nlayer
   return o;
 }
 
-// device copies of the network's tables and weights, refreshed when stale
+bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(st, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+// the device weights were written on st
+int weights_written(NetH &n, cudaStream_t st) {
+  int rc;
+  if (!n.wev && (rc = ck(cudaEventCreateWithFlags(&n.wev, cudaEventDisableTiming), "event")))
+    return rc;
+  n.wst = st;
+  n.wev_set = true;
+  return ck(cudaEventRecord(n.wev, st), "weights event");
+}
+
+// the host copy of the weights, fetched if the device's is newer
+int host_weights(NetH &n) {
+  if (!n.host_stale) return RC_OK;
+  int rc = RC_OK;
+  if (n.wev_set) rc = ck(cudaEventSynchronize(n.wev), "weights event");
+  if (!rc) rc = ck(cudaMemcpy(n.w.data(), n.dn.w64, sizeof(double) * n.w.size(),
+                              cudaMemcpyDeviceToHost), "weights D2H");
+  if (!rc) n.host_stale = false;
+  return rc;
+}
+
+// device buffers of the weights
+int net_buffers(NetH &n) {
+  DevNet &d = n.dn;
+  if (d.w64) return RC_OK;
+  d.nlayer = n.nlayer;
+  d.dims = n.dims;
+  d.nw = (int)n.w.size();
+  d.woff.assign(n.nlayer, 0);
+  for (int l = 2; l <= n.nlayer; ++l) d.woff[l - 1] = layer_off(n, l);
+  int rc;
+  if ((rc = ck(cudaMalloc(&d.w64, n.w.size() * sizeof(double)), "cudaMalloc"))) return rc;
+  if ((rc = ck(cudaMalloc(&d.w32, n.w.size() * sizeof(float)), "cudaMalloc"))) return rc;
+  return ck(cudaMalloc(&d.wpk, 2 * n.w.size() * sizeof(double)), "cudaMalloc");
+}
+
+// device copies of the network's tables and weights, refreshed when stale,
+// ordered before what st runs next
 int net_device(NetH &n, cudaStream_t st) {
   int rc = device_ready();
   if (rc) return rc;
@@ -159,26 +208,38 @@ int net_device(NetH &n, cudaStream_t st) {
     if ((rc = upload_tables(n.ts, n.dt))) return rc;
     n.dt_ok = true;
   }
-  if (n.dn.uploaded != n.wver) {
-    DevNet &d = n.dn;
-    if (!d.w64) {
-      d.nlayer = n.nlayer;
-      d.dims = n.dims;
-      d.nw = (int)n.w.size();
-      d.woff.assign(n.nlayer, 0);
-      for (int l = 2; l <= n.nlayer; ++l) d.woff[l - 1] = layer_off(n, l);
-      if ((rc = ck(cudaMalloc(&d.w64, n.w.size() * sizeof(double)), "cudaMalloc"))) return rc;
-      if ((rc = ck(cudaMalloc(&d.w32, n.w.size() * sizeof(float)), "cudaMalloc"))) return rc;
-      if ((rc = ck(cudaMalloc(&d.wpk, 2 * n.w.size() * sizeof(double)), "cudaMalloc"))) return rc;
-    }
+  DevNet &d = n.dn;
+  if ((rc = net_buffers(n))) return rc;
+  if (d.uploaded != n.wver) {
     if ((rc = ck(cudaMemcpyAsync(d.w64, n.w.data(), n.w.size() * sizeof(double),
-                                 cudaMemcpyHostToDevice, st), "weights H2D")))
+                                 cudaMemcpyHostToDevice, st), "weights H2D")) ||
+        (rc = weights_written(n, st)))
       return rc;
-    if ((rc = weights_to_f32(d.w64, d.w32, n.w.size(), st))) return rc;
-    if ((rc = gemm_tc_prepare(&d, n.w.data(), st))) return rc;
     d.uploaded = n.wver;
+  } else if (n.wev_set && n.wst != st && !capturing(st)) {
+    if ((rc = ck(cudaStreamWaitEvent(st, n.wev, 0), "weights wait"))) return rc;
+  }
+  // the split path's operands follow the FP64 weights
+  if (n.prec == PREC_SPLIT && d.derived != n.wver) {
+    if ((rc = weights_to_f32(d.w64, d.w32, n.w.size(), st)) || (rc = gemm_tc_prepare(&d, st)) ||
+        (rc = weights_written(n, st)))
+      return rc;
+    d.derived = n.wver;
   }
   return RC_OK;
+}
+
+// makes st wait for what earlier calls left on the legacy default stream
+// (accumulators zeroed, Adam updates)
+int after_null_stream(cudaStream_t st) {
+  static cudaEvent_t ev[64] = {};
+  int dev = 0, rc;
+  if ((rc = ck(cudaGetDevice(&dev), "device"))) return rc;
+  if (dev < 0 || dev >= 64) return ck(cudaStreamSynchronize(nullptr), "sync");
+  if (!ev[dev] && (rc = ck(cudaEventCreateWithFlags(&ev[dev], cudaEventDisableTiming), "event")))
+    return rc;
+  if ((rc = ck(cudaEventRecord(ev[dev], nullptr), "event"))) return rc;
+  return ck(cudaStreamWaitEvent(st, ev[dev], 0), "wait");
 }
 
 int work_stream(WorkH &w) {
@@ -223,7 +284,13 @@ int plane_cap(const WorkH &w, const NetH &n) {
   return cap;
 }
 
+// the planes already hold want points in one chunk
+bool planes_hold(const WorkH &w, const NetH &n, int want) {
+  return w.p.base && w.p.prec == n.prec && w.p.cap_pts >= want && (w.chunk <= 0 || want <= w.chunk);
+}
+
 int work_planes(WorkH &w, NetH &n, int want, bool exact) {
+  if (planes_hold(w, n, want)) return RC_OK;  // no need to ask for the free memory
   const int cap = plane_cap(w, n);
   int need = std::min(want, cap);
   if (exact && want > cap) {
@@ -297,6 +364,8 @@ int flush_queue(int tid) {
                                cudaMemcpyHostToDevice, w.st), "H2D")))
     return rc;
   if ((rc = work_planes(w, n, np, false))) return rc;
+  if ((rc = after_null_stream(w.st))) return rc;
+  w.kept = false;
   DevRule given;
   given.kind = SEED_GIVEN;
   BatchArgs a;
@@ -464,8 +533,8 @@ int run_eval(int nid, WorkH &w, int npts, const double *x, double *tm,
     }
   }
   if (host) {
-    if ((rc = ck(cudaStreamSynchronize(w.st), "eval"))) return rc;
-    return gemm_tc_flag(&n.dn, w.st);
+    if (n.prec == PREC_SPLIT) return gemm_tc_flag(&n.dn, w.st);  // waits for st
+    return ck(cudaStreamSynchronize(w.st), "eval");
   }
   return RC_OK;
 }
@@ -511,30 +580,19 @@ int host_train(int nid, int tid, int npts, const double *x, int kind,
   const int na = n.ts.na, d0 = n.ts.d0, nout = n.dims[n.nlayer - 1];
   const int cap = w.p.cap_pts;
   const int nw = (int)n.w.size();
-  double *dseed = nullptr, *drows = nullptr, *dloss = nullptr;
-  if (kind == SEED_GIVEN) {
-    if ((rc = ck(cudaMalloc(&dseed, sizeof(double) * (size_t)cap * nout * na), "cudaMalloc"))) return rc;
-  }
-  if (rows) {
-    if ((rc = ck(cudaMalloc(&drows, sizeof(double) * (size_t)cap * nw), "cudaMalloc"))) {
-      if (dseed) cudaFree(dseed);
-      return rc;
-    }
-  }
-  if ((rc = ck(cudaMalloc(&dloss, sizeof(double)), "cudaMalloc"))) {
-    if (dseed) cudaFree(dseed);
-    if (drows) cudaFree(drows);
-    return rc;
-  }
   const int nres = rule ? rule->r.nres : 0;
-  double *dsrc = nullptr;
-  if (src && nres > 0 &&
-      (rc = ck(cudaMalloc(&dsrc, sizeof(double) * (size_t)cap * nres), "cudaMalloc"))) {
-    if (dseed) cudaFree(dseed);
-    if (drows) cudaFree(drows);
-    cudaFree(dloss);
+  DevScratch seeds, rowbuf, srcs;
+  if (kind == SEED_GIVEN &&
+      (rc = ck(seeds.take(sizeof(double) * (size_t)cap * nout * na, w.st), "scratch")))
     return rc;
-  }
+  if (rows && (rc = ck(rowbuf.take(sizeof(double) * (size_t)cap * nw, w.st), "scratch"))) return rc;
+  if (src && nres > 0 &&
+      (rc = ck(srcs.take(sizeof(double) * (size_t)cap * nres, w.st), "scratch")))
+    return rc;
+  double *dseed = seeds.as<double>(), *drows = rowbuf.as<double>(), *dsrc = srcs.as<double>();
+  double *dloss = w.p.loss;
+  if ((rc = after_null_stream(w.st))) return rc;
+  w.kept = false;
   cudaMemsetAsync(dloss, 0, sizeof(double), w.st);
   std::vector<double> sm, tbuf;
   for (int c0 = 0; c0 < npts && !rc; c0 += cap) {
@@ -570,36 +628,46 @@ int host_train(int nid, int tid, int npts, const double *x, int kind,
       if (rc) break;
     }
     if (t || resid || tmall) {
-      tbuf.resize((size_t)np * na * nout);
-      rc = ck(cudaMemcpyAsync(tbuf.data(), w.p.out, sizeof(double) * tbuf.size(),
+      // [npts][na][nout]: with one output this is every caller's layout
+      double *to = nout == 1 ? (tmall ? tmall : t) : nullptr;
+      if (to) {
+        to += (size_t)c0 * na;
+      } else {
+        tbuf.resize((size_t)np * na * nout);
+        to = tbuf.data();
+      }
+      rc = ck(cudaMemcpyAsync(to, w.p.out, sizeof(double) * (size_t)np * na * nout,
                               cudaMemcpyDeviceToHost, w.st), "D2H");
       if (!rc) rc = ck(cudaStreamSynchronize(w.st), "sync");
       if (rc) break;
-      if (tmall) relayout(tbuf.data(), tmall + (size_t)c0 * nout * na, np, na, nout, false);
-      std::vector<double> t1((size_t)np * na);
-      relayout(tbuf.data(), t1.data(), np, na, nout, true);
-      if (t) std::memcpy(t + (size_t)c0 * na, t1.data(), sizeof(double) * t1.size());
+      if (nout > 1) {
+        if (tmall) relayout(to, tmall + (size_t)c0 * nout * na, np, na, nout, false);
+        if (t) relayout(to, t + (size_t)c0 * na, np, na, nout, true);
+      } else if (t && tmall) {
+        std::memcpy(t + (size_t)c0 * na, to, sizeof(double) * (size_t)np * na);
+      }
       if (resid && rule) {
         const SeedRuleHost &r = rule->r;
         for (int p = 0; p < np; ++p) {
-          const double *tp = &t1[(size_t)p * na];
+          const double *tp = to + (size_t)p * na * nout;  // output 1: stride nout
           double R = 0.0;
-          for (size_t k = 0; k < r.coeff.size(); ++k)
-            R = r.nonlin[k] ? R + r.coeff[k] * tp[0] * tp[r.ind[k]] : R + r.coeff[k] * tp[r.ind[k]];
+          for (size_t k = 0; k < r.coeff.size(); ++k) {
+            const double v = tp[(size_t)r.ind[k] * nout];
+            R = r.nonlin[k] ? R + r.coeff[k] * tp[0] * v : R + r.coeff[k] * v;
+          }
           resid[c0 + p] = R;
         }
       }
     }
   }
-  double lv = 0.0;
-  if (!rc) rc = ck(cudaMemcpyAsync(&lv, dloss, sizeof(double), cudaMemcpyDeviceToHost, w.st), "D2H");
-  if (!rc) rc = ck(cudaStreamSynchronize(w.st), "train batch");
-  if (!rc) rc = gemm_tc_flag(&n.dn, w.st);
-  if (loss) *loss = lv;
-  if (dseed) cudaFree(dseed);
-  if (drows) cudaFree(drows);
-  if (dsrc) cudaFree(dsrc);
-  cudaFree(dloss);
+  double own = 0.0, *lv = pinned_page();
+  if (!lv) lv = &own;
+  else ++lv;  // the first word is the flag read's
+  if (!rc) rc = ck(cudaMemcpyAsync(lv, dloss, sizeof(double), cudaMemcpyDeviceToHost, w.st), "D2H");
+  // one wait for the work, the loss and the split path's error flag
+  if (!rc && n.prec == PREC_SPLIT) rc = gemm_tc_flag(&n.dn, w.st);
+  else if (!rc) rc = ck(cudaStreamSynchronize(w.st), "train batch");
+  if (loss) *loss = rc ? 0.0 : *lv;
   return rc;
 }
 
@@ -753,6 +821,7 @@ int dnnf90_net_set_layer(int nid, int l, const double *wrow) {
   if (bad_net(nid) || l < 2 || l > g_net[nid].nlayer || !wrow) return RC_BAD_ARG;
   NetH &n = g_net[nid];
   flush_for_net(nid);  // queued points were added under the old weights
+  if (int rc = host_weights(n)) return rc;
   size_t o = layer_off(n, l);
   std::memcpy(&n.w[o], wrow, sizeof(double) * n.dims[l - 1] * (n.dims[l - 2] + 1));
   n.wver++;
@@ -764,6 +833,7 @@ int dnnf90_net_free(int nid) {
   if (bad_net(nid)) return RC_BAD_ARG;
   comm_forget(nid, 0);
   NetH &n = g_net[nid];
+  if (n.wev) cudaEventDestroy(n.wev);
   n.dt.release();
   n.dn.release();
   scratch_trim();  // the scratch kept for calls on it goes back too
@@ -804,6 +874,7 @@ int dnnf90_eval(int nid, int wid, const double *x, double *t) {
   if (rc) return rc;
   NetH &n = g_net[nid];
   const int na = n.ts.na, nout = n.dims[n.nlayer - 1];
+  if (nout == 1) return run_eval(nid, g_wrk[wid], 1, x, t, true);
   std::vector<double> tm((size_t)na * nout);
   if ((rc = run_eval(nid, g_wrk[wid], 1, x, tm.data(), true))) return rc;
   for (int ia = 0; ia < na; ++ia) t[ia] = tm[(size_t)ia * nout];
@@ -818,9 +889,10 @@ int dnnf90_eval_batch(int nid, int wid, int npts, const double *x, double *t) {
   if (npts == 0) return RC_OK;
   NetH &n = g_net[nid];
   const int na = n.ts.na, nout = n.dims[n.nlayer - 1];
-  std::vector<double> tm((size_t)npts * na * nout);
-  if ((rc = run_eval(nid, g_wrk[wid], npts, x, tm.data(), true))) return rc;
-  relayout(tm.data(), t, npts, na, nout, true);
+  if (nout == 1) return run_eval(nid, g_wrk[wid], npts, x, t, true);
+  std::unique_ptr<double[]> tm(new double[(size_t)npts * na * nout]);
+  if ((rc = run_eval(nid, g_wrk[wid], npts, x, tm.get(), true))) return rc;
+  relayout(tm.get(), t, npts, na, nout, true);
   return RC_OK;
 }
 
@@ -832,9 +904,10 @@ int dnnf90_eval_batch_multi(int nid, int wid, int npts, const double *x, double 
   if (npts == 0) return RC_OK;
   NetH &n = g_net[nid];
   const int na = n.ts.na, nout = n.dims[n.nlayer - 1];
-  std::vector<double> tm((size_t)npts * na * nout);
-  if ((rc = run_eval(nid, g_wrk[wid], npts, x, tm.data(), true))) return rc;
-  relayout(tm.data(), tmo, npts, na, nout, false);
+  if (nout == 1) return run_eval(nid, g_wrk[wid], npts, x, tmo, true);
+  std::unique_ptr<double[]> tm(new double[(size_t)npts * na * nout]);
+  if ((rc = run_eval(nid, g_wrk[wid], npts, x, tm.get(), true))) return rc;
+  relayout(tm.get(), tmo, npts, na, nout, false);
   return RC_OK;
 }
 
@@ -899,7 +972,8 @@ int dnnf90_grad_zero(int gid) {
   for (int t = 1; t <= MAXH; ++t)  // zeroing discards what was queued
     if (g_twk[t].used && g_twk[t].qgid == gid) g_twk[t].qn = 0;
   GradH &g = g_grd[gid];
-  if (g.d) return ck(cudaMemset(g.d, 0, sizeof(double) * std::max(1, g.nw)), "grad_zero");
+  if (g.d)
+    return ck(cudaMemsetAsync(g.d, 0, sizeof(double) * std::max(1, g.nw), nullptr), "grad_zero");
   return RC_OK;
 }
 
@@ -940,17 +1014,18 @@ int dnnf90_adam_step(int nid, int gid, double eta, double beta1, double beta2,
   if (!g.m) {
     if ((rc = ck(cudaMalloc(&g.m, sizeof(double) * g.nw), "cudaMalloc"))) return rc;
     if ((rc = ck(cudaMalloc(&g.v, sizeof(double) * g.nw), "cudaMalloc"))) return rc;
-    cudaMemset(g.m, 0, sizeof(double) * g.nw);
-    cudaMemset(g.v, 0, sizeof(double) * g.nw);
+    cudaMemsetAsync(g.m, 0, sizeof(double) * g.nw, nullptr);
+    cudaMemsetAsync(g.v, 0, sizeof(double) * g.nw, nullptr);
   }
   if ((rc = adam_device(n.dn.w64, g.d, g.m, g.v, g.nw, eta, beta1, beta2, eps, nbatch,
                         istep, nullptr)))
     return rc;
-  if ((rc = ck(cudaMemcpy(n.w.data(), n.dn.w64, sizeof(double) * n.w.size(),
-                          cudaMemcpyDeviceToHost), "weights D2H")))
-    return rc;
-  n.wver++;  // the device FP32 / split copies follow on the next use
-  return RC_OK;
+  // the weights stay on the device; the host copy is fetched when it is asked
+  // for, the split operands follow on the next use
+  n.wver++;
+  n.dn.uploaded = n.wver;
+  n.host_stale = true;
+  return weights_written(n, nullptr);
 }
 
 // ------------------------------------------------------------- extensions
@@ -971,6 +1046,7 @@ int dnnf90_net_get_layer(int nid, int l, double *wrow) {
   std::lock_guard<std::recursive_mutex> lk(g_mu);
   if (bad_net(nid) || l < 2 || l > g_net[nid].nlayer || !wrow) return RC_BAD_ARG;
   NetH &n = g_net[nid];
+  if (int rc = host_weights(n)) return rc;
   std::memcpy(wrow, &n.w[layer_off(n, l)], sizeof(double) * n.dims[l - 1] * (n.dims[l - 2] + 1));
   return RC_OK;
 }
@@ -979,6 +1055,7 @@ int dnnf90_net_save(int nid, const char *filename) {
   std::lock_guard<std::recursive_mutex> lk(g_mu);
   if (bad_net(nid) || !filename) return RC_BAD_ARG;
   NetH &n = g_net[nid];
+  if (int rc = host_weights(n)) return rc;
   FILE *f = std::fopen(filename, "w");
   if (!f) return RC_BAD_FILE;
   std::fprintf(f, "0\nfunc %d\nActivation_out 0\n%d\n", n.ts.iact, n.nlayer);
@@ -1220,11 +1297,33 @@ int dnnf90_set_weights_dev(int nid, const double *w_dev, void *stream) {
   NetH &n = g_net[nid];
   flush_for_net(nid);
   cudaStream_t st = (cudaStream_t)stream;
-  if ((rc = ck(cudaMemcpyAsync(n.w.data(), w_dev, sizeof(double) * n.w.size(),
-                               cudaMemcpyDeviceToHost, st), "weights D2H")))
+  if (capturing(st)) {  // the call waits for st
+    set_error("dnnf90_set_weights_dev cannot be captured into a CUDA graph");
+    return RC_DEVICE;
+  }
+  if ((rc = net_buffers(n))) return rc;
+  if (n.wev_set && n.wst != st && (rc = ck(cudaStreamWaitEvent(st, n.wev, 0), "weights wait")))
     return rc;
-  if ((rc = ck(cudaStreamSynchronize(st), "sync"))) return rc;
-  n.wver++;
+  // the device copy is compared while it is replaced: equal weights keep
+  // their version, so that planes kept by a forward stay valid for the
+  // backward that sets the same weights again
+  int own = 1, *changed = (int *)pinned_page();
+  const bool first = n.dn.uploaded != n.wver || !changed;
+  if (first) {
+    changed = &own;
+    rc = ck(cudaMemcpyAsync(n.dn.w64, w_dev, sizeof(double) * n.w.size(),
+                            cudaMemcpyDeviceToDevice, st), "weights D2D");
+  } else {
+    *changed = 0;
+    rc = weights_set(n.dn.w64, w_dev, (int)n.w.size(), changed, st);
+  }
+  if (rc || (rc = ck(cudaStreamSynchronize(st), "sync"))) return rc;
+  if (*changed) {
+    n.wver++;
+    n.dn.uploaded = n.wver;
+    n.host_stale = true;
+    if ((rc = weights_written(n, st))) return rc;
+  }
   return net_device(n, st);
 }
 
@@ -1241,7 +1340,12 @@ int dnnf90_forward_dev(int nid, int tid, int npts, const double *x_dev, double *
   if ((rc = net_device(n, st))) return rc;
   if ((rc = work_planes(w, n, npts, keep != 0))) return rc;
   if (keep) {
+    w.kept = false;
     if ((rc = forward_keep(n.dt, n.dn, w.p, n.prec, npts, x_dev, tm_dev, st))) return rc;
+    // the points stay beside their planes, for the backward to compare
+    if ((rc = ck(cudaMemcpyAsync(w.p.X, x_dev, sizeof(double) * (size_t)npts * n.ts.d0,
+                                 cudaMemcpyDeviceToDevice, st), "points D2D")))
+      return rc;
     w.kept = true;
     w.kept_x = x_dev;
     w.kept_n = npts;
@@ -1261,7 +1365,8 @@ int dnnf90_keep_fits(int nid, int tid, int npts, int *fits) {
   if (rc) return rc;
   if (npts < 0 || !fits) return RC_BAD_ARG;
   if ((rc = device_ready())) return rc;
-  *fits = npts <= plane_cap(g_twk[tid], g_net[nid]) ? 1 : 0;
+  *fits = planes_hold(g_twk[tid], g_net[nid], npts) ||
+          npts <= plane_cap(g_twk[tid], g_net[nid]) ? 1 : 0;
   return RC_OK;
 }
 
@@ -1276,8 +1381,16 @@ int dnnf90_backward_dev(int nid, int tid, int npts, const double *x_dev,
   WorkH &w = g_twk[tid];
   cudaStream_t st = (cudaStream_t)stream;
   if ((rc = net_device(n, st))) return rc;
-  if (w.kept && w.kept_x == x_dev && w.kept_n == npts && w.kept_ver == n.wver &&
-      w.p.prec == n.prec)
+  bool kept = w.kept && w.kept_x == x_dev && w.kept_n == npts && w.kept_ver == n.wver &&
+              w.p.prec == n.prec;
+  if (int *differs = (int *)pinned_page(); kept && differs && !capturing(st)) {
+    *differs = 0;
+    if ((rc = same_values(w.p.X, x_dev, (size_t)npts * n.ts.d0, differs, st)) ||
+        (rc = ck(cudaStreamSynchronize(st), "sync")))
+      return rc;
+    kept = *differs == 0;
+  }
+  if (kept)
     return dev_finish(n, st,
                       adjoint_kept(n.dt, n.dn, w.p, n.prec, npts, x_dev, seedm_dev, grad_dev, st));
   // recompute mode: the forward runs again inside the adjoint
@@ -1764,6 +1877,7 @@ int dnnf90_kf_update_rows(int kid, int nobs, const double *rows, const double *x
   KfH &k = g_kf[kid];
   NetH &n = g_net[k.nid];
   flush_for_net(k.nid);  // queued points belong to the weights before the update
+  if ((rc = host_weights(n))) return rc;
   if (!k.st && (rc = ck(cudaStreamCreateWithFlags(&k.st, cudaStreamNonBlocking), "stream")))
     return rc;
   const size_t nw = n.w.size();
@@ -1848,6 +1962,7 @@ int kf_pass(int kid, int tid, int npts, const double *x, int rid, double rnoise,
   RuleH &rule = g_rule[rid];
   if ((rc = flush_queue(tid))) return rc;
   flush_for_net(nid);
+  if ((rc = host_weights(n))) return rc;  // what a failed pass falls back to
   if ((rc = work_stream(w))) return rc;
   if ((rc = net_device(n, w.st))) return rc;
   if ((rc = rule_device(rule, n))) return rc;
@@ -1899,7 +2014,11 @@ int kf_pass(int kid, int tid, int npts, const double *x, int rid, double rnoise,
                                    cudaMemcpyDeviceToHost, w.st), "D2H");
   KfState s;
   if (!rc) rc = kf_state(k.d, &s, w.st);
-  n.wver++;  // the host copy now holds what the device computed
+  n.wver++;  // both copies now hold what the device computed
+  if (!rc) {
+    n.dn.uploaded = n.wver;
+    rc = weights_written(n, w.st);
+  }
   return rc ? rc : kf_status_rc(s);
 }
 }  // namespace
@@ -1948,6 +2067,7 @@ int dnnf90_kf_pass_sys(int kid, int tid, int npts, const double *x, const double
   WorkH &w = g_twk[tid];
   if ((rc = flush_queue(tid))) return rc;
   flush_for_net(nid);
+  if ((rc = host_weights(n))) return rc;  // what a failed pass falls back to
   if ((rc = work_stream(w))) return rc;
   if ((rc = net_device(n, w.st))) return rc;
   if ((rc = rule_device(rule, n))) return rc;
@@ -2005,6 +2125,10 @@ int dnnf90_kf_pass_sys(int kid, int tid, int npts, const double *x, const double
   KfState s;
   if (!rc) rc = kf_state(k.d, &s, w.st);
   n.wver++;
+  if (!rc) {
+    n.dn.uploaded = n.wver;
+    rc = weights_written(n, w.st);
+  }
   return rc ? rc : kf_status_rc(s);
 }
 
@@ -2013,7 +2137,8 @@ int dnnf90_kf_iekf_begin(int kid) {
   int rc = kf_check(kid);
   if (rc) return rc;
   KfH &k = g_kf[kid];
-  const NetH &n = g_net[k.nid];
+  NetH &n = g_net[k.nid];
+  if ((rc = host_weights(n))) return rc;
   if ((rc = ck(cudaMemcpy(k.d.wprior, n.w.data(), n.w.size() * 8, cudaMemcpyHostToDevice),
                "H2D")))
     return rc;
@@ -2037,6 +2162,7 @@ int dnnf90_kf_iekf_iter(int kid, const double *row, double resid, double rnoise,
   }
   NetH &n = g_net[k.nid];
   flush_for_net(k.nid);
+  if ((rc = host_weights(n))) return rc;
   if (!k.st && (rc = ck(cudaStreamCreateWithFlags(&k.st, cudaStreamNonBlocking), "stream")))
     return rc;
   const size_t nw = n.w.size();

@@ -21,6 +21,7 @@
 #include "bell.hpp"
 #include "engine.hpp"
 #include "kernels.cuh"
+#include "scratch.hpp"
 
 namespace dnnf90 {
 
@@ -1412,11 +1413,7 @@ static int sm_count_b() {
 // device (occupancy of this kernel at this shared-memory size), at most one
 // per work item, so no block waits for a second wave
 static int persistent_grid(const void *k, int threads, size_t smem, long items) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
-  const long g = (long)grid_sms() * per_sm;
+  const long g = (long)grid_sms() * blocks_per_sm(k, threads, smem);
   return (int)std::max(1L, std::min(g, items));
 }
 

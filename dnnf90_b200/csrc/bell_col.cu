@@ -28,6 +28,7 @@
 #include "bell_col.hpp"
 #include "engine.hpp"
 #include "kernels.cuh"
+#include "scratch.hpp"
 
 namespace dnnf90 {
 
@@ -287,11 +288,7 @@ __global__ void __launch_bounds__(NT) k_bell_adj_col(ColArgs a) {
 }
 
 int resident_grid(const void *k, int threads, size_t smem) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
-  return grid_sms() * per_sm;
+  return grid_sms() * blocks_per_sm(k, threads, smem);
 }
 
 // ------------------------------------------------------------ first layer

@@ -28,6 +28,7 @@
 #include "bell.hpp"
 #include "engine.hpp"
 #include "kernels.cuh"
+#include "scratch.hpp"
 #include "tile_plan.hpp"
 
 namespace dnnf90 {
@@ -573,11 +574,7 @@ __global__ void __launch_bounds__(TWA * 32, 1) k_bell_adj10(Adj10Args a) {
 }
 
 int grid_for(const void *k, int threads, size_t smem, long items) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
-  const long g = (long)grid_sms() * per_sm;
+  const long g = (long)grid_sms() * blocks_per_sm(k, threads, smem);
   return (int)std::max(1L, std::min(g, items));
 }
 

@@ -22,6 +22,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <string>
 #include <type_traits>
@@ -161,6 +162,28 @@ void DevScratch::release() {
 void scratch_trim() {
   cudaMemPool_t pool = scratch_pool(false);
   if (pool) cudaMemPoolTrimTo(pool, 0);
+}
+double *pinned_page() {
+  static double *page = [] {
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, PIN_DOUBLES * sizeof(double),
+                      cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess)
+      p = nullptr;
+    return (double *)p;
+  }();
+  return page;
+}
+int blocks_per_sm(const void *k, int threads, size_t smem) {
+  static std::mutex mu;
+  static std::map<std::tuple<int, const void *, int, size_t>, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lk(mu);
+  int &n = known[{dev, k, threads, smem}];
+  if (n < 1 && (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k, threads, smem) != cudaSuccess ||
+                n < 1))
+    n = 1;
+  return n;
 }
 
 int device_ready() {
@@ -1409,11 +1432,7 @@ void set_grid_cap(int sms) { g_grid_cap = sms; }
 
 // blocks of k resident at once on the SMs a launch may fill
 static int occ_grid(const void *k, int threads, size_t smem) {
-  int per_sm = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, threads, smem) != cudaSuccess ||
-      per_sm < 1)
-    per_sm = 1;
-  return grid_sms() * per_sm;
+  return grid_sms() * blocks_per_sm(k, threads, smem);
 }
 
 template <typename R, int KK>
@@ -1831,6 +1850,32 @@ int adam_device(double *w, const double *g, double *m, double *v, int nw,
   }
   LAUNCH("k_adam", st, k_adam<<<std::max(1, std::min((nw + 255) / 256, 1024)), 256, 0, st>>>(
       w, g, m, v, nw, eta, b1, b2, eps, (double)nbatch, 1.0 - p1, 1.0 - p2));
+  CK(cudaGetLastError());
+  return RC_OK;
+}
+
+// w64 <- w, and *changed = 1 if any bit of it differed; and the comparison
+// alone
+__global__ void k_weights_set(double *w64, const double *w, int n, volatile int *changed) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double v = w[i];
+  if (__double_as_longlong(w64[i]) == __double_as_longlong(v)) return;
+  w64[i] = v;
+  *changed = 1;
+}
+__global__ void k_same(const double *a, const double *b, size_t n, volatile int *differs) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
+       i += (size_t)gridDim.x * blockDim.x)
+    if (__double_as_longlong(a[i]) != __double_as_longlong(b[i])) *differs = 1;
+}
+int weights_set(double *w64, const double *w, int n, int *changed, cudaStream_t st) {
+  LAUNCH("k_weights_set", st, k_weights_set<<<(n + 255) / 256, 256, 0, st>>>(w64, w, n, changed));
+  CK(cudaGetLastError());
+  return RC_OK;
+}
+int same_values(const double *a, const double *b, size_t n, int *differs, cudaStream_t st) {
+  LAUNCH("k_same", st, k_same<<<(int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 592)), 256, 0, st>>>(a, b, n, differs));
   CK(cudaGetLastError());
   return RC_OK;
 }

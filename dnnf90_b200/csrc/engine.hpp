@@ -107,7 +107,8 @@ struct DevNet {
                              // rewritten before each use (gemm_f64.cu)
   float *w32 = nullptr;      // FP32 copy for the split path
   void *tc = nullptr;        // pre-split tensor-core weight operands
-  uint64_t uploaded = 0;     // host weight version on the device
+  uint64_t uploaded = 0;     // weight version in w64
+  uint64_t derived = 0;      // weight version in w32 and tc
   void release();
 };
 
@@ -180,6 +181,12 @@ int forward_keep(const DevTables &t, const DevNet &n, Planes &p, int prec,
 int adjoint_kept(const DevTables &t, const DevNet &n, Planes &p, int prec,
                  int npts, const double *X, const double *seed, double *grad,
                  cudaStream_t st);
+
+// w64 <- w (device arrays of n doubles), *changed = 1 if any bit differed;
+// *differs = 1 if two arrays differ in any bit.  The flags are device-visible
+// host memory the caller has cleared.
+int weights_set(double *w64, const double *w, int n, int *changed, cudaStream_t st);
+int same_values(const double *a, const double *b, size_t n, int *differs, cudaStream_t st);
 
 // Adam update on the device (opt_adam_step, lib/train_module.f90:656-683);
 // m and v are allocated by the caller and zero on the first call

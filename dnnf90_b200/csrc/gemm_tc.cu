@@ -40,6 +40,7 @@
 
 #include "engine.hpp"
 #include "gemm_tc.hpp"
+#include "scratch.hpp"
 
 namespace dnnf90 {
 
@@ -750,54 +751,45 @@ __global__ void __launch_bounds__(DW_NTH, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, 512;" ::"r"(tmem) : "memory");
 }
 
-// host-side split of one FP32 value into three bf16 terms (round to nearest
-// even, as __float2bfloat16_rn)
-static uint16_t bf16_rn(float f) {
-  uint32_t u;
-  std::memcpy(&u, &f, 4);
-  if ((u & 0x7fffffffu) > 0x7f800000u) return (uint16_t)((u >> 16) | 0x40);
-  uint32_t r = u + 0x7fffu + ((u >> 16) & 1u);
-  return (uint16_t)(r >> 16);
-}
-static float bf16_f(uint16_t h) {
-  uint32_t u = (uint32_t)h << 16;
-  float f;
-  std::memcpy(&f, &u, 4);
-  return f;
-}
-static size_t kmaj_off_h(int row, int k) {
-  return (size_t)((row >> 3) * 1024 + (row & 7) * ROWB + ((((k >> 3) ^ (row & 7)) & 7) << 4) +
-                  (k & 7) * 2);
-}
-
-// pre-split weights of one GEMM: Bmat(nrow = N, k = K) element source
-// fn(n, k), laid out [N tile][term][K block][BN rows][128 B]
-template <typename F>
-static std::vector<uint8_t> prep_b(int N, int K, int BN, F fn) {
-  const int nkb = (K + BK - 1) / BK, ntn = (N + BN - 1) / BN;
+// The pre-split weight operands of one layer W[n][m + 1] (bias first): FWD's
+// B(row j, k = i) and DT's B(row i, k = j), value (float)W[j][1 + i] as three
+// bf16 terms, laid out [N tile][term][K block][BN rows][128 B] (swizzled);
+// fwd or dt null: not used.  The padding past N and K is zeroed once.
+struct PrepArgs {
+  const double *W;
+  int n, m, bnf, bnd;
+  uint8_t *fwd, *dt;
+  float *bias;
+};
+__device__ __forceinline__ void put_terms(uint8_t *out, int BN, int K, int row, int k,
+                                          const __nv_bfloat16 (&h)[3]) {
+  const int nkb = (K + BK - 1) / BK, tn = row / BN, r = row - tn * BN;
   const size_t btile = (size_t)BN * ROWB;
-  std::vector<uint8_t> out((size_t)ntn * 3 * nkb * btile, 0);
-  for (int tn = 0; tn < ntn; ++tn)
-    for (int r = 0; r < BN; ++r) {
-      const int n = tn * BN + r;
-      if (n >= N) continue;
-      for (int k = 0; k < K; ++k) {
-        float x = fn(n, k);
-        uint16_t h1 = bf16_rn(x);
-        float rr = x - bf16_f(h1);
-        uint16_t h2 = bf16_rn(rr);
-        rr = rr - bf16_f(h2);
-        uint16_t h3 = bf16_rn(rr);
-        const int kb = k / BK, kk = k % BK;
-        const uint16_t hs[3] = {h1, h2, h3};
-        for (int p = 0; p < 3; ++p) {
-          size_t off = (size_t)tn * 3 * nkb * btile + ((size_t)p * nkb + kb) * btile +
-                       kmaj_off_h(r, kk);
-          std::memcpy(&out[off], &hs[p], 2);
-        }
-      }
-    }
-  return out;
+#pragma unroll
+  for (int p = 0; p < 3; ++p)
+    *(__nv_bfloat16 *)(out + (size_t)tn * 3 * nkb * btile +
+                       ((size_t)p * nkb + k / BK) * btile + kmaj_off(r, k % BK)) = h[p];
+}
+__global__ void k_prep_weights(PrepArgs a) {
+  const int e = blockIdx.x * blockDim.x + threadIdx.x;
+  if (e >= a.n * a.m) return;
+  const int j = e / a.m, i = e - j * a.m;
+  const double *w = a.W + (size_t)j * (a.m + 1);
+  const float x = (float)w[1 + i];
+  __nv_bfloat16 h[3];
+  h[0] = __float2bfloat16_rn(x);
+  float r = x - __bfloat162float(h[0]);
+  h[1] = __float2bfloat16_rn(r);
+  r = r - __bfloat162float(h[1]);
+  h[2] = __float2bfloat16_rn(r);
+  if (a.fwd) {
+    put_terms(a.fwd, a.bnf, a.m, j, i, h);
+    if (i == 0) a.bias[j] = (float)w[0];
+  }
+  if (a.dt) put_terms(a.dt, a.bnd, a.n, i, j, h);
+}
+static size_t prep_bytes(int N, int K, int BN) {
+  return (size_t)((N + BN - 1) / BN) * 3 * ((K + BK - 1) / BK) * BN * ROWB;
 }
 
 }  // namespace tc
@@ -854,8 +846,8 @@ static int tc_bn(int N, int K) {
 // Pre-split weights of a network.  The buffers are allocated on the first
 // call and rewritten in place afterwards (a network's shapes never change),
 // so kernels captured in a graph keep valid weight addresses across weight
-// updates.  The copies are ordered on st and complete before the return.
-int gemm_tc_prepare(DevNet *net, const double *hw, cudaStream_t st) {
+// updates.  Ordered on st, from the network's FP64 device weights.
+int gemm_tc_prepare(DevNet *net, cudaStream_t st) {
   if (!gemm_tc_available()) return RC_OK;
   TcWeights *w = (TcWeights *)net->tc;
   const int L = net->nlayer;
@@ -872,25 +864,30 @@ int gemm_tc_prepare(DevNet *net, const double *hw, cudaStream_t st) {
   }
   for (int l = 3; l < L; ++l) {  // hidden layers with a GEMM
     const int n = net->dims[l - 1], m = net->dims[l - 2];
-    const double *Wl = hw + net->woff[l - 1];
-    if (const int BN = tc_bn(n, m)) {
-      auto b = tc::prep_b(n, m, BN, [&](int j, int k) { return (float)Wl[(size_t)j * (m + 1) + 1 + k]; });
-      if (!w->fwd[l - 1]) CKT(cudaMalloc(&w->fwd[l - 1], b.size()));
-      CKT(cudaMemcpyAsync(w->fwd[l - 1], b.data(), b.size(), cudaMemcpyHostToDevice, st));
-      std::vector<float> bias(n);
-      for (int j = 0; j < n; ++j) bias[j] = (float)Wl[(size_t)j * (m + 1)];
+    tc::PrepArgs a{net->w64 + net->woff[l - 1], n, m, tc_bn(n, m), tc_bn(m, n), nullptr, nullptr,
+                   nullptr};
+    auto place = [&](uint8_t *&buf, size_t bytes) -> int {
+      if (buf) return RC_OK;
+      CKT(cudaMalloc(&buf, bytes));
+      CKT(cudaMemsetAsync(buf, 0, bytes, st));
+      return RC_OK;
+    };
+    int rc;
+    if (a.bnf) {
+      if ((rc = place(w->fwd[l - 1], tc::prep_bytes(n, m, a.bnf)))) return rc;
       if (!w->bias[l - 1]) CKT(cudaMalloc(&w->bias[l - 1], n * sizeof(float)));
-      CKT(cudaMemcpyAsync(w->bias[l - 1], bias.data(), n * sizeof(float), cudaMemcpyHostToDevice, st));
-      w->bn_fwd[l - 1] = BN;
-      CKT(cudaStreamSynchronize(st));  // b and bias leave scope
+      a.fwd = w->fwd[l - 1];
+      a.bias = w->bias[l - 1];
+      w->bn_fwd[l - 1] = a.bnf;
     }
-    if (const int BN = tc_bn(m, n)) {
-      auto b = tc::prep_b(m, n, BN, [&](int i, int j) { return (float)Wl[(size_t)j * (m + 1) + 1 + i]; });
-      if (!w->dt[l - 1]) CKT(cudaMalloc(&w->dt[l - 1], b.size()));
-      CKT(cudaMemcpyAsync(w->dt[l - 1], b.data(), b.size(), cudaMemcpyHostToDevice, st));
-      w->bn_dt[l - 1] = BN;
-      CKT(cudaStreamSynchronize(st));
+    if (a.bnd) {
+      if ((rc = place(w->dt[l - 1], tc::prep_bytes(m, n, a.bnd)))) return rc;
+      a.dt = w->dt[l - 1];
+      w->bn_dt[l - 1] = a.bnd;
     }
+    if (!a.fwd && !a.dt) continue;
+    LAUNCH("k_prep_weights", st, (tc::k_prep_weights<<<(n * m + 255) / 256, 256, 0, st>>>(a)));
+    CKT(cudaGetLastError());
   }
   return RC_OK;
 }
@@ -1106,14 +1103,16 @@ int gemm_tc_syrk(const float *J, int nrow, int nw, int ldj, double *G, cudaStrea
 int gemm_tc_flag(const DevNet *net, cudaStream_t st) {
   TcWeights *w = (TcWeights *)net->tc;
   if (!w) return RC_OK;
-  int h = 0;
-  CKT(cudaMemcpyAsync(&h, w->flag, sizeof(int), cudaMemcpyDeviceToHost, st));
+  int own = 0, *h = (int *)pinned_page();
+  if (!h) h = &own;
+  CKT(cudaMemcpyAsync(h, w->flag, sizeof(int), cudaMemcpyDeviceToHost, st));
   CKT(cudaStreamSynchronize(st));
-  if (h) {
+  if (*h) {
+    const int code = *h;
     // report once, then clear, so that the next call runs afresh
     cudaMemsetAsync(w->flag, 0, sizeof(int), st);
     cudaStreamSynchronize(st);
-    set_error("tensor-core GEMM: an mbarrier wait timed out (code " + std::to_string(h) + ")");
+    set_error("tensor-core GEMM: an mbarrier wait timed out (code " + std::to_string(code) + ")");
     return RC_DEVICE;
   }
   return RC_OK;

@@ -19,8 +19,8 @@ struct DevNet;
 bool gemm_tc_available();
 void gemm_tc_release_weights(DevNet *net);
 // Pre-splits and pre-swizzles the weight operands of every hidden layer
-// from the host weights hw (flat layer layout).
-int gemm_tc_prepare(DevNet *net, const double *hw, cudaStream_t st);
+// from its FP64 device weights.
+int gemm_tc_prepare(DevNet *net, cudaStream_t st);
 // Reads the wait time-out flag of the network's tensor-core GEMMs
 // (synchronises st); RC_DEVICE if a wait ran out.
 int gemm_tc_flag(const DevNet *net, cudaStream_t st);
@@ -32,10 +32,9 @@ int gemm_tc_dt(const DevNet *net, int l, int M, int n, int m, const void *Sb,
 int gemm_tc_dw(const DevNet *net, int l, int M, int n, int m, const void *Sb,
                const void *Tm, double *G, cudaStream_t st);
 
-// G[i][j] += sum_r J[r][i] J[r][j] on the lower triangle (FP64 G), J in FP64
-// rows carried as three bf16 terms on the tensor cores
-// G[i][j] += sum_r J[r][i] J[r][j] from an FP32 copy J[nrow][ldj] (ldj a
-// multiple of 4, columns nw..ldj-1 zero), G [nw][nw] FP64; synchronises st
+// G[i][j] += sum_r J[r][i] J[r][j], j <= i, from an FP32 copy J[nrow][ldj]
+// (ldj a multiple of 16, columns nw..ldj-1 zero), carried as three bf16 terms
+// on the tensor cores, G [nw][nw] FP64; synchronises st
 int gemm_tc_syrk(const float *J, int nrow, int nw, int ldj, double *G, cudaStream_t st);
 
 int weights_to_f32(const double *w, float *w32, size_t n, cudaStream_t st);

@@ -38,4 +38,14 @@ class DevScratch {
 // returns what the current device's pool holds unused
 void scratch_trim();
 
+// One page of pinned, device-mapped host memory of the process, through
+// which calls read small results back without a staged copy.  Its users hold
+// the library's lock from the write to the read.  Null if it cannot be had.
+constexpr int PIN_DOUBLES = 64;
+double *pinned_page();
+
+// resident blocks of kernel k per SM, asked of the runtime once per (device,
+// kernel, threads, shared memory): the query costs more than a launch
+int blocks_per_sm(const void *k, int threads, size_t smem);
+
 }  // namespace dnnf90
