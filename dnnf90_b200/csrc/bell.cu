@@ -60,6 +60,7 @@ void DevBellPlan::release() {
   for (void *p : ps)
     if (p) cudaFree(p);
   tile.release();
+  tile64.release();
   col.release();
   *this = DevBellPlan();
 }
@@ -186,6 +187,7 @@ int upload_bell_plan(const TableSet &t, DevBellPlan &d) {
   d.nrows = P.nrows;
   d.dt_off = P.dt_off;
   if ((rc = upload_tile_plan(t, d.tile))) return rc;
+  if ((rc = upload_tile64_plan(t, d.tile64))) return rc;
   if ((rc = upload_col(t, d.col))) return rc;
   d.ready = true;
   return RC_OK;
@@ -1596,12 +1598,15 @@ static int fwd5_dispatch(const DevBellPlan &bp, const DevTables &t, int n, int n
   }
   // variant 0: records in global memory; 1: records in shared memory;
   // 2: v8 (lean per-degree loops over 16-bit offset records); 3: the
-  // register-tiled Horner forward (bell_tile.cu; FP32, dense sets), the
-  // default wherever it applies
+  // register-tiled Horner forward (bell_tile.cu, in FP64 bell_tile64.cu;
+  // dense sets), the default wherever it applies
   const bool srec_fits = smem + (size_t)bp.nrec32 * 4 <= 227 * 1024;
   const bool v8_ok = bp.f8.ok && bp.f8.smem <= 227 * 1024;
-  const bool tile_ok = sizeof(R) == 4 && tile_fwd_applies(bp.tile, n);
+  const bool tile_ok =
+      sizeof(R) == 4 ? tile_fwd_applies(bp.tile, n) : tile64_fwd_applies(bp.tile64, n);
   auto launch = [&](int v, bool) -> int {
+    if (v == 3 && sizeof(R) == 8)
+      return bell_fwd_tile64(bp.tile64, t, n, npts, S, T, h, train, st);
     if (v == 3) return bell_fwd_tile(bp.tile, t, n, npts, S, T, h, train, st);
     if (v == 2) {
       Fwd8Args b;
@@ -1747,10 +1752,12 @@ static int adj2_t(const DevBellPlan &bp, const DevTables &t, int n, int npts, co
       CKB(cudaGetLastError());
       return RC_OK;
     };
-    // variant 3: the register-tiled correlation (bell_tile.cu; FP32, dense
-    // sets).  Every variant that applies is timed; the default is the tiled
+    // variant 3: the register-tiled correlation (bell_tile.cu, in FP64
+    // bell_tile64.cu; dense sets).  Every variant that applies is timed; the default is the tiled
     // kernel where it applies, else v7, else the last that applies
     auto launch_t = [&](int v, bool last) -> int {
+      if (v == 3 && sizeof(R) == 8)
+        return bell_adj_tile64(bp.tile64, n, npts, Tb, h, Sb, last ? gbias : nullptr, gstride, st);
       if (v == 3)
         return bell_adj_tile(bp.tile, n, npts, Tb, h, Sb, last ? gbias : nullptr, gstride, st);
       return launch_all(v, last);
@@ -1758,7 +1765,8 @@ static int adj2_t(const DevBellPlan &bp, const DevTables &t, int n, int npts, co
     std::vector<int> ids{0};
     if (srec_fits) ids.push_back(1);
     if (v7_fits) ids.push_back(2);
-    if (sizeof(R) == 4 && tile_adj_applies(bp.tile, n)) ids.push_back(3);
+    if (sizeof(R) == 4 ? tile_adj_applies(bp.tile, n) : tile64_adj_applies(bp.tile64, n))
+      ids.push_back(3);
     int dflt = (int)ids.size() - 1;
     if (v7_fits && ids.back() != 3) dflt = srec_fits ? 2 : 1;
     return tuned_ids(TuneKey{bp.id, 2, n, (int)sizeof(R), t.d0, t.k, t.na}, ids, dflt,

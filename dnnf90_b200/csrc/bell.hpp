@@ -33,6 +33,22 @@ struct TileDev {
   void release();
 };
 
+// the same for the FP64 kernels (bell_tile64.cu)
+struct Tile64Dev {
+  bool f_ok = false, a_ok = false;
+  int td = 0, k = 0, na = 0;
+  int nfunit = 0, nfrec = 0, naunit = 0, narec = 0, nafin = 0, nzero = 0;
+  int *flist = nullptr, *funit = nullptr, *alist = nullptr, *aunit = nullptr;
+  int *aflist = nullptr, *afin = nullptr, *perm = nullptr, *rowslot = nullptr;
+  uint32_t *frec = nullptr, *arec = nullptr;
+  double *fact = nullptr, *ifact = nullptr;
+  int f_o_d0 = 0, f_o_d1 = 0, f_o_sig = 0, f_o_list = 0, f_o_unit = 0, f_o_rec = 0;
+  int f_o_perm = 0, f_o_rowslot = 0, f_o_fact = 0, f_o_ifact = 0, f_smem = 0;
+  int a_o_scr = 0, a_o_zero = 0, a_o_list = 0, a_o_flist = 0, a_o_unit = 0, a_o_fin = 0;
+  int a_o_rec = 0, a_o_perm = 0, a_o_rowslot = 0, a_o_fact = 0, a_o_ifact = 0, a_smem = 0;
+  void release();
+};
+
 struct DevBellPlan {
   bool ready = false;
   uint64_t id = 0;              // distinct per upload (autotuner key)
@@ -84,6 +100,7 @@ struct DevBellPlan {
     bool ok = false;
   } f9;
   TileDev tile;            // register-tiled kernels (dense sets, FP32)
+  Tile64Dev tile64;        // the same in FP64
   ColDev col;              // column kernels (small sets)
   double *sc64 = nullptr;  // [3][na]: a!, 1/a!, 1/a! (Tb, h, Sb scales)
   float *sc32 = nullptr;
@@ -116,6 +133,14 @@ int bell_fwd_tile(const TileDev &d, const DevTables &t, int n, int npts, const v
                   void *h, bool train, cudaStream_t st);
 int bell_adj_tile(const TileDev &d, int n, int npts, const void *Tb, const void *h, void *Sb,
                   double *gbias, int gstride, cudaStream_t st);
+// and in FP64 (bell_tile64.cu): dense sets with K <= 7, n even
+int upload_tile64_plan(const TableSet &t, Tile64Dev &d);
+bool tile64_fwd_applies(const Tile64Dev &d, int n);
+bool tile64_adj_applies(const Tile64Dev &d, int n);
+int bell_fwd_tile64(const Tile64Dev &d, const DevTables &t, int n, int npts, const void *S,
+                    void *T, void *h, bool train, cudaStream_t st);
+int bell_adj_tile64(const Tile64Dev &d, int n, int npts, const void *Tb, const void *h, void *Sb,
+                    double *gbias, int gstride, cudaStream_t st);
 // The first hidden layer is analytic: h^g = s^(|g|+1)(S^0) W^g.  With these
 // inputs the adjoint (bell_adj_l2a) forms h itself (graded slots) from the
 // s^(q) the forward kept, and reads no h plane.

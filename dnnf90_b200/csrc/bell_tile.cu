@@ -26,6 +26,7 @@
 #include <vector>
 
 #include "bell.hpp"
+#include "bell_tile.cuh"
 #include "engine.hpp"
 #include "kernels.cuh"
 #include "scratch.hpp"
@@ -36,41 +37,6 @@ namespace dnnf90 {
 namespace {
 
 constexpr int TWF = TILE_WARPS_F, TWA = TILE_WARPS_A;
-
-// ------------------------------------------------------------ tile algebra
-// entries of a tile of side L in td dimensions, and the graded index maps
-__host__ __device__ constexpr int tsize(int td, int L) { return td == 2 ? L * (L + 1) / 2 : L; }
-__host__ __device__ constexpr int tdeg(int td, int e) {
-  int s = 0;
-  if (td == 1) return e;
-  while ((s + 1) * (s + 2) / 2 <= e) ++s;
-  return s;
-}
-__host__ __device__ constexpr int tsecond(int td, int e) {
-  return td == 1 ? 0 : e - tdeg(2, e) * (tdeg(2, e) + 1) / 2;
-}
-__host__ __device__ constexpr int tfirst(int td, int e) {
-  return td == 1 ? e : tdeg(2, e) - tsecond(2, e);
-}
-__host__ __device__ constexpr int tindex(int td, int a1, int a2) {
-  return td == 1 ? a1 : (a1 + a2) * (a1 + a2 + 1) / 2 + a2;
-}
-// index of the sum of entries e and c
-__host__ __device__ constexpr int tadd(int td, int e, int c) {
-  return tindex(td, tfirst(td, e) + tfirst(td, c), tsecond(td, e) + tsecond(td, c));
-}
-
-__device__ __forceinline__ uint32_t smem_addr(const void *p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void cp16(void *dst, const void *src, int src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_addr(dst)), "l"(src),
-               "r"(src_bytes)
-               : "memory");
-}
-__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
 
 // Rows of a [na][n] plane slice (neurons j0 .. j0+31) into shared rows
 // perm[r] of dst (128 bytes each), 16-byte pieces; columns at or beyond n
@@ -85,19 +51,6 @@ __device__ __forceinline__ void stage_perm(unsigned char *dst, const float *src,
     const int ok = col < n ? 16 : 0;
     cp16(dst + perm[r] * 128 + piece * 16, src + (size_t)r * n + (ok ? col : 0), ok);
   }
-}
-
-// copy of n 32-bit words of a table into shared memory
-__device__ __forceinline__ void copy_words(void *dst, const void *src, int nwords) {
-  for (int i = threadIdx.x; i < nwords; i += blockDim.x)
-    ((uint32_t *)dst)[i] = __ldg((const uint32_t *)src + i);
-}
-
-// items [it0, it1) of this block: a contiguous share of npts * gy items,
-// item = point + npts * (32-neuron tile)
-__device__ __forceinline__ void block_items(long nitem, long &it0, long &it1) {
-  it0 = (long)blockIdx.x * nitem / gridDim.x;
-  it1 = (long)(blockIdx.x + 1) * nitem / gridDim.x;
 }
 
 // ------------------------------------------------------------ forward
@@ -572,34 +525,6 @@ __global__ void __launch_bounds__(TWA * 32, 1) k_bell_adj10(Adj10Args a) {
   flush(gb, gj, -1);
   flush(gbp, gjp, -1);
 }
-
-int grid_for(const void *k, int threads, size_t smem, long items) {
-  const long g = (long)grid_sms() * blocks_per_sm(k, threads, smem);
-  return (int)std::max(1L, std::min(g, items));
-}
-
-template <typename T>
-int put_vec(T **d, const std::vector<T> &h) {
-  if (h.empty()) return RC_OK;
-  if (cudaMalloc(d, h.size() * sizeof(T)) != cudaSuccess) {
-    set_error("device allocation failed (tile plan)");
-    return RC_NOMEM;
-  }
-  if (cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) {
-    set_error("copy to the device failed (tile plan)");
-    return RC_DEVICE;
-  }
-  return RC_OK;
-}
-
-#define CKT(x)                                                         \
-  do {                                                                 \
-    cudaError_t e_ = (x);                                              \
-    if (e_ != cudaSuccess) {                                           \
-      set_error(std::string("bell_tile: ") + cudaGetErrorString(e_));  \
-      return RC_DEVICE;                                                \
-    }                                                                  \
-  } while (0)
 
 }  // namespace
 

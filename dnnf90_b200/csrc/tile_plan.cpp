@@ -342,4 +342,160 @@ TilePlan build_tile_plan(const TableSet &t, int fwarps, int awarps) {
   return P;
 }
 
+static TileAdj64 adj64_ways(const TilePlan &P, int warps, int ways) {
+  TileAdj64 A;
+  const int td = P.td, K = P.k, dout = P.d0 - td;
+  const auto outer = outer_indices(dout, K);
+  std::map<std::vector<int>, int> oidx;
+  for (size_t i = 0; i < outer.size(); ++i) oidx[outer[i]] = (int)i;
+  // records of an output tile by E = degree of eps, in outer order
+  auto records = [&](int o, std::vector<std::vector<uint32_t>> &byE) {
+    const int gd = deg_of(outer[o]);
+    byE.assign(K - gd + 1, {});
+    for (size_t o2 = 0; o2 < outer.size(); ++o2) {
+      const int E = deg_of(outer[o2]);
+      if (gd + E > K) continue;
+      std::vector<int> sum(dout);
+      for (int j = 0; j < dout; ++j) sum[j] = outer[o][j] + outer[o2][j];
+      byE[E].push_back((uint32_t)P.tbase[o2] | (uint32_t)P.tbase[oidx.at(sum)] << 14 |
+                       (uint32_t)(K - gd - E + 1) << 28);
+    }
+  };
+  struct Step {
+    uint32_t a, b;
+    int E;
+    long cost;
+  };
+  struct U {
+    int lo, pair, outA, outB;
+    std::vector<Step> st;
+    long cost = 0;
+  };
+  std::vector<U> us;
+  for (int g = 0; g <= K; ++g) {
+    std::vector<int> tiles;
+    for (size_t o = 0; o < outer.size(); ++o)
+      if (deg_of(outer[o]) == g) tiles.push_back((int)o);
+    const int lo = K - g + 1;
+    for (size_t i = 0; i < tiles.size(); i += 2) {
+      U u;
+      u.lo = lo;
+      u.pair = i + 1 < tiles.size();
+      u.outA = P.tbase[tiles[i]];
+      u.outB = u.pair ? P.tbase[tiles[i + 1]] : u.outA;
+      std::vector<std::vector<uint32_t>> ra, rb;
+      records(tiles[i], ra);
+      if (u.pair) records(tiles[i + 1], rb);
+      for (int E = 0; E < (int)ra.size(); ++E) {
+        const long c = tile_pairs(td, lo - E) + 2 * tile_size(td, lo - E) + 40;
+        if (u.pair) {
+          if (ra[E].size() != rb[E].size()) return TileAdj64();
+          for (size_t r = 0; r < ra[E].size(); ++r) u.st.push_back({ra[E][r], rb[E][r], E, c});
+        } else {
+          for (size_t r = 0; r < ra[E].size(); r += 2)
+            u.st.push_back({ra[E][r], r + 1 < ra[E].size() ? ra[E][r + 1] : ra[E][r] | TILE_NULL, E, c});
+        }
+      }
+      for (auto &x : u.st) {
+        u.cost += x.cost;
+        A.steps_fma += tile_pairs(td, lo - x.E);
+      }
+      us.push_back(std::move(u));
+    }
+  }
+  long total = 0, maxstep = 0;
+  for (auto &u : us) {
+    total += u.cost;
+    for (auto &x : u.st) maxstep = std::max(maxstep, x.cost);
+  }
+  const long cap = std::max(maxstep, (total + ways - 1) / ways);
+  struct Part {
+    int lo, pair, scr, s0, s1, u, rowA, rowB;
+    long cost;
+  };
+  std::vector<Part> parts;
+  std::vector<int> elems;
+  for (size_t i = 0; i < us.size(); ++i) {
+    const U &u = us[i];
+    const int ns = (int)u.st.size(), nt = tile_size(td, u.lo);
+    // steps of one E in a part are counted in 4 bits
+    if (u.cost <= cap || ways <= 1) {
+      parts.push_back({u.lo, u.pair, 0, 0, ns, (int)i, u.outA, u.outB, u.cost});
+      continue;
+    }
+    const int np = (int)((u.cost + cap - 1) / cap);
+    const long share = (u.cost + np - 1) / np;
+    const int first = A.nscratch;
+    int start = 0, made = 0;
+    long acc = 0;
+    for (int q = 0; q < ns; ++q) {
+      acc += u.st[q].cost;
+      const bool last = q + 1 == ns;
+      if (last || (acc >= share && made < np - 1)) {
+        parts.push_back({u.lo, u.pair, 1, start, q + 1, (int)i, A.nscratch, A.nscratch + nt, acc});
+        A.nscratch += (u.pair ? 2 : 1) * nt;
+        start = q + 1;
+        acc = 0;
+        ++made;
+      }
+    }
+    const int stride = (u.pair ? 2 : 1) * nt;
+    for (int h = 0; h < (u.pair ? 2 : 1); ++h)
+      for (int e = 0; e < nt; ++e) {
+        elems.push_back((h ? u.outB : u.outA) + e);
+        elems.push_back(made);
+        elems.push_back(first + h * nt + e);
+        elems.push_back(stride);
+      }
+  }
+  std::vector<long> cost;
+  for (auto &p : parts) cost.push_back(p.cost + ADJ_UNIT_COST / 2);
+  const auto own = lpt(cost, warps);
+  A.list.assign((size_t)warps * 2, 0);
+  for (int w = 0; w < warps; ++w) {
+    A.list[w * 2] = (int)A.unit.size() / 8;
+    int cnt = 0;
+    for (size_t i = 0; i < parts.size(); ++i) {
+      if (own[i] != w) continue;
+      const Part &p = parts[i];
+      uint32_t cw = 0;
+      const int first = (int)A.rec.size() / 2;
+      for (int q = p.s0; q < p.s1; ++q) {
+        const Step &x = us[p.u].st[q];
+        if (x.E > 7 || ((cw >> (4 * x.E)) & 15u) == 15u) return TileAdj64();
+        cw += 1u << (4 * x.E);
+        A.rec.push_back(x.a);
+        A.rec.push_back(x.b);
+      }
+      const int f[8] = {p.lo | p.pair << 8 | p.scr << 9, first, (int)cw, p.rowA, p.rowB, 0, 0, 0};
+      A.unit.insert(A.unit.end(), f, f + 8);
+      ++cnt;
+    }
+    A.list[w * 2 + 1] = cnt;
+  }
+  A.flist.assign((size_t)warps * 2, 0);
+  const int nfin = (int)elems.size() / 4;
+  for (int w = 0; w < warps; ++w) {
+    A.flist[w * 2] = (int)A.fin.size() / 4;
+    int cnt = 0;
+    for (int f = w; f < nfin; f += warps) {
+      A.fin.insert(A.fin.end(), elems.begin() + 4 * f, elems.begin() + 4 * f + 4);
+      ++cnt;
+    }
+    A.flist[w * 2 + 1] = cnt;
+  }
+  A.ok = true;
+  return A;
+}
+
+TileAdj64 build_tile_adj64(const TableSet &t, const TilePlan &P, int warps, int max_scratch) {
+  (void)t;
+  if (!P.ok || warps < 1) return TileAdj64();
+  for (int ways = warps; ways >= 1; --ways) {
+    TileAdj64 A = adj64_ways(P, warps, ways);
+    if (A.ok && A.nscratch <= max_scratch) return A;
+  }
+  return TileAdj64();
+}
+
 }  // namespace dnnf90

@@ -41,6 +41,10 @@ namespace dnnf90 {
 constexpr int TILE_WARPS_F = 16;
 constexpr int TILE_WARPS_A = 16;
 constexpr int TILE_KMAX = 7;    // longest tile side is K + 1 <= 8
+// FP64: a tile's registers are twice as wide, so twelve warps of at most 168
+// registers (three to each quarter of the SM)
+constexpr int TILE_WARPS64_F = 12;
+constexpr int TILE_WARPS64_A = 12;
 
 struct TilePlan {
   bool ok = false;
@@ -75,6 +79,30 @@ struct TilePlan {
 // The plan of a dense table set with 1 <= K <= TILE_KMAX (ok = false
 // otherwise, and the caller keeps the general kernels).
 TilePlan build_tile_plan(const TableSet &t, int fwarps, int awarps);
+
+// Adjoint work lists of the FP64 kernel, in the row layout of a TilePlan.
+// Its rows are 16 neurons, and the two half-warps run two records of the same
+// tile side at a time (a step): of two output tiles of one degree (a pair:
+// every tile of a degree has the same record sides), or, for the odd tile of
+// a degree, the even and the odd records of each side, whose sums the halves
+// exchange at the end.  A missing odd record is its neighbour with a factor
+// tile of zeros (TILE_NULL).
+constexpr uint32_t TILE_NULL = 1u << 13;
+struct TileAdj64 {
+  bool ok = false;
+  std::vector<int> list;        // [warps][2]: first unit, units
+  std::vector<int> unit;        // [*][8]: Lout | pair << 8 | scratch << 9, first step,
+                                //   step counts (4 bits per E as in TilePlan), output or
+                                //   scratch row of half 0, of half 1 (pairs), 0, 0, 0
+  std::vector<uint32_t> rec;    // [steps][2]: h row | Tb row << 14 | L << 28
+  std::vector<int> fin;         // [*][4] as TilePlan::afin
+  std::vector<int> flist;       // [warps][2] into fin
+  int nscratch = 0;             // scratch rows
+  long steps_fma = 0;           // multiply-adds of all steps (diagnostic)
+};
+// at most max_scratch scratch rows (the output tiles are split over warps as
+// far as that allows)
+TileAdj64 build_tile_adj64(const TableSet &t, const TilePlan &P, int warps, int max_scratch);
 
 // entries of a tile of side L
 inline int tile_size(int td, int L) { return td == 2 ? L * (L + 1) / 2 : L; }

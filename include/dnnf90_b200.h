@@ -257,10 +257,9 @@ int dnnf90_tune_report(char *buf, int len);
  * 1 records in shared memory, 2 per-degree loops over 16-bit offset records)
  * or adjoint (which 1: 0 pairs in global memory, 1 in shared memory,
  * 2 grouped correlation) kernels, or (either) 3 the register-tiled kernels
- * of dense sets in FP32, 4 the one-thread-per-neuron kernels of small sets
- * (these run by rule, without a timed trial), for every later launch;
- * variant -1 hands
- * the choice back to the autotuner, and a variant a launch shape cannot use
+ * of dense sets (both precisions), 4 the one-thread-per-neuron kernels of
+ * small sets (these run by rule, without a timed trial), for every later
+ * launch; variant -1 hands the choice back to the autotuner, and a variant a launch shape cannot use
  * runs its default.  which 2 switches the tanh forward by the series
  * identity tanh' = 1 - tanh^2 (for tanh on sets closed under b <= a whose
  * state fits shared memory): 1 on, 0 or -1 off (the default; the Bell
