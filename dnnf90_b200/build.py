@@ -17,7 +17,8 @@ LIBDIR = os.path.join(HERE, "_lib")
 LIB = os.path.join(LIBDIR, "libdnnf90_b200.so")
 
 SOURCES = ["tables.cpp", "bell_plan.cpp", "tile_plan.cpp", "api.cpp", "engine.cu", "bell.cu",
-           "bell_tile.cu", "bell_tile64.cu", "bell_col.cu", "gemm_tc.cu", "gemm_f64.cu", "ngd.cu", "kalman.cu"]
+           "bell_tile.cu", "bell_tile64.cu", "bell_col.cu", "point.cu",
+           "gemm_tc.cu", "gemm_f64.cu", "ngd.cu", "kalman.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVFLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
            "--expt-relaxed-constexpr", "-Xcompiler", "-Wall"]

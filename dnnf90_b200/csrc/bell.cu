@@ -62,6 +62,7 @@ void DevBellPlan::release() {
   tile.release();
   tile64.release();
   col.release();
+  point.release();
   *this = DevBellPlan();
 }
 
@@ -189,6 +190,7 @@ int upload_bell_plan(const TableSet &t, DevBellPlan &d) {
   if ((rc = upload_tile_plan(t, d.tile))) return rc;
   if ((rc = upload_tile64_plan(t, d.tile64))) return rc;
   if ((rc = upload_col(t, d.col))) return rc;
+  if ((rc = upload_point(t, d.point))) return rc;
   d.ready = true;
   return RC_OK;
 }
@@ -1483,6 +1485,8 @@ int tune_force(int which, int variant) {
   g_force[which] = variant;
   return RC_OK;
 }
+
+bool tune_pinned() { return g_force[0] >= 0 || g_force[1] >= 0 || g_series_fwd; }
 
 // the column kernels (bell_col.cu) run wherever they apply unless another
 // variant is pinned

@@ -6,6 +6,7 @@
 
 #include "bell_col.hpp"
 #include "bell_plan.hpp"
+#include "point.hpp"
 
 namespace dnnf90 {
 
@@ -102,6 +103,7 @@ struct DevBellPlan {
   TileDev tile;            // register-tiled kernels (dense sets, FP32)
   Tile64Dev tile64;        // the same in FP64
   ColDev col;              // column kernels (small sets)
+  PointDev point;          // one launch for a small network's step
   double *sc64 = nullptr;  // [3][na]: a!, 1/a!, 1/a! (Tb, h, Sb scales)
   float *sc32 = nullptr;
   void release();
@@ -116,6 +118,8 @@ std::string tune_report();
 // series forward: 1 on wherever it applies, 0 or -1 off (the default: the
 // Bell recurrence everywhere).
 int tune_force(int which, int variant);
+// whether a Bell variant is pinned or the series forward is on
+bool tune_pinned();
 
 // RC_UNSUPPORTED when the set does not fit (K > 8 or the per-point state
 // exceeds shared memory): the caller then uses the generic kernels.

@@ -1787,6 +1787,8 @@ int run_batch(const DevTables &t, const DevNet &net, const DevRule &rule,
     set_error("Jacobian rows requested without a row buffer");
     return RC_BAD_ARG;
   }
+  if (point_applies(t, net, rule, a.npts, a.train, a.prec))
+    return run_point(t, net, rule, a, st);
   return a.prec == PREC_F64 ? run_all<double>(t, net, rule, p, a, st)
                             : run_all<float>(t, net, rule, p, a, st);
 }
