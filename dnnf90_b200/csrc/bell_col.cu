@@ -21,8 +21,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
-#include <map>
 #include <string>
+#include <unordered_map>
 
 #include "bell.hpp"
 #include "bell_col.hpp"
@@ -46,23 +46,23 @@ ColProg build_col_prog(const TableSet &t) {
   ColProg P;
   const int na = t.na, d0 = t.d0;
   for (int a = 0; a < na; ++a) P.kt = std::max(P.kt, t.deg[a]);
-  std::map<std::vector<int>, int> at;
-  std::vector<std::vector<int>> al(na);
+  // a multi-index as one word, four bits a component (K <= 15, D0 <= 16): no
+  // component of a - b borrows from the next when b <= a
+  std::unordered_map<uint64_t, int> at;
+  std::vector<uint64_t> key(na, 0);
+  at.reserve(2 * na);
   for (int a = 0; a < na; ++a) {
-    al[a].assign(t.alpha.begin() + (size_t)a * d0, t.alpha.begin() + (size_t)(a + 1) * d0);
-    at[al[a]] = a;
+    for (int i = 0; i < d0; ++i) key[a] |= (uint64_t)t.alpha[(size_t)a * d0 + i] << (4 * i);
+    at[key[a]] = a;
   }
   std::vector<std::vector<uint32_t>> f(na), adj(na);
-  std::vector<int> g(d0);
   for (int a = 0; a < na; ++a)
     for (int b = 0; b < na; ++b) {
-      bool le = true;
-      for (int i = 0; i < d0; ++i) {
-        g[i] = al[a][i] - al[b][i];
-        if (g[i] < 0) le = false;
-      }
+      bool le = t.deg[b] <= t.deg[a];
+      const int *x = &t.alpha[(size_t)a * d0], *y = &t.alpha[(size_t)b * d0];
+      for (int i = 0; le && i < d0; ++i) le = y[i] <= x[i];
       if (!le) continue;
-      const int ig = at.at(g);  // the set is downward closed
+      const int ig = at.at(key[a] - key[b]);  // the set is downward closed
       if (b != 0 && b == a) f[a].insert(f[a].begin(), (uint32_t)b);
       else if (b != 0) f[a].push_back((uint32_t)b | ((uint32_t)ig << 16));
       adj[b].push_back((uint32_t)a | ((uint32_t)ig << 16));
@@ -659,7 +659,7 @@ constexpr long COL_THREADS = 8192;
 
 int upload_col(const TableSet &t, ColDev &d) {
   d.release();
-  if (t.na > COL_MAX) return RC_OK;
+  if (t.na > COL_MAX || t.d0 > D0MAX) return RC_OK;
   const ColProg P = build_col_prog(t);
   int rc;
   if ((rc = put_col(&d.fhdr, P.fhdr)) || (rc = put_col(&d.ahdr, P.ahdr)) ||

@@ -638,24 +638,26 @@ int upload_point(const TableSet &t, PointDev &d) {
       al.assign(t.alpha.begin() + (size_t)a * t.d0, t.alpha.begin() + (size_t)(a + 1) * t.d0);
       if (al[i]-- > 0) dn[(size_t)a * t.d0 + i] = (short)t.find(al.data());
     }
-  const size_t nf = p.frec.size(), nad = p.arec.size();
-  CKP(cudaMalloc(&d.base, (size_t)t.na * 16 + (nf + nad + t.na) * 4 + dn.size() * 2));
-  char *q = (char *)d.base;
-  auto put = [&](const void *src, size_t bytes) {
-    void *at = q;
-    q += bytes;
-    return cudaMemcpy(at, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess ? at : nullptr;
+  // one block of memory: headers, records, exponents, neighbours
+  std::vector<unsigned char> all;
+  auto add = [&](const void *src, size_t bytes) {
+    const size_t at = all.size();
+    all.insert(all.end(), (const unsigned char *)src, (const unsigned char *)src + bytes);
+    return at;
   };
-  d.fhdr = (int2 *)put(p.fhdr.data(), (size_t)t.na * 8);
-  d.ahdr = (int2 *)put(p.ahdr.data(), (size_t)t.na * 8);
-  d.frec = (uint32_t *)put(p.frec.data(), nf * 4);  // both of even length
-  d.arec = (uint32_t *)put(p.arec.data(), nad * 4);
-  d.ex = (uint32_t *)put(ex.data(), (size_t)t.na * 4);
-  d.dn = (short *)put(dn.data(), dn.size() * 2);
-  if (!d.dn || !d.fhdr || !d.ahdr || !d.frec || !d.arec || !d.ex) {
-    set_error("point: table copy failed");
-    return RC_DEVICE;
-  }
+  const size_t fh = add(p.fhdr.data(), (size_t)t.na * 8), ah = add(p.ahdr.data(), (size_t)t.na * 8);
+  const size_t fr = add(p.frec.data(), p.frec.size() * 4);  // both of even length
+  const size_t ar = add(p.arec.data(), p.arec.size() * 4);
+  const size_t xo = add(ex.data(), (size_t)t.na * 4), no = add(dn.data(), dn.size() * 2);
+  CKP(cudaMalloc(&d.base, all.size()));
+  CKP(cudaMemcpy(d.base, all.data(), all.size(), cudaMemcpyHostToDevice));
+  char *q = (char *)d.base;
+  d.fhdr = (int2 *)(q + fh);
+  d.ahdr = (int2 *)(q + ah);
+  d.frec = (uint32_t *)(q + fr);
+  d.arec = (uint32_t *)(q + ar);
+  d.ex = (uint32_t *)(q + xo);
+  d.dn = (short *)(q + no);
   d.ok = true;
   return RC_OK;
 }
