@@ -134,10 +134,11 @@ __device__ __forceinline__ void fwd_unit(const FwdCtx &c, int4 u, int q, float i
     const uint32_t r = c.rec[u.y];
     tile_fwd<TD, L, true>(c.S + (r & 0xffffu) * 32, c.Dr + (r >> 16) * 32, acc);
   }
-  int i = u.y + 1;
   const int end = u.y + u.z;
-  for (; i < end; ++i) {
-    const uint32_t r = c.rec[i];
+  uint32_t rn = c.rec[u.y + 1];  // a record ahead (past the last: the next table's word)
+  for (int i = u.y + 1; i < end; ++i) {
+    const uint32_t r = rn;
+    rn = c.rec[i + 1];
     tile_fwd<TD, L, false>(c.S + (r & 0xffffu) * 32, c.Dr + (r >> 16) * 32, acc);
   }
   const float2 iv = make_float2(inv, inv);

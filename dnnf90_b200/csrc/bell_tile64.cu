@@ -126,8 +126,10 @@ __device__ __forceinline__ void fwd_unit(const FwdCtx &c, int4 u, int q, double 
     tile_fwd<TD, L, true>(c.S + (r & 0xffffu) * NPB, c.Dr + (r >> 16) * 32, acc);
   }
   const int end = u.y + u.z;
+  uint32_t rn = c.rec[u.y + 1];  // a record ahead (past the last: the next table's word)
   for (int i = u.y + 1; i < end; ++i) {
-    const uint32_t r = c.rec[i];
+    const uint32_t r = rn;
+    rn = c.rec[i + 1];
     tile_fwd<TD, L, false>(c.S + (r & 0xffffu) * NPB, c.Dr + (r >> 16) * 32, acc);
   }
 #pragma unroll
