@@ -17,8 +17,8 @@
 // Bound: issue and latency (ncu, 1184 points of 128 neurons: 35 % of issue
 // slots, FP64 pipe 19 % in the forward and 11 % in the adjoint; 46 K warp
 // instructions per item, 10.6 K of them multiply-adds).  One launch over 8191
-// points of 128 neurons at D0 = 4, K = 7: forward 7.8 ms against 15.1 for v8,
-// adjoint 4.7 against 7.8 for v7 (bell.cu), which gather one operand per
+// points of 128 neurons at D0 = 4, K = 7: forward 7.1 ms (7.8 before its
+// records were read one ahead) against 15.1 for v8, adjoint 4.7 against 7.8 for v7 (bell.cu), which gather one operand per
 // multiply-add.
 #include <cuda_runtime.h>
 

@@ -1054,7 +1054,9 @@ __global__ void __launch_bounds__(256, VEC ? 3 : 1) k_output_fwdv(OutArgs a) {
 // Adjoint of the output layer, one warp per point (see k_output_adj):
 // Tb_{L-1}^a[i] = sum_o W_L[o][1+i] seed[o][a], dW_L[o][1+i] += sum_a
 // seed[o][a] T_{L-1}^a[i].  Lane i + 32 t holds neuron i + 32 t, t < NT.
-template <typename R, int MAXO, int NT>
+// RED: the block's warps are summed in shared memory before the atomics
+// (outadjv_k says when).
+template <typename R, int MAXO, int NT, bool RED>
 __global__ void __launch_bounds__(256) k_output_adjv(OutAdjArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int m = a.m, na = a.na, nout = a.nout;
@@ -1080,22 +1082,57 @@ __global__ void __launch_bounds__(256) k_output_adjv(OutAdjArgs a) {
     for (int o = 0; o < MAXO; ++o)
 #pragma unroll
       for (int t = 0; t < NT; ++t) pg[o][t] = 0.0;
+    if constexpr (RED) {
+      // U slots at a time, their loads ahead of their stores
+      constexpr int U = NT <= 4 ? 2 : 1;
+      for (int ia0 = 0; ia0 < na; ia0 += U) {
+        R tv[U][NT];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            const int i = lane + 32 * t;
+            tv[u][t] = i < m && ia0 + u < na ? __ldg(Tm + (size_t)(ia0 + u) * m + i) : (R)0;
+          }
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+          const int ia = ia0 + u;
+          if (ia >= na) break;
+          double so[MAXO];
+#pragma unroll
+          for (int o = 0; o < MAXO; ++o) so[o] = o < nout ? __ldg(sd + o * na + ia) : 0.0;
+#pragma unroll
+          for (int t = 0; t < NT; ++t) {
+            const int i = lane + 32 * t;
+            if (i < m) {
+              double tb = 0.0;
+#pragma unroll
+              for (int o = 0; o < MAXO; ++o) tb += w[o][t] * so[o];
+              Tb[(size_t)ia * m + i] = (R)tb;
+#pragma unroll
+              for (int o = 0; o < MAXO; ++o) pg[o][t] += so[o] * (double)tv[u][t];
+            }
+          }
+        }
+      }
+    } else {
 #pragma unroll 2
-    for (int ia = 0; ia < na; ++ia) {
-      double so[MAXO];
+      for (int ia = 0; ia < na; ++ia) {
+        double so[MAXO];
 #pragma unroll
-      for (int o = 0; o < MAXO; ++o) so[o] = o < nout ? __ldg(sd + o * na + ia) : 0.0;
+        for (int o = 0; o < MAXO; ++o) so[o] = o < nout ? __ldg(sd + o * na + ia) : 0.0;
 #pragma unroll
-      for (int t = 0; t < NT; ++t) {
-        const int i = lane + 32 * t;
-        if (i < m) {
-          double tb = 0.0;
+        for (int t = 0; t < NT; ++t) {
+          const int i = lane + 32 * t;
+          if (i < m) {
+            double tb = 0.0;
 #pragma unroll
-          for (int o = 0; o < MAXO; ++o) tb += w[o][t] * so[o];
-          Tb[(size_t)ia * m + i] = (R)tb;
-          const double tv = (double)Tm[(size_t)ia * m + i];
+            for (int o = 0; o < MAXO; ++o) tb += w[o][t] * so[o];
+            Tb[(size_t)ia * m + i] = (R)tb;
+            const double tv = (double)Tm[(size_t)ia * m + i];
 #pragma unroll
-          for (int o = 0; o < MAXO; ++o) pg[o][t] += so[o] * tv;
+            for (int o = 0; o < MAXO; ++o) pg[o][t] += so[o] * tv;
+          }
         }
       }
     }
@@ -1119,23 +1156,31 @@ __global__ void __launch_bounds__(256) k_output_adjv(OutAdjArgs a) {
     }
   }
   if (a.rows || !a.g) return;
-  // the block's warps first, in turn, through shared memory: thousands of
-  // warps adding to the same few lines took most of a launch with few slots
-  // (16384 points of 5 slots x 64 neurons: 57 -> 23 us)
-  __shared__ double part[8][32 * NT + 1];
+  if constexpr (RED) {
+    __shared__ double part[8][32 * NT + 1];
 #pragma unroll
-  for (int o = 0; o < MAXO; ++o) {
-    if (o >= nout) break;
-    __syncthreads();
+    for (int o = 0; o < MAXO; ++o) {
+      if (o >= nout) break;
+      __syncthreads();
 #pragma unroll
-    for (int t = 0; t < NT; ++t) part[warp][1 + lane + 32 * t] = acc[o][t];
-    if (lane == 0) part[warp][0] = acc0[o];
-    __syncthreads();
-    for (int i = threadIdx.x; i <= m; i += blockDim.x) {
-      double v = 0.0;
-      for (int x = 0; x < nw; ++x) v += part[x][i];
-      atomicAdd(a.g + (size_t)o * (m + 1) + i, v);
+      for (int t = 0; t < NT; ++t) part[warp][1 + lane + 32 * t] = acc[o][t];
+      if (lane == 0) part[warp][0] = acc0[o];
+      __syncthreads();
+      for (int i = threadIdx.x; i <= m; i += blockDim.x) {
+        double v = 0.0;
+        for (int x = 0; x < nw; ++x) v += part[x][i];
+        atomicAdd(a.g + (size_t)o * (m + 1) + i, v);
+      }
     }
+  } else {
+#pragma unroll
+    for (int o = 0; o < MAXO; ++o)
+      if (o < nout) {
+#pragma unroll
+        for (int t = 0; t < NT; ++t)
+          if (lane + 32 * t < m) atomicAdd(a.g + (size_t)o * (m + 1) + 1 + lane + 32 * t, acc[o][t]);
+        if (lane == 0) atomicAdd(a.g + (size_t)o * (m + 1), acc0[o]);
+      }
   }
 }
 
@@ -1538,13 +1583,25 @@ static int launch_output_fwdv(const OutArgs &o, cudaStream_t st) {
   return RC_OK;
 }
 
-template <typename R, int NO, int NT>
-static int outadjv_k(const OutAdjArgs &o, cudaStream_t st) {
-  const void *k = (const void *)k_output_adjv<R, NO, NT>;
+// Where a warp has little to read, the atomics of the gradient take most of
+// the launch (thousands of warps adding to the same few lines), and a block's
+// warps are summed first: 16384 points of 5 slots x 64 neurons 57 -> 20 us in
+// FP64, 61 -> 21 in FP32.  FP32 warps with much to read lose by it (32768
+// points of 330 slots x 128: 2.0 ms without, 3.2 with); in FP64 the two are
+// level there (0.92 ms at 8191 points).
+template <typename R, int NO, int NT, bool RED>
+static int outadjv_launch(const OutAdjArgs &o, cudaStream_t st) {
+  const void *k = (const void *)k_output_adjv<R, NO, NT, RED>;
   const int grid = std::max(1, std::min((o.npts + 7) / 8, occ_grid(k, 256, 0)));
-  LAUNCH("k_output_adj", st, (k_output_adjv<R, NO, NT><<<grid, 256, 0, st>>>(o)));
+  LAUNCH("k_output_adj", st, (k_output_adjv<R, NO, NT, RED><<<grid, 256, 0, st>>>(o)));
   CK(cudaGetLastError());
   return RC_OK;
+}
+template <typename R, int NO, int NT>
+static int outadjv_k(const OutAdjArgs &o, cudaStream_t st) {
+  const long rows = (long)o.npts * o.na;  // the line: about 300 rows a resident warp
+  return sizeof(R) == 8 || rows <= (1L << 20) ? outadjv_launch<R, NO, NT, true>(o, st)
+                                              : outadjv_launch<R, NO, NT, false>(o, st);
 }
 
 template <typename R, int NO>
