@@ -620,6 +620,13 @@ size_t layout(const DevTables &t, const DevNet &net, bool train, PointArgs &a) {
   return (size_t)cur * sizeof(double);
 }
 
+// blocks of 512 threads an SM holds (0 after an error)
+int point_blocks(size_t smem) {
+  if (cudaFuncSetAttribute(k_point<512>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM))
+    return 0;
+  return blocks_per_sm((const void *)k_point<512>, 512, smem);
+}
+
 }  // namespace
 
 int upload_point(const TableSet &t, PointDev &d) {
@@ -690,13 +697,10 @@ bool point_applies(const DevTables &t, const DevNet &net, const DevRule &rule, i
     return false;
   PointArgs a;
   const size_t smem = layout(t, net, train, a);
-  const auto attr = cudaFuncAttributeMaxDynamicSharedMemorySize;
-  if (smem > PT_SMEM || cudaFuncSetAttribute(k_point<512>, attr, PT_SMEM) ||
-      cudaFuncSetAttribute(k_point<1024>, attr, PT_SMEM))
-    return false;
-  const int per = blocks_per_sm((const void *)k_point<512>, 512, smem);
-  const long most = H == 1 || per < 2 ? 3 : t.na > 36 ? 16 : 8;
-  return npts <= most * grid_sms();
+  if (smem > PT_SMEM) return false;
+  if (npts <= 3L * grid_sms()) return true;
+  const int per = point_blocks(smem);
+  return H > 1 && per >= 2 && npts <= (t.na > 36 ? 16L : 8L) * grid_sms();
 }
 
 int run_point(const DevTables &t, const DevNet &net, const DevRule &rule, const BatchArgs &b,
@@ -725,11 +729,11 @@ int run_point(const DevTables &t, const DevNet &net, const DevRule &rule, const 
     a.sfac = rule.sfac;
   }
   if (b.npts <= grid_sms()) {
+    CKP(cudaFuncSetAttribute(k_point<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, PT_SMEM));
     LAUNCH("k_point", st, (k_point<1024><<<b.npts, 1024, smem, st>>>(a)));
   } else {
-    const int per = blocks_per_sm((const void *)k_point<512>, 512, smem);
-    LAUNCH("k_point", st,
-           (k_point<512><<<std::min(b.npts, grid_sms() * per), 512, smem, st>>>(a)));
+    const int grid = std::min(b.npts, grid_sms() * std::max(1, point_blocks(smem)));
+    LAUNCH("k_point", st, (k_point<512><<<grid, 512, smem, st>>>(a)));
   }
   CKP(cudaGetLastError());
   return RC_OK;
