@@ -521,17 +521,20 @@ def kalman_bench(args):
     prof = api.profile_read()
     api.profile_enable(False)
     hbm, _, src = peaks()
-    tl_n, tl_ms = prof.get("k_kf_tiles", (0, 0.0))
+    # a grouped call passes over the triangle once per eight updates
+    name = "k_kf_gtiles" if "k_kf_gtiles" in prof else "k_kf_tiles"
+    tl_n, tl_ms = prof.get(name, (0, 0.0))
     roof = None
     if tl_n:
         per = tl_ms / tl_n
         alg = kf_packed_elems(nw) * 8 * 2        # packed triangles read and written once
         ach = alg / (per * 1e-3) / 1e9
-        roof = {"bound": "hbm", "kernel": "k_kf_tiles", "achieved": ach, "peak": hbm,
+        roof = {"bound": "hbm", "kernel": name, "achieved": ach, "peak": hbm,
                 "unit": "GB/s", "frac": ach / hbm, "peak_source": src,
                 "alg_bytes_per_launch": alg, "launch_ms": per, "traffic": None,
-                "note": "one launch applies one update: the upper triangle of P read and "
-                        "written once, the products with the next row formed in the same read"}
+                "note": "one launch applies one update (k_kf_tiles) or up to eight "
+                        "(k_kf_gtiles; a call's first launch only reads): the upper triangle of "
+                        "P read and written once, the next rows' products formed in the same read"}
     cpu = (kf_cpu_baseline(max(1, min(2000, int(1.5e8 / kf_packed_elems(nw)))))
            if (rank == 0 and ws == 1) else None)
     if rank == 0:
@@ -695,12 +698,12 @@ def ngd_bench(args):
     api.profile_enable(False)
     prof = api.profile_read()
     _, tc, src = peaks()
-    gram_n, gram_ms = prof.get("k_tc_gemm_dw", (0, 0.0))
+    gram_n, gram_ms = prof.get("k_tc_syrk", (0, 0.0))
     roof = None
     if gram_n:
         flops = 2.0 * npts * nw * (nw + 1) / 2       # the lower triangle of J^T J
         ach = flops / (gram_ms / gram_n * 1e-3) / 1e12
-        roof = {"bound": "tensor", "kernel": "k_tc_gemm_dw (J^T J)", "achieved": ach, "peak": tc,
+        roof = {"bound": "tensor", "kernel": "k_tc_syrk (J^T J)", "achieved": ach, "peak": tc,
                 "unit": "TFLOP/s", "frac": ach / tc, "peak_source": src, "traffic": None,
                 "useful_flops_per_launch": flops, "launch_ms": gram_ms / gram_n,
                 "note": "useful flops of the lower triangle; the split products run 6 bf16 "
