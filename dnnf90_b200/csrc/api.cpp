@@ -1989,6 +1989,8 @@ int kf_pass(int kid, int tid, int npts, const double *x, int rid, double rnoise,
   a.loss = dloss;
   a.train = true;
   a.prec = PREC_F64;
+  a.xi = dxi;  // the innovation -R, or R itself for the iterated update
+  a.xi_sign = niter > 0 ? 1.0 : -1.0;
   if (niter > 0 &&
       (rc = ck(cudaMemsetAsync(&k.d.st->status, 0, sizeof(int), w.st), "status reset")))
     return rc;
@@ -1996,7 +1998,6 @@ int kf_pass(int kid, int tid, int npts, const double *x, int rid, double rnoise,
     a.X = dX + (size_t)p * d0;
     if (niter == 0) {
       if ((rc = run_batch(n.dt, n.dn, rule.d, w.p, a, w.st))) break;
-      if ((rc = kf_resid_xi(rule.d, w.p.out, nout, dxi, w.st))) break;
       rc = kf_run(k.d, 1, drow, nw, dxi, dsc, n.dn.w64, w.st, p, false, true);
       continue;
     }
@@ -2005,7 +2006,6 @@ int kf_pass(int kid, int tid, int npts, const double *x, int rid, double rnoise,
       break;
     for (int it = 0; it < niter && !rc; ++it) {
       if ((rc = run_batch(n.dt, n.dn, rule.d, w.p, a, w.st))) break;
-      if ((rc = kf_resid_xi(rule.d, w.p.out, nout, dxi, w.st, 1.0))) break;  // R itself
       rc = kf_iekf(k.d, drow, dxi, dsc, n.dn.w64, it == niter - 1, w.st, p, false);
     }
   }

@@ -1854,10 +1854,16 @@ int run_batch(const DevTables &t, const DevNet &net, const DevRule &rule,
     set_error("Jacobian rows requested without a row buffer");
     return RC_BAD_ARG;
   }
+  if (a.xi && (a.npts != 1 || rule.kind != SEED_JROW || !a.out)) {
+    set_error("a residual is formed beside one point's Jacobian row");
+    return RC_BAD_ARG;
+  }
   if (point_applies(t, net, rule, a.npts, a.train, a.prec))
     return run_point(t, net, rule, a, st);
-  return a.prec == PREC_F64 ? run_all<double>(t, net, rule, p, a, st)
-                            : run_all<float>(t, net, rule, p, a, st);
+  const int rc = a.prec == PREC_F64 ? run_all<double>(t, net, rule, p, a, st)
+                                    : run_all<float>(t, net, rule, p, a, st);
+  return rc || !a.xi ? rc
+                     : kf_resid_xi(rule, a.out, net.dims[net.nlayer - 1], a.xi, st, a.xi_sign);
 }
 
 // Forward of npts <= cap points keeping every plane (for a later

@@ -151,6 +151,9 @@ struct BatchArgs {
   double *loss = nullptr;
   bool train = false;
   int prec = PREC_F64;
+  // one point under a Jacobian-row rule: xi[0] = xi_sign * R beside its row
+  double *xi = nullptr;
+  double xi_sign = 1.0;
 };
 
 // device-side seed rule

@@ -71,7 +71,8 @@ struct PointArgs {
   const int2 *fhdr, *ahdr;
   const uint32_t *frec, *arec, *ex;
   const short *dn;
-  double *out, *grad, *rows, *loss;
+  double *out, *grad, *rows, *loss, *xi;
+  double xi_sign;
   int kind, nterm, nres;
   double fac;
   const double *coeff, *wres;
@@ -302,6 +303,7 @@ __device__ double point_seed(const PointArgs &a, const double *tl, double *sd, i
     else R0 = R0 + a.coeff[t] * tl[ind];
   }
   double Rs = R0, fac = a.fac, l = 0.0;
+  if (a.xi) *a.xi = a.xi_sign * R0;  // one point's residual (see k_kf_resid)
   if (a.kind == SEED_JROW) { Rs = 1.0; fac = 1.0; }
   else l = 0.5 * a.fac * R0 * R0;
   for (int t = 0; t < a.nterm; ++t) {
@@ -724,6 +726,7 @@ int run_point(const DevTables &t, const DevNet &net, const DevRule &rule, const 
     a.rows = rule.kind == SEED_JROW ? b.rows : nullptr;
     a.grad = a.rows ? nullptr : b.grad;
     a.loss = rule.kind == SEED_GIVEN || rule.kind == SEED_JROW ? nullptr : b.loss;
+    a.xi = b.xi; a.xi_sign = b.xi_sign;
     a.nterm = rule.nterm; a.nres = rule.nres; a.fac = rule.fac; a.coeff = rule.coeff;
     a.wres = rule.wres; a.ind = rule.ind; a.nonlin = rule.nonlin; a.sys = rule.sys;
     a.sfac = rule.sfac;
