@@ -59,8 +59,9 @@ struct WorkH {
   Planes p;
   cudaStream_t st = nullptr;
   int chunk = 0;
-  // planes kept by a keep=1 forward
-  bool kept = false;
+  // planes kept by a keep=1 forward; kept_graph: one that was captured into a
+  // graph, which an eager backward does not build on (it may not have run)
+  bool kept = false, kept_graph = false;
   const double *kept_x = nullptr;
   int kept_n = 0;
   uint64_t kept_ver = 0;
@@ -300,6 +301,15 @@ int work_planes(WorkH &w, NetH &n, int want, bool exact) {
   if (w.p.base && w.p.prec == n.prec && w.p.cap_pts >= need) return RC_OK;
   w.kept = false;
   return ensure_planes(n.dt, n.dn, n.prec, std::max(need, 1), w.p);
+}
+
+// The run that follows on st rewrites w's planes.  One that is captured
+// rewrites them on every replay too, long after this call, and leaves its
+// mark beside them then (Planes::dirty).
+int planes_taken(WorkH &w, cudaStream_t st) {
+  w.kept = false;
+  if (!capturing(st)) return RC_OK;
+  return ck(cudaMemsetAsync(w.p.dirty, 1, sizeof(int), st), "planes mark");
 }
 
 int grad_alloc(GradH &g) {
@@ -1339,20 +1349,18 @@ int dnnf90_forward_dev(int nid, int tid, int npts, const double *x_dev, double *
   cudaStream_t st = (cudaStream_t)stream;
   if ((rc = net_device(n, st))) return rc;
   if ((rc = work_planes(w, n, npts, keep != 0))) return rc;
+  if ((rc = planes_taken(w, st))) return rc;
   if (keep) {
-    w.kept = false;
     if ((rc = forward_keep(n.dt, n.dn, w.p, n.prec, npts, x_dev, tm_dev, st))) return rc;
-    // the points stay beside their planes, for the backward to compare
-    if ((rc = ck(cudaMemcpyAsync(w.p.X, x_dev, sizeof(double) * (size_t)npts * n.ts.d0,
-                                 cudaMemcpyDeviceToDevice, st), "points D2D")))
-      return rc;
+    // the points stay beside their planes, for an eager backward to compare
+    w.kept_graph = capturing(st);
+    if (!w.kept_graph && (rc = keep_points(w.p, x_dev, (size_t)npts * n.ts.d0, st))) return rc;
     w.kept = true;
     w.kept_x = x_dev;
     w.kept_n = npts;
     w.kept_ver = n.wver;
     return dev_finish(n, st, RC_OK);
   }
-  w.kept = false;
   DevRule none;
   BatchArgs a;
   a.npts = npts; a.X = x_dev; a.out = tm_dev; a.prec = n.prec;
@@ -1383,19 +1391,23 @@ int dnnf90_backward_dev(int nid, int tid, int npts, const double *x_dev,
   if ((rc = net_device(n, st))) return rc;
   bool kept = w.kept && w.kept_x == x_dev && w.kept_n == npts && w.kept_ver == n.wver &&
               w.p.prec == n.prec;
-  if (int *differs = (int *)pinned_page(); kept && differs && !capturing(st)) {
-    *differs = 0;
-    if ((rc = same_values(w.p.X, x_dev, (size_t)npts * n.ts.d0, differs, st)) ||
-        (rc = ck(cudaStreamSynchronize(st), "sync")))
-      return rc;
-    kept = *differs == 0;
+  if (kept && !capturing(st)) {
+    int *stale = (int *)pinned_page();
+    kept = stale && !w.kept_graph;
+    if (kept) {
+      *stale = 0;
+      if ((rc = kept_stale(w.p, x_dev, (size_t)npts * n.ts.d0, stale, st)) ||
+          (rc = ck(cudaStreamSynchronize(st), "sync")))
+        return rc;
+      kept = *stale == 0;
+    }
   }
   if (kept)
     return dev_finish(n, st,
                       adjoint_kept(n.dt, n.dn, w.p, n.prec, npts, x_dev, seedm_dev, grad_dev, st));
   // recompute mode: the forward runs again inside the adjoint
   if ((rc = work_planes(w, n, npts, false))) return rc;
-  w.kept = false;
+  if ((rc = planes_taken(w, st))) return rc;
   DevRule given;
   given.kind = SEED_GIVEN;
   BatchArgs a;
@@ -1418,7 +1430,7 @@ int dnnf90_grad_rule_dev(int nid, int tid, int npts, const double *x_dev, int ri
   if ((rc = net_device(n, st))) return rc;
   if ((rc = rule_device(g_rule[rid], n))) return rc;
   if ((rc = work_planes(w, n, npts, false))) return rc;
-  w.kept = false;
+  if ((rc = planes_taken(w, st))) return rc;
   BatchArgs a;
   a.npts = npts; a.X = x_dev; a.out = tm_dev; a.grad = grad_dev; a.loss = loss_dev;
   a.train = true; a.prec = n.prec;
@@ -1439,7 +1451,7 @@ int dnnf90_jrow_dev(int nid, int tid, int npts, const double *x_dev, int rid,
   if ((rc = net_device(n, st))) return rc;
   if ((rc = rule_device(g_rule[rid], n))) return rc;
   if ((rc = work_planes(w, n, npts, false))) return rc;
-  w.kept = false;
+  if ((rc = planes_taken(w, st))) return rc;
   BatchArgs a;
   a.npts = npts; a.X = x_dev; a.out = tm_dev; a.rows = rows_dev;
   a.train = true; a.prec = n.prec;
@@ -1712,6 +1724,7 @@ int dnnf90_committee_step(int nnet, const int *nids, const int *tids, const int 
     }
     if ((rc = comm_build(*C))) return rc;
   }
+  for (int i = 0; i < nnet; ++i) g_twk[tids[i]].kept = false;  // a replay rewrites the planes
   if ((rc = ck(cudaEventRecord(C->ready, caller), "event"))) return rc;
   if ((rc = ck(cudaStreamWaitEvent(C->origin, C->ready, 0), "wait"))) return rc;
   if ((rc = ck(cudaGraphLaunch(C->exec, C->origin), "graph launch"))) return rc;
@@ -1967,6 +1980,7 @@ int kf_pass(int kid, int tid, int npts, const double *x, int rid, double rnoise,
   if ((rc = net_device(n, w.st))) return rc;
   if ((rc = rule_device(rule, n))) return rc;
   if ((rc = work_planes(w, n, 1, false))) return rc;
+  w.kept = false;
   const int nw = (int)n.w.size(), d0 = n.ts.d0, nout = n.dims[n.nlayer - 1];
   const size_t need = ((size_t)npts * d0 + nw + 3) * sizeof(double);
   if ((rc = kf_stage(k, need))) return rc;

@@ -1394,6 +1394,7 @@ int ensure_planes(const DevTables &t, const DevNet &net, int prec, int cap_pts,
   p.X = (double *)(b + oX);
   p.out = (double *)(b + oOut);
   p.loss = (double *)(b + oLoss);
+  p.dirty = (int *)(p.loss + 1);
   // Bell state spill when a block of 32 threads cannot hold it in smem
   int nthr;
   size_t smem;
@@ -1929,8 +1930,7 @@ int adam_device(double *w, const double *g, double *m, double *v, int nw,
   return RC_OK;
 }
 
-// w64 <- w, and *changed = 1 if any bit of it differed; and the comparison
-// alone
+// w64 <- w, and *changed = 1 if any bit of it differed
 __global__ void k_weights_set(double *w64, const double *w, int n, volatile int *changed) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -1939,18 +1939,33 @@ __global__ void k_weights_set(double *w64, const double *w, int n, volatile int 
   w64[i] = v;
   *changed = 1;
 }
-__global__ void k_same(const double *a, const double *b, size_t n, volatile int *differs) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n;
-       i += (size_t)gridDim.x * blockDim.x)
-    if (__double_as_longlong(a[i]) != __double_as_longlong(b[i])) *differs = 1;
+__global__ void k_keep_points(double *X, const double *x, size_t n, int *dirty) {
+  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  for (size_t i = t; i < n; i += (size_t)gridDim.x * blockDim.x) X[i] = x[i];
+  if (t == 0) *dirty = 0;
+}
+__global__ void k_kept_stale(const double *X, const double *x, size_t n, const int *dirty,
+                             volatile int *stale) {
+  const size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  for (size_t i = t; i < n; i += (size_t)gridDim.x * blockDim.x)
+    if (__double_as_longlong(X[i]) != __double_as_longlong(x[i])) *stale = 1;
+  if (t == 0 && *dirty) *stale = 1;
 }
 int weights_set(double *w64, const double *w, int n, int *changed, cudaStream_t st) {
   LAUNCH("k_weights_set", st, k_weights_set<<<(n + 255) / 256, 256, 0, st>>>(w64, w, n, changed));
   CK(cudaGetLastError());
   return RC_OK;
 }
-int same_values(const double *a, const double *b, size_t n, int *differs, cudaStream_t st) {
-  LAUNCH("k_same", st, k_same<<<(int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 592)), 256, 0, st>>>(a, b, n, differs));
+static int points_grid(size_t n) {
+  return (int)std::max<size_t>(1, std::min<size_t>((n + 255) / 256, 592));
+}
+int keep_points(const Planes &p, const double *x, size_t n, cudaStream_t st) {
+  LAUNCH("k_keep_points", st, k_keep_points<<<points_grid(n), 256, 0, st>>>(p.X, x, n, p.dirty));
+  CK(cudaGetLastError());
+  return RC_OK;
+}
+int kept_stale(const Planes &p, const double *x, size_t n, int *stale, cudaStream_t st) {
+  LAUNCH("k_kept_stale", st, k_kept_stale<<<points_grid(n), 256, 0, st>>>(p.X, x, n, p.dirty, stale));
   CK(cudaGetLastError());
   return RC_OK;
 }

@@ -126,6 +126,9 @@ struct Planes {
   double *X = nullptr;       // [P][d0] staged inputs
   double *out = nullptr;     // [P][na][nout]
   double *loss = nullptr;    // [1]
+  // 0: the planes are those of the last kept forward, whose points are in X;
+  // a captured run that rewrites them sets it on every replay
+  int *dirty = nullptr;
   void release();
 };
 
@@ -185,11 +188,13 @@ int adjoint_kept(const DevTables &t, const DevNet &n, Planes &p, int prec,
                  int npts, const double *X, const double *seed, double *grad,
                  cudaStream_t st);
 
-// w64 <- w (device arrays of n doubles), *changed = 1 if any bit differed;
-// *differs = 1 if two arrays differ in any bit.  The flags are device-visible
-// host memory the caller has cleared.
+// w64 <- w (device arrays of n doubles), *changed = 1 if any bit differed.
+// The flags here are device-visible host memory the caller has cleared.
 int weights_set(double *w64, const double *w, int n, int *changed, cudaStream_t st);
-int same_values(const double *a, const double *b, size_t n, int *differs, cudaStream_t st);
+// The n doubles of a kept forward's points x stay beside its planes, and
+// *stale = 1 if the planes are not (or no longer) those of points x.
+int keep_points(const Planes &p, const double *x, size_t n, cudaStream_t st);
+int kept_stale(const Planes &p, const double *x, size_t n, int *stale, cudaStream_t st);
 
 // Adam update on the device (opt_adam_step, lib/train_module.f90:656-683);
 // m and v are allocated by the caller and zero on the first call
