@@ -703,22 +703,28 @@ __global__ void k_rows_dot(const double *J, int nrow, int nw, const double *x, d
   }
 }
 
-// s[i] += sum_r J[r][i] y[r] over this block's rows; s is zeroed before
+// part[c][i] = sum_r J[r][i] y[r] over the rows of chunk c = blockIdx.y
 __global__ void __launch_bounds__(128) k_cols_dot(const double *J, int nrow, int nw,
-                                                  const double *y, int rchunk, double *s) {
+                                                  const double *y, int rchunk, double *part) {
   const int i = blockIdx.x * 128 + threadIdx.x;
   const int r0 = blockIdx.y * rchunk, r1 = min(nrow, r0 + rchunk);
   if (i >= nw) return;
   double v = 0.0;
 #pragma unroll 8
   for (int r = r0; r < r1; ++r) v = fma(__ldcs(J + (size_t)r * nw + i), __ldg(y + r), v);
-  atomicAdd(s + i, v);
+  part[(size_t)blockIdx.y * nw + i] = v;
 }
 
-// u[i] = (b[i] / nb - u[i] / nb) / mu, u[i] = sum_r J[r][i] y[r] before
-__global__ void k_dual_step(int nw, const double *b, double inv_nb, double inv_mu, double *u) {
+// u[i] = (b[i] / nb - sum_c part[c][i] / nb) / mu, the chunks in order; u may
+// be b
+__global__ void k_dual_step(int nw, int nchunk, const double *part, const double *b, double inv_nb,
+                            double inv_mu, double *u) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < nw) u[i] = (b[i] * inv_nb - u[i] * inv_nb) * inv_mu;
+  if (i >= nw) return;
+  double s = 0.0;
+#pragma unroll 8
+  for (int c = 0; c < nchunk; ++c) s += part[(size_t)c * nw + i];
+  u[i] = (b[i] * inv_nb - s * inv_nb) * inv_mu;
 }
 
 int ngd_device_dual(const double *rows, int nrow, int nw, const double *b, int nb, double mu,
@@ -727,11 +733,16 @@ int ngd_device_dual(const double *rows, int nrow, int nw, const double *b, int n
     set_error("the dual natural-gradient step needs a positive damping mu");
     return RC_BAD_ARG;
   }
-  DevScratch Ks, JTs, ys, infos;
+  DevScratch Ks, JTs, ys, infos, parts;
   CKN(Ks.take(sizeof(double) * (size_t)nrow * nrow, st));
   CKN(JTs.take(sizeof(double) * (size_t)nrow * nw, st));
   CKN(ys.take(sizeof(double) * (size_t)nrow, st));
   CKN(infos.take(sizeof(int), st));
+  // J^T y: about four blocks per SM share the rows, at least 16 rows each
+  const int gx = (nw + 127) / 128;
+  const int gy = std::max(1, std::min((nrow + 15) / 16, grid_sms() * 4 / gx));
+  const int rchunk = (nrow + gy - 1) / gy, nchunk = (nrow + rchunk - 1) / rchunk;
+  CKN(parts.take(sizeof(double) * (size_t)nchunk * nw, st));
   double *K = Ks.as<double>(), *JT = JTs.as<double>(), *y = ys.as<double>();
   int *info = infos.as<int>();
   // K = J J^T: the Gram product of the transposed rows, always in FP64.
@@ -750,14 +761,10 @@ int ngd_device_dual(const double *rows, int nrow, int nw, const double *b, int n
     rc = cudaGetLastError() == cudaSuccess ? RC_OK : RC_DEVICE;
     if (!rc) rc = chol_solve(K, nrow, y, info, st);
     if (!rc) {
-      // about four blocks per SM share the rows, at least 16 rows each
-      const int gx = (nw + 127) / 128;
-      const int gy = std::max(1, std::min((nrow + 15) / 16, grid_sms() * 4 / gx));
-      const int rchunk = (nrow + gy - 1) / gy;
-      if (cudaMemsetAsync(u, 0, sizeof(double) * nw, st) != cudaSuccess) rc = RC_DEVICE;
-      LAUNCH("k_cols_dot", st, (k_cols_dot<<<dim3(gx, (nrow + rchunk - 1) / rchunk), 128, 0, st>>>(rows, nrow, nw, y, rchunk, u)));
-      LAUNCH("k_dual_step", st, k_dual_step<<<(nw + 255) / 256, 256, 0, st>>>(nw, b, inv_nb, 1.0 / mu, u));
-      if (!rc) rc = cudaGetLastError() == cudaSuccess ? RC_OK : RC_DEVICE;
+      double *part = parts.as<double>();
+      LAUNCH("k_cols_dot", st, (k_cols_dot<<<dim3(gx, nchunk), 128, 0, st>>>(rows, nrow, nw, y, rchunk, part)));
+      LAUNCH("k_dual_step", st, k_dual_step<<<(nw + 255) / 256, 256, 0, st>>>(nw, nchunk, part, b, inv_nb, 1.0 / mu, u));
+      rc = cudaGetLastError() == cudaSuccess ? RC_OK : RC_DEVICE;
       if (!rc && cudaStreamSynchronize(st) != cudaSuccess) rc = RC_DEVICE;
     }
   }
