@@ -42,10 +42,11 @@ struct NetH {
   uint64_t wver = 1;      // bumped on every weight change
   // w64 on the device is newer than w (host_weights fetches it)
   bool host_stale = false;
-  // recorded after the last write of w64, on wst: a call on another stream
-  // waits for it
+  // recorded after the last write of w64 or of the operands made from it;
+  // set: not yet known to be done, every call's stream waits for it.  (The
+  // stream it was recorded on is not kept: a handle does not name a stream
+  // for good, and the per-thread stream's is the same in every thread.)
   cudaEvent_t wev = nullptr;
-  cudaStream_t wst = nullptr;
   bool wev_set = false;
   int prec = PREC_F64;
   bool dt_ok = false;
@@ -169,7 +170,6 @@ int weights_written(NetH &n, cudaStream_t st) {
   int rc;
   if (!n.wev && (rc = ck(cudaEventCreateWithFlags(&n.wev, cudaEventDisableTiming), "event")))
     return rc;
-  n.wst = st;
   n.wev_set = true;
   return ck(cudaEventRecord(n.wev, st), "weights event");
 }
@@ -181,7 +181,7 @@ int host_weights(NetH &n) {
   if (n.wev_set) rc = ck(cudaEventSynchronize(n.wev), "weights event");
   if (!rc) rc = ck(cudaMemcpy(n.w.data(), n.dn.w64, sizeof(double) * n.w.size(),
                               cudaMemcpyDeviceToHost), "weights D2H");
-  if (!rc) n.host_stale = false;
+  if (!rc) n.host_stale = n.wev_set = false;
   return rc;
 }
 
@@ -211,14 +211,13 @@ int net_device(NetH &n, cudaStream_t st) {
   }
   DevNet &d = n.dn;
   if ((rc = net_buffers(n))) return rc;
+  if (n.wev_set && !capturing(st) && (rc = ck(cudaStreamWaitEvent(st, n.wev, 0), "weights wait"))) return rc;
   if (d.uploaded != n.wver) {
     if ((rc = ck(cudaMemcpyAsync(d.w64, n.w.data(), n.w.size() * sizeof(double),
                                  cudaMemcpyHostToDevice, st), "weights H2D")) ||
         (rc = weights_written(n, st)))
       return rc;
     d.uploaded = n.wver;
-  } else if (n.wev_set && n.wst != st && !capturing(st)) {
-    if ((rc = ck(cudaStreamWaitEvent(st, n.wev, 0), "weights wait"))) return rc;
   }
   // the split path's operands follow the FP64 weights
   if (n.prec == PREC_SPLIT && d.derived != n.wver) {
@@ -543,8 +542,10 @@ int run_eval(int nid, WorkH &w, int npts, const double *x, double *tm,
     }
   }
   if (host) {
-    if (n.prec == PREC_SPLIT) return gemm_tc_flag(&n.dn, w.st);  // waits for st
-    return ck(cudaStreamSynchronize(w.st), "eval");
+    rc = n.prec == PREC_SPLIT ? gemm_tc_flag(&n.dn, w.st)  // waits for st
+                              : ck(cudaStreamSynchronize(w.st), "eval");
+    if (!rc) n.wev_set = false;  // st waited for the weights
+    return rc;
   }
   return RC_OK;
 }
@@ -677,6 +678,7 @@ int host_train(int nid, int tid, int npts, const double *x, int kind,
   // one wait for the work, the loss and the split path's error flag
   if (!rc && n.prec == PREC_SPLIT) rc = gemm_tc_flag(&n.dn, w.st);
   else if (!rc) rc = ck(cudaStreamSynchronize(w.st), "train batch");
+  if (!rc) n.wev_set = false;  // st waited for the weights
   if (loss) *loss = rc ? 0.0 : *lv;
   return rc;
 }
@@ -1312,8 +1314,7 @@ int dnnf90_set_weights_dev(int nid, const double *w_dev, void *stream) {
     return RC_DEVICE;
   }
   if ((rc = net_buffers(n))) return rc;
-  if (n.wev_set && n.wst != st && (rc = ck(cudaStreamWaitEvent(st, n.wev, 0), "weights wait")))
-    return rc;
+  if (n.wev_set && (rc = ck(cudaStreamWaitEvent(st, n.wev, 0), "weights wait"))) return rc;
   // the device copy is compared while it is replaced: equal weights keep
   // their version, so that planes kept by a forward stay valid for the
   // backward that sets the same weights again
