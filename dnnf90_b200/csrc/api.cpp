@@ -200,18 +200,42 @@ int net_buffers(NetH &n) {
   return ck(cudaMalloc(&d.wpk, 2 * n.w.size() * sizeof(double)), "cudaMalloc");
 }
 
+// Waits on the host, from within a capture, for the last write of the device
+// weights: a graph's replays cannot wait for an event of before the capture.
+int weights_wait_host(NetH &n) {
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // the event is not the capture's
+  int rc = ck(cudaThreadExchangeStreamCaptureMode(&mode), "capture mode");
+  if (rc) return rc;
+  rc = ck(cudaEventSynchronize(n.wev), "weights event");
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (!rc) n.wev_set = false;
+  return rc;
+}
+
 // device copies of the network's tables and weights, refreshed when stale,
-// ordered before what st runs next
+// ordered before what st runs next.  A capture records no refresh: it would
+// run at each replay, while the eager calls until then take the copies for
+// current.
 int net_device(NetH &n, cudaStream_t st) {
   int rc = device_ready();
   if (rc) return rc;
+  const bool stale = !n.dt_ok || !n.dn.w64 || n.dn.uploaded != n.wver ||
+                     (n.prec == PREC_SPLIT && n.dn.derived != n.wver);
+  if ((stale || n.wev_set) && capturing(st)) {
+    if (stale) {
+      set_error("the network's copies on the device are older than its weights or precision: "
+                "a call outside the capture brings them up to date");
+      return RC_DEVICE;
+    }
+    return weights_wait_host(n);
+  }
   if (!n.dt_ok) {
     if ((rc = upload_tables(n.ts, n.dt))) return rc;
     n.dt_ok = true;
   }
   DevNet &d = n.dn;
   if ((rc = net_buffers(n))) return rc;
-  if (n.wev_set && !capturing(st) && (rc = ck(cudaStreamWaitEvent(st, n.wev, 0), "weights wait"))) return rc;
+  if (n.wev_set && (rc = ck(cudaStreamWaitEvent(st, n.wev, 0), "weights wait"))) return rc;
   if (d.uploaded != n.wver) {
     if ((rc = ck(cudaMemcpyAsync(d.w64, n.w.data(), n.w.size() * sizeof(double),
                                  cudaMemcpyHostToDevice, st), "weights H2D")) ||

@@ -202,7 +202,14 @@ int dnnf90_kf_status(int kid);
  * a cudaStream_t, NULL for the legacy default stream).  On the split path
  * the compute entries return after the work on stream has finished, having
  * checked the tensor-core GEMMs' error flag (-3 if one gave up); while the
- * stream is being captured into a graph they return without waiting. ---- */
+ * stream is being captured into a graph they return without waiting.
+ *
+ * A captured call reads the weights in place at each replay and, on the split
+ * path, the operands that the last call outside a capture made from them.  It
+ * is refused (-3) while the weights, the tables or those operands on the
+ * device are not current: any call outside the capture refreshes them, and
+ * the same holds before a replay for weights changed since.  A replay is
+ * ordered by the caller after calls that change the weights. ---- */
 /* weights from a device array in the flat layout */
 int dnnf90_set_weights_dev(int nid, const double *w_dev, void *stream);
 /* forward of npts points: tm_dev[npts][na][nout] (may be NULL).  keep = 1
