@@ -1057,11 +1057,15 @@ int dnnf90_adam_step(int nid, int gid, double eta, double beta1, double beta2,
                         istep, nullptr)))
     return rc;
   // the weights stay on the device; the host copy is fetched when it is asked
-  // for, the split operands follow on the next use
+  // for, the split operands follow on the next use.  The call ends with the
+  // update done: a replay of a caller's graph, which waits for no event of
+  // this library, may follow.
   n.wver++;
   n.dn.uploaded = n.wver;
   n.host_stale = true;
-  return weights_written(n, nullptr);
+  rc = ck(cudaStreamSynchronize(nullptr), "adam step");
+  if (!rc) n.wev_set = false;
+  return rc;
 }
 
 // ------------------------------------------------------------- extensions

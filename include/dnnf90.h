@@ -81,7 +81,8 @@ int dnnf90_grad_zero(int gid);
  * reference interface can observe an accumulator before then. */
 int dnnf90_grad_point(int nid, int tid, const double *x,
                       const double *seed, int gid);
-/* replaces dnnf90_adam_step, lib/c_api_module.f90:384-400 */
+/* replaces dnnf90_adam_step, lib/c_api_module.f90:384-400.  Returns with the
+ * weights written. */
 int dnnf90_adam_step(int nid, int gid, double eta, double beta1,
                      double beta2, double eps, int nbatch, int istep);
 

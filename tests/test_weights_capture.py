@@ -119,3 +119,26 @@ def test_capture_waits_for_operands_still_being_made():
         c.check()
         c.eager()
     c.free()
+
+
+@pytest.mark.parametrize("prec", [api.PREC_F64, api.PREC_SPLIT])
+def test_adam_step_ends_with_the_update(prec):
+    """The weights are written when the call returns, also behind work that
+    was on the default stream already, so a replay may follow at once."""
+    import torch
+    c = Case(prec, [2, 32, 32, 1])
+    assert c.step() == 0
+    graph, rc = c.capture()
+    assert rc == 0
+    for istep in (1, 2):
+        c.grad.zero()
+        c.grad.rule_batch(c.X, c.rule)
+        torch.cuda._sleep(20_000_000)  # some 10 ms
+        c.grad.adam(1e-2, 0.9, 0.999, 1e-8, NP, istep)
+        assert torch.cuda.default_stream().query()
+        if prec == api.PREC_SPLIT:     # the operands follow on a call outside the graph
+            c.net.eval(c.X[:1])
+        with torch.cuda.stream(c.stream):
+            graph.replay()
+        c.check()
+    c.free()
