@@ -469,7 +469,8 @@ struct DwArgs {
   int kb_per_cta;        // blocks of DW_RB rows per block of the grid
   double *G;
   int gld, gcol0;
-  int low;               // grid y runs over the tiles of the lower triangle (A = B), j <= i kept
+  unsigned low;          // A = B: tiles of the lower triangle, j <= i kept; the grid's y and
+                         // z run over them, TRI_Y to a z (0: y and z are the tile)
   int *flag;
 };
 
@@ -549,6 +550,8 @@ __device__ __forceinline__ void add16(uint32_t (&d)[32], const uint32_t (&p)[16]
   }
 }
 
+constexpr int TRI_Y = 65535;  // blocks of a grid's y
+
 __global__ void __launch_bounds__(DW_NTH, 1)
     k_tc_dw(DwArgs g, const __grid_constant__ CUtensorMap amap,
             const __grid_constant__ CUtensorMap bmap) {
@@ -563,11 +566,13 @@ __global__ void __launch_bounds__(DW_NTH, 1)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int tn = blockIdx.y, tm = blockIdx.z;  // output tile: A columns tm*128.., B columns tn*128..
   if (g.low) {
-    const int e = blockIdx.y;
-    tm = (int)((sqrtf(8.f * e + 1.f) - 1.f) * 0.5f);
-    while (tm > 0 && tm * (tm + 1) / 2 > e) --tm;
-    while ((tm + 1) * (tm + 2) / 2 <= e) ++tm;
-    tn = e - tm * (tm + 1) / 2;
+    const long long e = (long long)blockIdx.z * TRI_Y + blockIdx.y;
+    if (e >= g.low) return;  // the last z is not full; nothing is set up yet
+    long long t = (long long)((sqrtf(8.f * (float)e + 1.f) - 1.f) * 0.5f);
+    while (t > 0 && t * (t + 1) / 2 > e) --t;
+    while ((t + 1) * (t + 2) / 2 <= e) ++t;
+    tm = (int)t;
+    tn = (int)(e - t * (t + 1) / 2);
   }
   const int nkb_all = (g.K + DW_RB - 1) / DW_RB;
   const int kb0 = blockIdx.x * g.kb_per_cta;
@@ -1060,7 +1065,7 @@ int gemm_tc_syrk(const float *J, int nrow, int nw, int ldj, double *G, cudaStrea
   if (!gemm_tc_available() || nrow < 1 || nw < 1 || ldj % 16 || ldj < nw || ((uintptr_t)J & 15))
     return RC_UNSUPPORTED;
   const long nt = (nw + 127) / 128, low = nt * (nt + 1) / 2;
-  if (low > 65535) return RC_UNSUPPORTED;
+  if (nt > 65535) return RC_UNSUPPORTED;
   static int *flag = nullptr;
   if (!flag) {
     CKT(cudaMalloc(&flag, sizeof(int)));
@@ -1078,13 +1083,14 @@ int gemm_tc_syrk(const float *J, int nrow, int nw, int ldj, double *G, cudaStrea
   a.Mdw = nw; a.Ndw = nw; a.K = nrow;
   a.bwa = a.bwb = std::min(128, ldj);
   a.kb_per_cta = (nkb64 + ctas_k - 1) / ctas_k * (64 / tc::DW_RB);
-  a.G = G; a.gld = nw; a.gcol0 = 0; a.flag = flag; a.low = 1;
+  a.G = G; a.gld = nw; a.gcol0 = 0; a.flag = flag; a.low = (unsigned)low;
   CUtensorMap map;
   std::memset(&map, 0, sizeof map);
   int rc = f32_box_map(&map, J, nrow, ldj, ldj, a.bwa);
   if (rc) return rc;
   const int rows_cta = a.kb_per_cta * tc::DW_RB;
-  const dim3 grid((nrow + rows_cta - 1) / rows_cta, (unsigned)low, 1);
+  const dim3 grid((nrow + rows_cta - 1) / rows_cta, (unsigned)std::min<long>(low, tc::TRI_Y),
+                  (unsigned)((low + tc::TRI_Y - 1) / tc::TRI_Y));
   CKT(cudaFuncSetAttribute(tc::k_tc_dw, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)tc::DW_SMEM));
   LAUNCH("k_tc_syrk", st, tc::k_tc_dw<<<grid, tc::DW_NTH, tc::DW_SMEM, st>>>(a, map, map));
