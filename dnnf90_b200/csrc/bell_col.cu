@@ -294,6 +294,7 @@ int resident_grid(const void *k, int threads, size_t smem) {
 // ------------------------------------------------------------ first layer
 struct L2aArgs {
   int n, na, npts, k, nt, ppw, zsplit;
+  int chain;               // groups of slots to a run (k_adj_l2a)
   const int *up;           // [na][D0]: slot of g + e_i | (g_i + 1) << 16, or -1
   const int *par;          // [na]: slot of a - e_i | i << 16, i the first nonzero dimension
   const double *sc;        // [3][na]: a!, 1/a!, 1/a!
@@ -305,6 +306,11 @@ struct L2aArgs {
 };
 
 constexpr int L2T = 256;   // threads per block
+
+// bytes of k_adj_l2a's tables
+__host__ __device__ inline size_t l2a_tables(int na, int nt, int d0, size_t msz) {
+  return ((size_t)(na + 1) * nt + na + 3) * msz + (size_t)na * d0 * 4 + 16;
+}
 
 // a block's dW_2 sums, one set acc per thread: over the warps, then over the
 // lanes that share a neuron, then one atomic per weight
@@ -333,26 +339,35 @@ __device__ __forceinline__ void l2_reduce(const L2aArgs &a, double *red, const d
 //   Sb^{e_i} = sum_p s^(p) sum_{|a| = p} x_a M_{a - e_i}.
 // One lane per neuron of a tile (lanes beyond a narrow layer's neurons take
 // further points) and PT points at a time per thread: the tile's M rows sit
-// in shared memory and one read of a row serves PT points, so the kernel
-// streams Tb (65536 points x 128 at K = 7, D0 = 4 in FP32: 11 GB in 2.76 ms,
-// 4.0 TB/s; the kernel that staged every item through shared memory and
-// summed it over 32 warps took 6.44).  Gradient mode keeps FP64 sums over a
-// thread's points and may split the slots over blockIdx.z (dW_2 is linear
-// in each slot's share) when there are few points; row mode writes each
-// point's sums.
-template <typename R, int D0, int PT>
-__global__ void __launch_bounds__(L2T) k_adj_l2a(L2aArgs a) {
+// in shared memory and one read of a row serves PT points, and the slots go
+// in groups of G whose values are loaded a group ahead, so the kernel streams
+// Tb (32768 points x 128 at K = 7, D0 = 4 in FP32: 5.5 GB in 1.30 ms, 4.2
+// TB/s; in FP64, 16384 points, 5.5 GB in 1.03).
+// Precision: the degrees, the points and the blocks are added in FP64.  On
+// the split path a degree is summed in FP32 runs of at most a.chain groups
+// (BT = float), or in FP64 throughout (BT = MT = double) where a run would be
+// shorter than a group: never longer than the |A| / 32 slots that one of
+// k_adj_l2s's 32 warps sums, see l2a_k.
+// Gradient mode sums over a thread's points and may split the slots over
+// blockIdx.z (dW_2 is linear in each slot's share) when there are few
+// points; row mode writes each point's sums, a warp's own (L2_ROWS) or, when
+// there are few points, those of a block's eight warps, which share the
+// slots of the same points (L2_ROWS8).
+enum L2Mode { L2_GRAD, L2_ROWS, L2_ROWS8 };
+template <typename R, typename BT, typename MT, int D0, int PT, L2Mode MODE>
+__global__ void __launch_bounds__(L2T, 2) k_adj_l2a(L2aArgs a) {
+  constexpr int G = D0 == 1 ? 1 : 4;            // one slot a degree in one dimension
   extern __shared__ __align__(16) unsigned char sm2[];
   const int na = a.na, n = a.n, nt = a.nt;
-  R *M = (R *)sm2;                              // [na + 1][nt], row na zero
-  R *fact = M + (size_t)(na + 1) * nt;          // [na]
-  int *off = (int *)(fact + (na + (na & 1)));   // [na][D0]: word offset of row a - e_i
+  MT *fact = (MT *)sm2;                         // [na]
+  MT *M = fact + (na + (na & 1));               // [na + 1][nt], row na zero
+  int *off = (int *)(M + ((size_t)(na + 1) * nt + 1) / 2 * 2);  // [na][D0]: word offset of row a - e_i
   const int j0 = blockIdx.y * nt;
   for (int e = threadIdx.x; e < na * D0; e += L2T) off[e] = na * nt;
-  for (int e = threadIdx.x; e < na; e += L2T) fact[e] = (R)__ldg(a.sc + e);
+  for (int e = threadIdx.x; e < na; e += L2T) fact[e] = (MT)__ldg(a.sc + e);
   for (int e = threadIdx.x; e < nt; e += L2T) {
-    M[e] = (R)1;
-    M[(size_t)na * nt + e] = (R)0;
+    M[e] = (MT)1;
+    M[(size_t)na * nt + e] = (MT)0;
   }
   __syncthreads();
   for (int e = threadIdx.x; e < na * D0; e += L2T) {
@@ -367,88 +382,149 @@ __global__ void __launch_bounds__(L2T) k_adj_l2a(L2aArgs a) {
       // the exponent of dimension i: a! over (a - e_i)!
       const double f = __ldg(a.sc + ps) * __ldg(a.sc + na + r);
       M[(size_t)r * nt + jl] =
-          (R)((double)M[(size_t)ps * nt + jl] * (__ldg(a.W + (size_t)j * (D0 + 1) + 1 + i) * f));
+          (MT)((double)M[(size_t)ps * nt + jl] * (__ldg(a.W + (size_t)j * (D0 + 1) + 1 + i) * f));
     }
     __syncthreads();
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int jl = lane % nt, sub = lane / nt, j = j0 + jl;
-  const bool act = sub < a.ppw && j < n;
-  const R *Ml = M + jl;
-  // the slots of this block
-  const int a0 = (int)((long)na * blockIdx.z / a.zsplit);
-  const int a1 = (int)((long)na * (blockIdx.z + 1) / a.zsplit);
-  double acc[D0 + 1];
+  const int jl = lane % nt, sub = lane / nt;
+  const bool act = sub < a.ppw && j0 + jl < n;
+  const int j = min(j0 + jl, n - 1);
+  const MT *Ml = M + jl;
+  // the slots of this block, or of this warp
+  constexpr int NWP = L2T / 32;
+  const int part = MODE == L2_ROWS8 ? warp : (int)blockIdx.z;
+  const int nparts = MODE == L2_ROWS8 ? NWP : a.zsplit;
+  const int a0 = (int)((long)na * part / nparts), a1 = (int)((long)na * (part + 1) / nparts);
+  constexpr int NACC = MODE == L2_GRAD ? 1 : PT;  // sums over points, or each point's
+  double acc[NACC][D0 + 1];
 #pragma unroll
-  for (int o = 0; o <= D0; ++o) acc[o] = 0.0;
-  const long nwarp = (long)gridDim.x * (L2T / 32);
+  for (int k = 0; k < NACC; ++k)
+#pragma unroll
+    for (int o = 0; o <= D0; ++o) acc[k][o] = 0.0;
+  const long nwarp = MODE == L2_ROWS8 ? (long)gridDim.x : (long)gridDim.x * NWP;
+  const long w0 = MODE == L2_ROWS8 ? (long)blockIdx.x : (long)blockIdx.x * NWP + warp;
   const int step = a.ppw;
-  for (long w = (long)blockIdx.x * (L2T / 32) + warp; w * step * PT < a.npts; w += nwarp) {
-    if (!act) continue;
-    long pt[PT];
+  for (long w = w0; w * step * PT < a.npts; w += nwarp) {
+    if (MODE != L2_ROWS8 && !act) continue;  // with shared slots every thread meets the barriers
     const R *Tb[PT], *sg[PT];
-    R s[PT][D0 + 1];
+    bool on[PT];
+    double v0[PT];
 #pragma unroll
     for (int k = 0; k < PT; ++k) {
-      pt[k] = (w * PT + k) * step + sub;
-      const long q = pt[k] < a.npts ? pt[k] : (long)a.npts - 1;  // read twice, dropped below
+      const long pt = (w * PT + k) * step + sub;
+      on[k] = pt < a.npts;
+      const long q = on[k] ? pt : (long)a.npts - 1;  // read twice, times zero
       Tb[k] = (const R *)a.Tb + (size_t)q * na * n + j;
       sg[k] = (const R *)a.sig + (size_t)q * (a.k + 2) * n + j;
-#pragma unroll
-      for (int o = 0; o <= D0; ++o) s[k][o] = (R)0;
+      v0[k] = 0.0;
     }
+    if (MODE != L2_GRAD) {
+#pragma unroll
+      for (int k = 0; k < NACC; ++k)
+#pragma unroll
+        for (int o = 0; o <= D0; ++o) acc[k][o] = 0.0;
+    }
+    R xn[G][PT];  // the next G slots' values
+    auto load = [&](int r) {
+#pragma unroll
+      for (int u = 0; u < G; ++u)
+#pragma unroll
+        for (int k = 0; k < PT; ++k)
+          xn[u][k] = r + u < a1 ? __ldcs(Tb[k] + (size_t)(r + u) * n) : (R)0;
+    };
+    load(a0);
     for (int p = 0; p <= a.k; ++p) {
       const int r0 = max(a.ds[p], a0), r1 = min(a.ds[p + 1], a1);
       if (r0 >= r1) continue;
-      R b[PT][D0 + 1];
+      R s1[PT], sp[PT];
+#pragma unroll
+      for (int k = 0; k < PT; ++k) {
+        s1[k] = on[k] ? sg[k][(size_t)(p + 1) * n] : (R)0;
+        sp[k] = on[k] ? sg[k][(size_t)p * n] : (R)0;
+      }
+      BT b[PT][D0 + 1];
 #pragma unroll
       for (int k = 0; k < PT; ++k)
 #pragma unroll
-        for (int o = 0; o <= D0; ++o) b[k][o] = (R)0;
-#pragma unroll 4
-      for (int r = r0; r < r1; ++r) {
-        R x[PT];
+        for (int o = 0; o <= D0; ++o) b[k][o] = (BT)0;
+      int left = a.chain;
+      for (int q = r0; q < r1; q += G) {
+        BT x[G][PT];
 #pragma unroll
-        for (int k = 0; k < PT; ++k) x[k] = __ldcs(Tb[k] + (size_t)r * n);
-        const R f = fact[r], m0 = Ml[r * nt];
+        for (int u = 0; u < G; ++u)
+#pragma unroll
+          for (int k = 0; k < PT; ++k) x[u][k] = (BT)xn[u][k];
+        load(min(q + G, r1));
+#pragma unroll
+        for (int u = 0; u < G; ++u) {
+          const int r = q + u;
+          if (r >= r1) break;
+          const BT f = (BT)fact[r], m0 = (BT)Ml[r * nt];
+#pragma unroll
+          for (int k = 0; k < PT; ++k) {
+            x[u][k] *= f;
+            b[k][0] = fma(x[u][k], m0, b[k][0]);
+          }
+#pragma unroll
+          for (int i = 0; i < D0; ++i) {
+            const BT m = (BT)Ml[off[r * D0 + i]];
+#pragma unroll
+            for (int k = 0; k < PT; ++k) b[k][1 + i] = fma(x[u][k], m, b[k][1 + i]);
+          }
+        }
+        if (--left && q + G < r1) continue;
+        left = a.chain;
 #pragma unroll
         for (int k = 0; k < PT; ++k) {
-          x[k] *= f;
-          b[k][0] = fma(x[k], m0, b[k][0]);
+          v0[k] = fma((double)s1[k], (double)b[k][0], v0[k]);
+          b[k][0] = (BT)0;
+#pragma unroll
+          for (int i = 0; i < D0; ++i) {
+            double &s = acc[MODE == L2_GRAD ? 0 : k][1 + i];
+            s = fma((double)sp[k], (double)b[k][1 + i], s);
+            b[k][1 + i] = (BT)0;
+          }
         }
-#pragma unroll
-        for (int i = 0; i < D0; ++i) {
-          const R m = Ml[off[r * D0 + i]];
-#pragma unroll
-          for (int k = 0; k < PT; ++k) b[k][1 + i] = fma(x[k], m, b[k][1 + i]);
-        }
-      }
-#pragma unroll
-      for (int k = 0; k < PT; ++k) {
-        const R s1 = sg[k][(size_t)(p + 1) * n], sp = sg[k][(size_t)p * n];
-        s[k][0] = fma(s1, b[k][0], s[k][0]);
-#pragma unroll
-        for (int i = 0; i < D0; ++i) s[k][1 + i] = fma(sp, b[k][1 + i], s[k][1 + i]);
       }
     }
 #pragma unroll
     for (int k = 0; k < PT; ++k) {
-      if (pt[k] >= a.npts) continue;
-      const double *x = a.X + (size_t)pt[k] * D0;
-      if (a.rows) {
-        double *row = a.rows + (size_t)pt[k] * a.nw + a.woff + (size_t)j * (D0 + 1);
-        row[0] = (double)s[k][0];
+      if (!on[k]) continue;
+      const long pt = (w * PT + k) * step + sub;
+      const double *x = a.X + (size_t)pt * D0;
+      double(&s)[D0 + 1] = acc[MODE == L2_GRAD ? 0 : k];
+      s[0] += v0[k];
 #pragma unroll
-        for (int i = 0; i < D0; ++i) row[1 + i] = (double)s[k][0] * __ldg(x + i) + (double)s[k][1 + i];
-      } else {
-        acc[0] += (double)s[k][0];
+      for (int i = 0; i < D0; ++i) s[1 + i] = fma(v0[k], __ldg(x + i), s[1 + i]);
+      if (MODE == L2_ROWS) {
+        double *row = a.rows + (size_t)pt * a.nw + a.woff + (size_t)j * (D0 + 1);
 #pragma unroll
-        for (int i = 0; i < D0; ++i)
-          acc[1 + i] += (double)s[k][0] * __ldg(x + i) + (double)s[k][1 + i];
+        for (int o = 0; o <= D0; ++o) row[o] = s[o];
+      }
+    }
+    if (MODE == L2_ROWS8) {
+      // [value][warp][lane], the warps added in order
+      double *red = (double *)(sm2 + (l2a_tables(na, nt, D0, sizeof(MT)) + 15) / 16 * 16);
+      __syncthreads();  // the last points' sums are written
+#pragma unroll
+      for (int k = 0; k < PT; ++k)
+#pragma unroll
+        for (int o = 0; o <= D0; ++o)
+          red[((size_t)(k * (D0 + 1) + o) * NWP + warp) * 32 + lane] = acc[k][o];
+      __syncthreads();
+      for (int e = warp; e < PT * (D0 + 1); e += NWP) {
+        const int k = e / (D0 + 1), o = e - k * (D0 + 1);
+        const long pt = (w * PT + k) * step + sub;
+        if (!act || pt >= a.npts) continue;
+        double v = 0.0;
+#pragma unroll
+        for (int u = 0; u < NWP; ++u) v += red[((size_t)e * NWP + u) * 32 + lane];
+        a.rows[(size_t)pt * a.nw + a.woff + (size_t)j * (D0 + 1) + o] = v;
       }
     }
   }
-  if (a.g) l2_reduce<D0, L2T>(a, (double *)sm2, acc, act, j0);
+  if (MODE == L2_GRAD && a.g) l2_reduce<D0, L2T>(a, (double *)sm2, acc[0], act, j0);
 }
 
 // The first-layer adjoint of a small set in the order of k_adj_l2s: slot g's
@@ -536,9 +612,8 @@ __global__ void __launch_bounds__(L2RT) k_adj_l2r(L2aArgs a) {
 // neurons of a tile: the layer cut into equal tiles of at most 32
 int l2a_tile(int n) { return (n + (n + 31) / 32 - 1) / ((n + 31) / 32); }
 
-size_t l2a_smem(int na, int nt, int d0, size_t rsz) {
-  const size_t tab = (size_t)(na + 1) * nt * rsz + (size_t)(na + 1) * rsz + (size_t)na * d0 * 4 + 16;
-  return std::max(tab, (size_t)(d0 + 1) * L2T * 8);
+size_t l2a_smem(int na, int nt, int d0, size_t msz) {
+  return std::max(l2a_tables(na, nt, d0, msz), (size_t)(d0 + 1) * L2T * 8);
 }
 
 size_t l2r_smem(int na, int nt, int d0, size_t rsz) {
@@ -549,6 +624,40 @@ size_t l2r_smem(int na, int nt, int d0, size_t rsz) {
 // split path while its conversions to FP64, one set per slot, cost less than
 // the Tb plane's traffic (in FP64 both orders agree to rounding)
 constexpr int L2R_ROWS = 36, L2R_GRAD = 16;
+
+template <typename R, typename BT, typename MT, int D0, int PT, L2Mode MODE>
+int l2a_launch(L2aArgs a, cudaStream_t st) {
+  size_t smem = l2a_smem(a.na, a.nt, D0, sizeof(MT));
+  if (MODE == L2_ROWS8) smem = (smem + 15) / 16 * 16 + (size_t)PT * (D0 + 1) * L2T * 8;
+  if (smem > 227 * 1024) return RC_UNSUPPORTED;
+  const void *k = (const void *)k_adj_l2a<R, BT, MT, D0, PT, MODE>;
+  CKC(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const int gy = (a.n + a.nt - 1) / a.nt;
+  // points per block and pass
+  const long per = (MODE == L2_ROWS8 ? 1L : (long)(L2T / 32)) * a.ppw * PT;
+  const int full = resident_grid(k, L2T, smem);
+  const int gx = (int)std::max(1L, std::min((a.npts + per - 1) / per, (long)std::max(1, full / gy)));
+  // few points: the slots are split over blocks too, at least 8 to a block
+  // (300 points of 8 neurons, 330 slots: 113 us before, 19 here)
+  a.zsplit = MODE != L2_GRAD ? 1 : std::max(1, std::min(a.na / 8, full / std::max(1, gx * gy)));
+  LAUNCH("k_bell_adj_l2", st, (k_adj_l2a<R, BT, MT, D0, PT, MODE><<<dim3(gx, gy, a.zsplit), L2T, smem, st>>>(a)));
+  CKC(cudaGetLastError());
+  return RC_OK;
+}
+
+// Rows.  A block's warps share the points' slots while a warp's own would
+// leave SMs idle (split path, 330 slots x 32 neurons: 1 point 56 -> 29 us, 512
+// 80 -> 39, 2048 98 -> 95; without it 4096 points 105).
+template <typename R, typename BT, int D0>
+int l2a_rows(const L2aArgs &a, cudaStream_t st) {
+  constexpr int PT = sizeof(R) == 4 && D0 <= 5 ? 3 : 2;
+  const int gy = (a.n + a.nt - 1) / a.nt;
+  if ((long)a.npts * gy < 16L * grid_sms() * a.ppw) {
+    const int rc = l2a_launch<R, BT, BT, D0, 1, L2_ROWS8>(a, st);
+    if (rc != RC_UNSUPPORTED) return rc;
+  }
+  return l2a_launch<R, BT, BT, D0, PT, L2_ROWS>(a, st);
+}
 
 template <typename R, int D0>
 int l2a_k(L2aArgs a, cudaStream_t st) {
@@ -564,20 +673,20 @@ int l2a_k(L2aArgs a, cudaStream_t st) {
     CKC(cudaGetLastError());
     return RC_OK;
   }
-  constexpr int PT = sizeof(R) == 8 ? 2 : 4;
-  const size_t smem = l2a_smem(a.na, a.nt, D0, sizeof(R));
-  const void *k = (const void *)k_adj_l2a<R, D0, PT>;
-  CKC(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int gy = (a.n + a.nt - 1) / a.nt;
-  const long per = (long)(L2T / 32) * a.ppw * PT;  // points per block and pass
-  const int full = resident_grid(k, L2T, smem);
-  const int gx = (int)std::max(1L, std::min((a.npts + per - 1) / per, (long)std::max(1, full / gy)));
-  // few points: the slots are split over blocks too, at least 8 to a block
-  // (300 points of 8 neurons, 330 slots: 113 us before, 19 here)
-  a.zsplit = a.rows ? 1 : std::max(1, std::min(a.na / 8, full / std::max(1, gx * gy)));
-  LAUNCH("k_bell_adj_l2", st, (k_adj_l2a<R, D0, PT><<<dim3(gx, gy, a.zsplit), L2T, smem, st>>>(a)));
-  CKC(cudaGetLastError());
-  return RC_OK;
+  // Runs of FP32 sums: |A| / 32 slots in whole groups of four; below that a
+  // gradient's sums are FP64 (65536 points x 128, 35 slots: 0.46 ms, 0.41 in
+  // FP32).  k_adj_l2s added the parts of a row in FP32 too, so a row keeps its
+  // runs of one group.
+  const int run = (a.na + 31) / 32 / 4;
+  if constexpr (sizeof(R) == 4) {
+    a.chain = std::max(1, run);
+    if (a.rows) return l2a_rows<R, float, D0>(a, st);
+    if (run >= 1) return l2a_launch<R, float, float, D0, D0 <= 5 ? 4 : 3, L2_GRAD>(a, st);
+  }
+  a.chain = a.na;
+  if constexpr (sizeof(R) == 8)
+    if (a.rows) return l2a_rows<R, double, D0>(a, st);
+  return l2a_launch<R, double, double, D0, 3, L2_GRAD>(a, st);
 }
 
 template <typename R>
@@ -703,9 +812,9 @@ int bell_adj_col(const ColDev &d, const DevTables &t, int n, int npts, const voi
 }
 
 bool l2a_applies(int d0, int na, int n, int prec) {
-  const size_t rsz = prec == PREC_F64 ? 8 : 4;
+  const size_t msz = prec == PREC_F64 ? 8 : 4;  // the smallest form of the monomials
   return d0 >= 1 && d0 <= 8 && n >= 1 && na <= 65535 &&
-         l2a_smem(na, l2a_tile(n), d0, rsz) <= 227 * 1024;
+         l2a_smem(na, l2a_tile(n), d0, msz) <= 227 * 1024;
 }
 
 int bell_adj_l2a(const DevTables &t, int n, int npts, const void *Tb, const double *X, double *g,
