@@ -1054,9 +1054,10 @@ __global__ void __launch_bounds__(256, VEC ? 3 : 1) k_output_fwdv(OutArgs a) {
 // Adjoint of the output layer, one warp per point (see k_output_adj):
 // Tb_{L-1}^a[i] = sum_o W_L[o][1+i] seed[o][a], dW_L[o][1+i] += sum_a
 // seed[o][a] T_{L-1}^a[i].  Lane i + 32 t holds neuron i + 32 t, t < NT.
-// RED: the block's warps are summed in shared memory before the atomics
-// (outadjv_k says when).
-template <typename R, int MAXO, int NT, bool RED>
+// U: slots whose loads go ahead of their stores (0: as they come).  RED: the
+// block's warps are summed in shared memory before the atomics (outadjv_k
+// says when either).
+template <typename R, int MAXO, int NT, bool RED, int U>
 __global__ void __launch_bounds__(256) k_output_adjv(OutAdjArgs a) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int m = a.m, na = a.na, nout = a.nout;
@@ -1082,9 +1083,8 @@ __global__ void __launch_bounds__(256) k_output_adjv(OutAdjArgs a) {
     for (int o = 0; o < MAXO; ++o)
 #pragma unroll
       for (int t = 0; t < NT; ++t) pg[o][t] = 0.0;
-    if constexpr (RED) {
+    if constexpr (U > 0) {
       // U slots at a time, their loads ahead of their stores
-      constexpr int U = NT <= 4 ? 2 : 1;
       for (int ia0 = 0; ia0 < na; ia0 += U) {
         R tv[U][NT];
 #pragma unroll
@@ -1584,25 +1584,38 @@ static int launch_output_fwdv(const OutArgs &o, cudaStream_t st) {
   return RC_OK;
 }
 
-// Where a warp has little to read, the atomics of the gradient take most of
-// the launch (thousands of warps adding to the same few lines), and a block's
-// warps are summed first: 16384 points of 5 slots x 64 neurons 57 -> 20 us in
-// FP64, 61 -> 21 in FP32.  FP32 warps with much to read lose by it (32768
-// points of 330 slots x 128: 2.0 ms without, 3.2 with); in FP64 the two are
-// level there (0.92 ms at 8191 points).
-template <typename R, int NO, int NT, bool RED>
+template <typename R, int NO, int NT, bool RED, int U>
 static int outadjv_launch(const OutAdjArgs &o, cudaStream_t st) {
-  const void *k = (const void *)k_output_adjv<R, NO, NT, RED>;
+  const void *k = (const void *)k_output_adjv<R, NO, NT, RED, U>;
   const int grid = std::max(1, std::min((o.npts + 7) / 8, occ_grid(k, 256, 0)));
-  LAUNCH("k_output_adj", st, (k_output_adjv<R, NO, NT, RED><<<grid, 256, 0, st>>>(o)));
+  LAUNCH("k_output_adj", st, (k_output_adjv<R, NO, NT, RED, U><<<grid, 256, 0, st>>>(o)));
   CK(cudaGetLastError());
   return RC_OK;
 }
+// Block sums (RED) pay where the atomics take most of the launch: warps with
+// few slots each, and enough of them (16384 points of 5 slots x 64 neurons 57
+// -> 20 us in FP64, 61 -> 21 in FP32); loads ahead (U) where a warp's registers
+// allow.  Both by width and type, us (330 slots, 2048 points; plain, U, RED,
+// both):
+//   FP32   32 neurons 195  95  123   97     FP64   32 neurons 203  103  203  101
+//          64         217 152  291  215            64         238  154  304  144
+//         128         174 256  385  316           128         293  230  291  224
+//         256         469 447  463  398           256         568  695  559  811
+// so one launch of few points, a chain of its own latencies, decides the same
+// way (128 in FP32, one point: 66, 97, 133, 121).
 template <typename R, int NO, int NT>
 static int outadjv_k(const OutAdjArgs &o, cudaStream_t st) {
-  const long rows = (long)o.npts * o.na;  // the line: about 300 rows a resident warp
-  return sizeof(R) == 8 || rows <= (1L << 20) ? outadjv_launch<R, NO, NT, true>(o, st)
-                                              : outadjv_launch<R, NO, NT, false>(o, st);
+  constexpr bool F64 = sizeof(R) == 8;
+  constexpr int U = NT == 1 && !F64 ? 4 : NT <= 4 ? 2 : 1;
+  if constexpr (F64 ? NT <= 4 : NT == 1 || NT > 4) {
+    return outadjv_launch<R, NO, NT, true, U>(o, st);
+  } else {
+    const long rows = (long)o.npts * o.na;
+    const bool red = !o.rows && o.na <= 40 && o.npts >= 512 &&
+                     rows <= (NT == 2 ? 1L << 20 : 300000L);
+    if (red) return outadjv_launch<R, NO, NT, true, F64 ? 0 : U>(o, st);
+    return outadjv_launch<R, NO, NT, false, NT == 2 ? 2 : 0>(o, st);
+  }
 }
 
 template <typename R, int NO>
