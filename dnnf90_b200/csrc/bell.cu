@@ -1488,11 +1488,10 @@ int tune_force(int which, int variant) {
 
 bool tune_pinned() { return g_force[0] >= 0 || g_force[1] >= 0 || g_series_fwd; }
 
-// the column kernels (bell_col.cu) run wherever they apply unless another
-// variant is pinned
-static bool use_col(int which) {
+// the column kernels (bell_col.cu): by their own rule, or pinned
+static bool use_col(int which, const ColDev &col, int n, int npts, int prec) {
   const int f = g_force[which];
-  return f < 0 || f >= 4;
+  return f < 0 ? col_applies(col, n, npts, prec) : f >= 4 && col_fits(col, n, prec);
 }
 
 template <typename L>
@@ -1700,7 +1699,7 @@ static int fwd2_k(const DevBellPlan &bp, const DevTables &t, int n, int npts, co
 int bell_fwd2(const DevBellPlan &bp, const DevTables &t, int n, int npts, const void *S,
               void *T, void *h, bool train, int prec, cudaStream_t st) {
   if (!bp.ready) return RC_UNSUPPORTED;
-  if (use_col(0) && !(t.iact == 0 && bp.f9.ok && g_series_fwd) && col_applies(bp.col, n, npts, prec))
+  if (!(t.iact == 0 && bp.f9.ok && g_series_fwd) && use_col(0, bp.col, n, npts, prec))
     return bell_fwd_col(bp.col, t, n, npts, S, T, h, train, prec, st);
   return prec == PREC_F64 ? fwd2_k<double>(bp, t, n, npts, S, T, h, train, st)
                           : fwd2_k<float>(bp, t, n, npts, S, T, h, train, st);
@@ -1797,7 +1796,7 @@ int bell_adj2(const DevBellPlan &bp, const DevTables &t, int n, int npts, const 
               const void *h, void *Sb, double *gbias, int gstride, int prec,
               cudaStream_t st) {
   if (!bp.ready) return RC_UNSUPPORTED;
-  if (use_col(1) && col_applies(bp.col, n, npts, prec))
+  if (use_col(1, bp.col, n, npts, prec))
     return bell_adj_col(bp.col, t, n, npts, Tb, h, Sb, gbias, gstride, prec, st);
   return prec == PREC_F64 ? adj2_t<double>(bp, t, n, npts, Tb, h, Sb, gbias, gstride, st)
                           : adj2_t<float>(bp, t, n, npts, Tb, h, Sb, gbias, gstride, st);

@@ -759,12 +759,19 @@ void ColDev::release() {
 //         21: 200 + 123 against 904 + 404   56: 1145 + 704 against 1150 + 706
 // and in FP32 33 + 31 against 201 + 150 (10), 164 + 133 against 287 + 220
 // (35), 558 + 288 against 465 + 293 (56): the columns win while the state
-// leaves several warps per SM, up to 36 slots.  Below COL_THREADS neurons
-// there are too few threads to hide a long column's serial chain (2400
-// neurons: 11.5 against 12.8 us at 10 slots, 17 against 15 at 20, 44 against
-// 29 at 36), where only the shortest columns pay.
+// leaves several warps per SM, up to 36 slots.  A launch of few neurons is a
+// column's serial chain and hides nothing behind it; by neurons (points x
+// width, the width in whole 128-byte rows of the other kernels), forward and
+// adjoint, us, columns against the best of the others:
+//   FP32  15 slots  4096: 17/11 14/8   16384: 17/19 14/12   65536: 19/43 15/27
+//         28        4096: 28/12 20/9   16384: 29/23 21/15   32768: 30/33 21/21
+//         35        8192: 22/13 21/10  32768: 23/25 23/21   65536: 25/43 25/33
+//   FP64  15        2048: 17/10 15/8    8192: 17/19 15/13   16384: 17/27 15/19
+//         28        8192: 31/25 21/15  16384: 31/35 21/23   32768: 33/62 23/37
+// and half as many where the width is no multiple of 16 bytes, which the
+// others' fast forms need.
 constexpr int COL_MAX = 36, COL_SHORT = 16;
-constexpr long COL_THREADS = 8192;
+constexpr long COL_BYTES = 64 * 1024;  // of one slot's neurons; twice that beyond COL_SHORT
 
 int upload_col(const TableSet &t, ColDev &d) {
   d.release();
@@ -785,11 +792,17 @@ int upload_col(const TableSet &t, ColDev &d) {
   return RC_OK;
 }
 
-bool col_applies(const ColDev &d, int n, int npts, int prec) {
+bool col_fits(const ColDev &d, int n, int prec) {
   const size_t rsz = prec == PREC_F64 ? 8 : 4;
-  return d.ok && n >= 1 && (d.na <= COL_SHORT || (long)npts * n >= COL_THREADS) &&
-         col_fwd_smem(d.na, d.kt, d.nfrec, rsz) <= 227 * 1024 &&
+  return d.ok && n >= 1 && col_fwd_smem(d.na, d.kt, d.nfrec, rsz) <= 227 * 1024 &&
          col_adj_smem(d.na, d.narec, rsz) <= 226 * 1024;
+}
+
+bool col_applies(const ColDev &d, int n, int npts, int prec) {
+  const int row = prec == PREC_F64 ? 16 : 32;  // neurons of 128 bytes
+  const long bytes = (long)npts * ((n + row - 1) / row) * 128;
+  const long line = (d.na <= COL_SHORT ? 1 : 2) * COL_BYTES / (n % (row / 8) ? 2 : 1);
+  return bytes >= line && col_fits(d, n, prec);
 }
 
 int bell_fwd_col(const ColDev &d, const DevTables &t, int n, int npts, const void *S, void *T,

@@ -34,7 +34,9 @@ struct ColProg {
 ColProg build_col_prog(const TableSet &t);
 int upload_col(const TableSet &t, ColDev &d);
 
-// whether the column kernels take npts points of n neurons on this set
+// whether the column kernels can run on this set, and whether they are the
+// faster ones for npts points of n neurons
+bool col_fits(const ColDev &d, int n, int prec);
 bool col_applies(const ColDev &d, int n, int npts, int prec);
 int bell_fwd_col(const ColDev &d, const DevTables &t, int n, int npts, const void *S, void *T,
                  void *h, bool train, int prec, cudaStream_t st);
