@@ -609,6 +609,79 @@ __global__ void __launch_bounds__(L2RT) k_adj_l2r(L2aArgs a) {
   if (a.g) l2_reduce<D0, L2RT>(a, (double *)sm2, acc, act, j0);
 }
 
+// The rows of k_adj_l2r for few points, a block's eight warps to the points
+// that one warp takes there: the warps share the loads and the 32 partial
+// sums, which are then added in the same order, so that a row has the same
+// bits from either.  Bound: one point's chain (28 slots x 128 neurons, one
+// point: 21 -> 11 us).
+template <typename R, int D0>
+__global__ void __launch_bounds__(L2T) k_adj_l2r8(L2aArgs a) {
+  extern __shared__ __align__(16) unsigned char sm2[];
+  constexpr int NWP = L2T / 32;
+  const int na = a.na, n = a.n, nt = a.nt, j0 = blockIdx.y * nt, nsum = min(32, na);
+  R *tb = (R *)sm2, *hh = tb + (size_t)na * 32;      // [na][32]
+  R *red = hh + (size_t)na * 32;                     // [nsum][D0 + 1][32]
+  R *M = red + (size_t)nsum * (D0 + 1) * 32;         // [na][nt]
+  int *up = (int *)(M + ((size_t)na * nt + 1) / 2 * 2);  // [na][D0]
+  for (int e = threadIdx.x; e < na * D0; e += L2T) up[e] = __ldg(a.up + e);
+  for (int e = threadIdx.x; e < nt; e += L2T) M[e] = (R)1;
+  __syncthreads();
+  for (int p = 1; p <= a.k; ++p) {
+    const int r0 = a.ds[p], nr = a.ds[p + 1] - r0;
+    for (int e = threadIdx.x; e < nr * nt; e += L2T) {
+      const int r = r0 + e / nt, jl = e % nt, j = min(j0 + jl, n - 1), pk = __ldg(a.par + r);
+      M[(size_t)r * nt + jl] = (R)((double)M[(size_t)(pk & 0xffff) * nt + jl] *
+                                   __ldg(a.W + (size_t)j * (D0 + 1) + 1 + (pk >> 16)));
+    }
+    __syncthreads();
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int jl = lane % nt, sub = lane / nt, j = min(j0 + jl, n - 1);
+  const bool act = sub < a.ppw && j0 + jl < n;
+  tb += lane;
+  hh += lane;
+  red += lane;
+  for (long w0 = blockIdx.x; w0 * a.ppw < a.npts; w0 += gridDim.x) {
+    const long pt = w0 * a.ppw + sub, q = min(pt, (long)a.npts - 1);
+    const R *Tb = (const R *)a.Tb + (size_t)q * na * n + j;
+    const R *sg = (const R *)a.sig + (size_t)q * (a.k + 2) * n + j;
+    for (int g = warp, p = 0; g < na; g += NWP) {
+      while (g >= a.ds[p + 1]) ++p;
+      tb[g * 32] = __ldcs(Tb + (size_t)g * n);
+      hh[g * 32] = sg[(size_t)(p + 1) * n] * M[(size_t)g * nt + jl];
+    }
+    __syncthreads();
+    for (int w = warp; w < nsum; w += NWP) {
+      R s[D0 + 1];
+#pragma unroll
+      for (int o = 0; o <= D0; ++o) s[o] = (R)0;
+      for (int g = w; g < na; g += 32) {
+        const R hg = hh[g * 32];
+        s[0] += tb[g * 32] * hg;
+#pragma unroll
+        for (int i = 0; i < D0; ++i) {
+          const int u = up[g * D0 + i];
+          if (u >= 0) s[1 + i] += (R)(u >> 16) * tb[(u & 0xffff) * 32] * hg;
+        }
+      }
+#pragma unroll
+      for (int o = 0; o <= D0; ++o) red[(w * (D0 + 1) + o) * 32] = s[o];
+    }
+    __syncthreads();  // the next points' values go in behind this too: they meet the one above
+    if (!act || pt >= a.npts) continue;
+    double *row = a.rows + (size_t)pt * a.nw + a.woff + (size_t)j * (D0 + 1);
+    for (int o = warp; o <= D0; o += NWP) {
+      R v0 = (R)0, v = (R)0;
+#pragma unroll 8
+      for (int w = 0; w < nsum; ++w) {
+        v0 += red[(w * (D0 + 1)) * 32];
+        v += red[(w * (D0 + 1) + o) * 32];
+      }
+      row[o] = o ? (double)v0 * __ldg(a.X + (size_t)pt * D0 + o - 1) + (double)v : (double)v0;
+    }
+  }
+}
+
 // neurons of a tile: the layer cut into equal tiles of at most 32
 int l2a_tile(int n) { return (n + (n + 31) / 32 - 1) / ((n + 31) / 32); }
 
@@ -619,6 +692,15 @@ size_t l2a_smem(int na, int nt, int d0, size_t msz) {
 size_t l2r_smem(int na, int nt, int d0, size_t rsz) {
   return std::max(((size_t)2 * na * L2RT + (size_t)na * nt + 1) * rsz + (size_t)na * d0 * 4 + 16,
                   (size_t)(d0 + 1) * L2RT * 8);
+}
+size_t l2r8_smem(int na, int nt, int d0, size_t rsz) {
+  return ((size_t)2 * na * 32 + (size_t)std::min(32, na) * (d0 + 1) * 32 + (size_t)na * nt + 1) * rsz +
+         (size_t)na * d0 * 4 + 16;
+}
+// points for which a block's warps share a point's rows: until a warp's own
+// fill the SMs
+bool l2_few(const L2aArgs &a) {
+  return (long)a.npts * ((a.n + a.nt - 1) / a.nt) < 16L * grid_sms() * a.ppw;
 }
 // the sets k_adj_l2r takes: rows while the columns fit, and gradients on the
 // split path while its conversions to FP64, one set per slot, cost less than
@@ -651,8 +733,7 @@ int l2a_launch(L2aArgs a, cudaStream_t st) {
 template <typename R, typename BT, int D0>
 int l2a_rows(const L2aArgs &a, cudaStream_t st) {
   constexpr int PT = sizeof(R) == 4 && D0 <= 5 ? 3 : 2;
-  const int gy = (a.n + a.nt - 1) / a.nt;
-  if ((long)a.npts * gy < 16L * grid_sms() * a.ppw) {
+  if (l2_few(a)) {
     const int rc = l2a_launch<R, BT, BT, D0, 1, L2_ROWS8>(a, st);
     if (rc != RC_UNSUPPORTED) return rc;
   }
@@ -661,6 +742,17 @@ int l2a_rows(const L2aArgs &a, cudaStream_t st) {
 
 template <typename R, int D0>
 int l2a_k(L2aArgs a, cudaStream_t st) {
+  if (a.rows && a.na <= L2R_ROWS && l2_few(a)) {
+    const size_t smem = l2r8_smem(a.na, a.nt, D0, sizeof(R));
+    const void *k = (const void *)k_adj_l2r8<R, D0>;
+    CKC(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    const int gy = (a.n + a.nt - 1) / a.nt;
+    const long groups = (a.npts + a.ppw - 1) / a.ppw;
+    const int gx = (int)std::min(groups, (long)std::max(1, resident_grid(k, L2T, smem) / gy));
+    LAUNCH("k_bell_adj_l2", st, (k_adj_l2r8<R, D0><<<dim3(gx, gy), L2T, smem, st>>>(a)));
+    CKC(cudaGetLastError());
+    return RC_OK;
+  }
   if (a.na <= (a.rows ? L2R_ROWS : sizeof(R) == 4 ? L2R_GRAD : 0)) {
     const size_t smem = l2r_smem(a.na, a.nt, D0, sizeof(R));
     const void *k = (const void *)k_adj_l2r<R, D0>;

@@ -96,3 +96,24 @@ def test_rows_add_up_to_the_gradient(prec, d0, k, n, npts):
     scale = np.sum(np.abs(rows), axis=0)
     assert np.all(np.abs(rows.sum(axis=0) - g) <= (k + 2 * net.na + npts) * u * np.max(scale))
     rule.free(); net.free(); ts.free()
+
+
+@pytest.mark.parametrize("prec", [api.PREC_F64, api.PREC_SPLIT])
+@pytest.mark.parametrize("d0,k,n", [(4, 3, 32), (2, 7, 33), (1, 5, 3), (3, 2, 129), (8, 1, 20),
+                                    (4, 3, 5)])
+def test_small_set_rows_have_one_rounding(prec, d0, k, n):
+    """A row of a set of at most 36 slots has the same bits alone, among few
+    points and among many (the block's warps share a point's slots or not)."""
+    ts = api.TableSet(d0, k)
+    dims = [d0, n, 1]
+    net = api.Net(ts, dims, weights=xavier_weights(dims, 6), precision=prec)
+    rule = api.SeedRule(api.SEED_JROW, [(1.0, net.na, False), (0.3, 1, False)])
+    X = np.random.default_rng(n).uniform(-1, 1, (40000, d0))
+    api.tune_force(0, 4)
+    try:
+        many = api.jacobian_rows(net, X, rule)[0]
+        for npts in (1, 2, 37, 700):
+            assert np.array_equal(api.jacobian_rows(net, X[:npts], rule)[0], many[:npts]), npts
+    finally:
+        api.tune_force(0, -1)
+    rule.free(); net.free(); ts.free()
