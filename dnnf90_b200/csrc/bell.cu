@@ -41,90 +41,40 @@ namespace dnnf90 {
 // switches it on.
 static std::atomic<bool> g_series_fwd{false};
 
-void DevBellPlan::release() {
-  {
-    void *q[] = {f8.list, f8.hdr, f8.cpdst, f8.rec, f9.list, f9.hdr, f9.rec, f9.sdeg64,
-                 f9.sdeg32};
-    for (void *p : q)
-      if (p) cudaFree(p);
-  }
-  for (auto &D : a7) {
-    void *q[] = {D.list, D.unit, D.out, D.fin, D.glist, D.rec};
-    for (void *p : q)
-      if (p) cudaFree(p);
-  }
-  void *ps[] = {fw_list, fw_arec, fw_grec, fw_gc64, fw_gc32, aj_list, aj_orec, aj_pair,
-                aj_c64, aj_c32, f3_list, f3_arec, f3_grec, f3_gc64, f3_gc32, a3_orec,
-                a3_pair, sc64, sc32, f4_grec, a4_pair, f5_list, f5_arec, f5_rec, f5_cpdst,
-                a5_pair, f6_rec};
-  for (void *p : ps)
-    if (p) cudaFree(p);
-  tile.release();
-  tile64.release();
-  col.release();
-  point.release();
-  *this = DevBellPlan();
-}
-
-template <typename T>
-static int put(T **d, const std::vector<T> &h) {
-  size_t n = std::max<size_t>(h.size(), 1);
-  CKB(cudaMalloc((void **)d, n * sizeof(T)));
-  if (!h.empty()) CKB(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-  return RC_OK;
-}
-
-int upload_bell_plan(const TableSet &t, DevBellPlan &d) {
+int upload_bell_plan(const TableSet &t, DevBellPlan &d, PlanBlock &b) {
   static std::atomic<uint64_t> next_id{1};
-  d.release();
+  d = DevBellPlan();
   d.id = next_id++;
   BellPlan P = build_bell_plan(t, BELL_WORKERS, ADJ_WORKERS);
   d.workers = P.workers;
   d.k = P.k;
   d.na = P.na;
   d.nslot = P.nslot;
-  std::vector<float> gc32(P.fw_gc.begin(), P.fw_gc.end());
-  std::vector<float> ac32(P.aj_c.begin(), P.aj_c.end());
-  int rc;
-  if ((rc = put(&d.fw_list, P.fw_list))) return rc;
-  if ((rc = put(&d.fw_arec, P.fw_arec))) return rc;
-  if ((rc = put(&d.fw_grec, P.fw_grec))) return rc;
-  if ((rc = put(&d.fw_gc64, P.fw_gc))) return rc;
-  if ((rc = put(&d.fw_gc32, gc32))) return rc;
-  if ((rc = put(&d.aj_list, P.aj_list))) return rc;
-  if ((rc = put(&d.aj_orec, P.aj_orec))) return rc;
-  if ((rc = put(&d.aj_pair, P.aj_pair))) return rc;
-  if ((rc = put(&d.aj_c64, P.aj_c))) return rc;
-  if ((rc = put(&d.aj_c32, ac32))) return rc;
-  std::vector<float> g3(P.f3_gc.begin(), P.f3_gc.end());
-  if ((rc = put(&d.f3_list, P.f3_list))) return rc;
-  if ((rc = put(&d.f3_arec, P.f3_arec))) return rc;
-  if ((rc = put(&d.f3_grec, P.f3_grec))) return rc;
-  if ((rc = put(&d.f3_gc64, P.f3_gc))) return rc;
-  if ((rc = put(&d.f3_gc32, g3))) return rc;
-  if ((rc = put(&d.a3_orec, P.a3_orec))) return rc;
-  if ((rc = put(&d.a3_pair, P.a3_pair))) return rc;
-  if ((rc = put(&d.f4_grec, P.f4_grec))) return rc;
-  std::vector<uint32_t> a4(P.a4_pair);
-  for (int i = 0; i < 4; ++i) a4.push_back(0);
-  if ((rc = put(&d.a4_pair, a4))) return rc;
-  d.nuv = P.nuv;
+  b.add(&d.fw_list, P.fw_list);
+  b.add(&d.fw_arec, P.fw_arec);
+  b.add(&d.fw_grec, P.fw_grec);
+  b.add(&d.fw_gc64, P.fw_gc);
+  b.add(&d.fw_gc32, std::vector<float>(P.fw_gc.begin(), P.fw_gc.end()));
+  b.add(&d.aj_list, P.aj_list);
+  b.add(&d.aj_orec, P.aj_orec);
+  b.add(&d.aj_pair, P.aj_pair);
+  b.add(&d.aj_c64, P.aj_c);
+  b.add(&d.aj_c32, std::vector<float>(P.aj_c.begin(), P.aj_c.end()));
   std::vector<double> sc(3 * (size_t)P.na);
   for (int i = 0; i < P.na; ++i) {
     sc[i] = P.fact[i];
     sc[P.na + i] = 1.0 / P.fact[i];
     sc[2 * P.na + i] = 1.0 / P.fact[i];
   }
-  std::vector<float> sc32(sc.begin(), sc.end());
-  if ((rc = put(&d.sc64, sc))) return rc;
-  if ((rc = put(&d.sc32, sc32))) return rc;
-  if ((rc = put(&d.f5_list, P.f5_list))) return rc;
-  if ((rc = put(&d.f5_arec, P.f5_arec))) return rc;
-  if ((rc = put(&d.f5_rec, P.f5_rec))) return rc;
-  if ((rc = put(&d.f5_cpdst, P.f5_cpdst))) return rc;
-  if ((rc = put(&d.f6_rec, P.f6_rec))) return rc;
+  b.add(&d.sc64, sc);
+  b.add(&d.sc32, std::vector<float>(sc.begin(), sc.end()));
+  b.add(&d.f5_list, P.f5_list);
+  b.add(&d.f5_arec, P.f5_arec);
+  b.add(&d.f5_rec, P.f5_rec);
+  b.add(&d.f5_cpdst, P.f5_cpdst);
+  b.add(&d.f6_rec, P.f6_rec);
   d.nrec32 = (int)P.f6_rec.size();
-  d.norec = (int)P.a3_orec.size() / 4;
+  d.norec = (int)P.aj_orec.size() / 4;
   {
     // adjoint pairs as (Tb row, h row) byte offsets; the kernel reads up to
     // three pairs past the last one of a list
@@ -132,17 +82,17 @@ int upload_bell_plan(const TableSet &t, DevBellPlan &d) {
     for (int i = 0; i < 8; ++i) a5.push_back(0);
     while (a5.size() % 4) a5.push_back(0);  // whole 16-byte pieces
     d.npair5 = (int)a5.size() / 2;
-    if ((rc = put(&d.a5_pair, a5))) return rc;
+    b.add(&d.a5_pair, a5);
   }
   for (int v = 0; v < 2; ++v) {
     const A7Plan &Q = v ? P.a7d : P.a7f;
     DevBellPlan::A7Dev &D = d.a7[v];
-    if ((rc = put(&D.list, Q.list))) return rc;
-    if ((rc = put(&D.unit, Q.unit))) return rc;
-    if ((rc = put(&D.out, Q.out))) return rc;
-    if ((rc = put(&D.glist, Q.glist))) return rc;
-    if ((rc = put(&D.rec, Q.rec))) return rc;
-    if ((rc = put(&D.fin, Q.fin))) return rc;
+    b.add(&D.list, Q.list);
+    b.add(&D.unit, Q.unit);
+    b.add(&D.out, Q.out);
+    b.add(&D.glist, Q.glist);
+    b.add(&D.rec, Q.rec);
+    b.add(&D.fin, Q.fin);
     D.nunit = (int)Q.unit.size() / 8;
     D.nout = (int)Q.out.size();
     D.nglist = (int)Q.glist.size();
@@ -153,10 +103,10 @@ int upload_bell_plan(const TableSet &t, DevBellPlan &d) {
   }
   {
     const F8Plan &F = P.f8;
-    if ((rc = put(&d.f8.list, F.list))) return rc;
-    if ((rc = put(&d.f8.hdr, F.hdr))) return rc;
-    if ((rc = put(&d.f8.cpdst, F.cpdst))) return rc;
-    if ((rc = put(&d.f8.rec, F.rec))) return rc;
+    b.add(&d.f8.list, F.list);
+    b.add(&d.f8.hdr, F.hdr);
+    b.add(&d.f8.cpdst, F.cpdst);
+    b.add(&d.f8.rec, F.rec);
     d.f8.nrec = (int)F.rec.size();
     d.f8.sbase1 = F.sbase1;
     d.f8.bbase = F.bbase;
@@ -169,12 +119,11 @@ int upload_bell_plan(const TableSet &t, DevBellPlan &d) {
   }
   {
     const F9Plan &F = P.f9;
-    std::vector<float> s32(F.sdeg.begin(), F.sdeg.end());
-    if ((rc = put(&d.f9.list, F.list))) return rc;
-    if ((rc = put(&d.f9.hdr, F.hdr))) return rc;
-    if ((rc = put(&d.f9.rec, F.rec))) return rc;
-    if ((rc = put(&d.f9.sdeg64, F.sdeg))) return rc;
-    if ((rc = put(&d.f9.sdeg32, s32))) return rc;
+    b.add(&d.f9.list, F.list);
+    b.add(&d.f9.hdr, F.hdr);
+    b.add(&d.f9.rec, F.rec);
+    b.add(&d.f9.sdeg64, F.sdeg);
+    b.add(&d.f9.sdeg32, std::vector<float>(F.sdeg.begin(), F.sdeg.end()));
     d.f9.pbase = F.pbase;
     d.f9.qbase = F.qbase;
     d.f9.smem = F.smem;
@@ -184,13 +133,13 @@ int upload_bell_plan(const TableSet &t, DevBellPlan &d) {
   d.nrows5 = P.nrows5;
   d.zuv5 = P.zuv5;
   d.dt_off5 = P.dt_off5;
-  d.f3_ok = P.f3_ok;
-  d.nrows = P.nrows;
-  d.dt_off = P.dt_off;
-  if ((rc = upload_tile_plan(t, d.tile))) return rc;
-  if ((rc = upload_tile64_plan(t, d.tile64))) return rc;
-  if ((rc = upload_col(t, d.col))) return rc;
-  if ((rc = upload_point(t, d.point))) return rc;
+  upload_tile_plan(t, d.tile, b);
+  upload_tile64_plan(t, d.tile64, b);
+  if (col_set(t) || point_set(t)) {
+    const ColProg C = build_col_prog(t);
+    if (col_set(t)) upload_col(t, C, d.col, b);
+    if (point_set(t)) upload_point(t, C, d.point, b);
+  }
   d.ready = true;
   return RC_OK;
 }
@@ -1715,7 +1664,7 @@ static int adj2_t(const DevBellPlan &bp, const DevTables &t, int n, int npts, co
     size_t smem5 = (size_t)4 * t.na * 128;
     Adj5Args b;
     b.n = n; b.na = t.na; b.npts = npts; b.gstride = gstride; b.list = bp.aj_list;
-    b.orec = (const int4 *)bp.a3_orec; b.pair = (const uint2 *)bp.a5_pair;
+    b.orec = (const int4 *)bp.aj_orec; b.pair = (const uint2 *)bp.a5_pair;
     b.norec = bp.norec; b.npair = bp.npair5;
     b.sc = sizeof(R) == 8 ? (const void *)bp.sc64 : (const void *)bp.sc32;
     b.Tb = Tb; b.h = h; b.Sb = Sb; b.gbias = gbias;

@@ -6,6 +6,7 @@
 
 #include "bell_col.hpp"
 #include "bell_plan.hpp"
+#include "plan_block.hpp"
 #include "point.hpp"
 
 namespace dnnf90 {
@@ -31,7 +32,6 @@ struct TileDev {
   int f_o_perm = 0, f_o_rowslot = 0, f_o_fact = 0, f_o_ifact = 0, f_smem = 0;
   int a_o_scr = 0, a_o_list = 0, a_o_flist = 0, a_o_unit = 0, a_o_fin = 0, a_o_rec = 0;
   int a_o_perm = 0, a_o_rowslot = 0, a_o_fact = 0, a_o_ifact = 0, a_smem = 0;
-  void release();
 };
 
 // the same for the FP64 kernels (bell_tile64.cu)
@@ -47,7 +47,6 @@ struct Tile64Dev {
   int f_o_perm = 0, f_o_rowslot = 0, f_o_fact = 0, f_o_ifact = 0, f_smem = 0;
   int a_o_scr = 0, a_o_zero = 0, a_o_list = 0, a_o_flist = 0, a_o_unit = 0, a_o_fin = 0;
   int a_o_rec = 0, a_o_perm = 0, a_o_rowslot = 0, a_o_fact = 0, a_o_ifact = 0, a_smem = 0;
-  void release();
 };
 
 struct DevBellPlan {
@@ -60,22 +59,13 @@ struct DevBellPlan {
   int *aj_list = nullptr, *aj_orec = nullptr, *aj_pair = nullptr;
   double *aj_c64 = nullptr;
   float *aj_c32 = nullptr;
-  // v3
-  bool f3_ok = false;
-  int nrows = 0, dt_off = 0;
-  int *f3_list = nullptr, *f3_arec = nullptr, *f3_grec = nullptr;
-  double *f3_gc64 = nullptr;
-  float *f3_gc32 = nullptr;
-  int *a3_orec = nullptr, *a3_pair = nullptr;
-  uint32_t *f4_grec = nullptr, *a4_pair = nullptr;
-  int nuv = 0;
   // v5
   bool f5_ok = false;
   int nrows5 = 0, dt_off5 = 0, zuv5 = 0;
   int *f5_list = nullptr, *f5_arec = nullptr, *f5_cpdst = nullptr;
   uint32_t *f5_rec = nullptr, *a5_pair = nullptr;
   uint32_t *f6_rec = nullptr;   // forward records as row indices
-  int nrec32 = 0, norec = 0, npair5 = 0;
+  int nrec32 = 0, norec = 0, npair5 = 0;   // norec: outputs of aj_orec
   // v7 adjoint (grouped correlation): [0] FP32 plan, [1] FP64 plan
   struct A7Dev {
     int *list = nullptr, *unit = nullptr, *out = nullptr, *fin = nullptr;
@@ -106,10 +96,9 @@ struct DevBellPlan {
   PointDev point;          // one launch for a small network's step
   double *sc64 = nullptr;  // [3][na]: a!, 1/a!, 1/a! (Tb, h, Sb scales)
   float *sc32 = nullptr;
-  void release();
 };
 
-int upload_bell_plan(const TableSet &t, DevBellPlan &d);
+int upload_bell_plan(const TableSet &t, DevBellPlan &d, PlanBlock &b);
 
 // the autotuner's choices: "kernel width precision variant ms..." lines
 std::string tune_report();
@@ -130,7 +119,7 @@ int bell_adj2(const DevBellPlan &bp, const DevTables &t, int n, int npts, const 
               cudaStream_t st);
 // register-tiled Bell forward and adjoint (bell_tile.cu): dense sets with
 // K <= 7, FP32 planes, n a multiple of 4; RC_UNSUPPORTED otherwise
-int upload_tile_plan(const TableSet &t, TileDev &d);
+void upload_tile_plan(const TableSet &t, TileDev &d, PlanBlock &b);
 bool tile_fwd_applies(const TileDev &d, int n);
 bool tile_adj_applies(const TileDev &d, int n);
 int bell_fwd_tile(const TileDev &d, const DevTables &t, int n, int npts, const void *S, void *T,
@@ -138,7 +127,7 @@ int bell_fwd_tile(const TileDev &d, const DevTables &t, int n, int npts, const v
 int bell_adj_tile(const TileDev &d, int n, int npts, const void *Tb, const void *h, void *Sb,
                   double *gbias, int gstride, cudaStream_t st);
 // and in FP64 (bell_tile64.cu): dense sets with K <= 7, n even
-int upload_tile64_plan(const TableSet &t, Tile64Dev &d);
+void upload_tile64_plan(const TableSet &t, Tile64Dev &d, PlanBlock &b);
 bool tile64_fwd_applies(const Tile64Dev &d, int n);
 bool tile64_adj_applies(const Tile64Dev &d, int n);
 int bell_fwd_tile64(const Tile64Dev &d, const DevTables &t, int n, int npts, const void *S,

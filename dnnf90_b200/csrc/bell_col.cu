@@ -796,13 +796,6 @@ int l2a_t(int d0, const L2aArgs &a, cudaStream_t st) {
   }
 }
 
-template <typename T>
-int put_col(T **d, const std::vector<T> &h) {
-  CKC(cudaMalloc(d, std::max<size_t>(1, h.size()) * sizeof(T)));
-  if (!h.empty()) CKC(cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice));
-  return RC_OK;
-}
-
 template <typename R>
 int fwd_col_t(const ColDev &d, const ColArgs &a, bool train, cudaStream_t st) {
   const size_t smem = col_fwd_smem(d.na, d.kt, d.nfrec, sizeof(R));
@@ -839,12 +832,6 @@ int adj_col_t(const ColDev &d, const ColArgs &a, cudaStream_t st) {
 }  // namespace
 
 // ------------------------------------------------------------ host side
-void ColDev::release() {
-  for (void *p : {(void *)fhdr, (void *)ahdr, (void *)frec, (void *)arec, (void *)dstart})
-    if (p) cudaFree(p);
-  *this = ColDev();
-}
-
 // The rule, by the forward and adjoint measured against the best of the
 // block-per-point kernels (us, 8192 points, layers of 64; FP64):
 //   |A|   10: 39 + 41 against 436 + 306     35: 352 + 284 against 660 + 482
@@ -865,23 +852,20 @@ void ColDev::release() {
 constexpr int COL_MAX = 36, COL_SHORT = 16;
 constexpr long COL_BYTES = 64 * 1024;  // of one slot's neurons; twice that beyond COL_SHORT
 
-int upload_col(const TableSet &t, ColDev &d) {
-  d.release();
-  if (t.na > COL_MAX || t.d0 > D0MAX) return RC_OK;
-  const ColProg P = build_col_prog(t);
-  int rc;
-  if ((rc = put_col(&d.fhdr, P.fhdr)) || (rc = put_col(&d.ahdr, P.ahdr)) ||
-      (rc = put_col(&d.frec, P.frec)) || (rc = put_col(&d.arec, P.arec)) ||
-      (rc = put_col(&d.dstart, P.dstart))) {
-    d.release();
-    return rc;
-  }
+bool col_set(const TableSet &t) { return t.na <= COL_MAX && t.d0 <= D0MAX; }
+
+void upload_col(const TableSet &t, const ColProg &P, ColDev &d, PlanBlock &b) {
+  d = ColDev();
+  b.add(&d.fhdr, P.fhdr);
+  b.add(&d.ahdr, P.ahdr);
+  b.add(&d.frec, P.frec);
+  b.add(&d.arec, P.arec);
+  b.add(&d.dstart, P.dstart);
   d.na = t.na;
   d.kt = P.kt;
   d.nfrec = (int)P.frec.size();
   d.narec = (int)P.arec.size();
   d.ok = true;
-  return RC_OK;
 }
 
 bool col_fits(const ColDev &d, int n, int prec) {

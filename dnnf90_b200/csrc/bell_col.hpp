@@ -6,6 +6,7 @@
 #include <cstdint>
 #include <vector>
 
+#include "plan_block.hpp"
 #include "tables.hpp"
 
 namespace dnnf90 {
@@ -20,7 +21,6 @@ struct ColDev {
   int *fhdr = nullptr, *ahdr = nullptr;      // [na][2]: first record, records
   uint32_t *frec = nullptr, *arec = nullptr;
   int *dstart = nullptr;                     // [kt + 2]: first slot of each degree
-  void release();
 };
 
 // The pair lists of a downward-closed set, per output slot.  Forward: the
@@ -32,7 +32,9 @@ struct ColProg {
   std::vector<uint32_t> frec, arec;
 };
 ColProg build_col_prog(const TableSet &t);
-int upload_col(const TableSet &t, ColDev &d);
+// whether a set is one of the column kernels'
+bool col_set(const TableSet &t);
+void upload_col(const TableSet &t, const ColProg &p, ColDev &d, PlanBlock &b);
 
 // whether the column kernels can run on this set, and whether they are the
 // faster ones for npts points of n neurons

@@ -88,25 +88,15 @@ struct BellPlan {
   std::vector<int> fw_grec;   // [*][4]: ib, g, gbase (state slot of B_{g,2}), qmax
   std::vector<double> fw_gc;  // C(a,b) per group
   std::vector<int> bbase;     // [na]: state slot of B_{a,2} (or -1)
-  // forward, v3 (top degree by the U/V convolution, banded groups, byte
-  // offsets into the shared-memory state; one state row = 128 bytes)
-  int nrows = 0;              // state rows: S | B | U | V | sigma
-  std::vector<int> f3_list;   // [(k+1) * workers][2]
-  std::vector<int> f3_arec;   // [*][8]: ia | p << 16, gstart, gcount, band_hi,
-                              //         b_off, u_off, v_off, band_lo
-  std::vector<int> f3_grec;   // [*][4]: s_b off, s_g off, B_g (or U_g) off, V_g off
-  std::vector<double> f3_gc;  // C(a,b)
-  int dt_off = 0;             // byte offset of the sigma rows
-  bool f3_ok = false;         // every band fits its 8-bit count
-  // forward v4: the same work lists over factorial-normalised state
-  // (rows hold S_b/b!, B_{a,q}/a!, U_g/g!, V_g/g!), so no coefficient is
-  // needed; one 32-bit record per group:
-  //   p < K : ib | g << 10 | (first row of the B run of g) << 20
-  //   p = K : ib | (U row of g) << 10         (V row = U row + nuv)
-  std::vector<uint32_t> f4_grec;
-  int nuv = 0;
-  // forward v5: the v4 work lists with flat records of two byte offsets
-  // into the shared state, no decoding in the inner loop.  Rows:
+  // forward v5: T_a = sum_q s^(q) B_{a,q} regrouped by b (0 < b < a),
+  //   T_a = s' S_a + sum_b C(a,b) S_b U_{a-b},  h_a = s'' S_a + sum_b C(a,b) S_b V_{a-b},
+  //   U_g = sum_{q=1}^{|g|} s^(q+1)/(q+1) B_{g,q},  V_g = sum s^(q+2)/(q+1) B_{g,q}
+  // (the q >= 2 terms of lib/train_module.f90:308-322 with the level index
+  // shifted).  The top degree uses it directly, so no Bell value of degree
+  // K-1 is kept; lower degrees run the recurrence, whose group of b reads
+  // every level of g = a - b (qmax = |g| + 1), so groups are banded by |g|.
+  // The state is factorial-normalised, so no coefficient is needed; flat
+  // records of two byte offsets into it, no decoding in the inner loop.  Rows:
   //   [0, na)       S_b / b!                         (double-buffered)
   //   B run of g    levels 1..|g| of B_{g,q} / g!, level 1 a copy of S_g/g!
   //                 (2 <= |g| <= K-2)
@@ -130,11 +120,10 @@ struct BellPlan {
   // adjoint v7, grouped correlation (A7Plan): FP32 units of up to 16
   // outputs, FP64 units of up to 8 (one lane's accumulators in registers)
   A7Plan a7f, a7d;
-  // adjoint, v3: Sb_b b! = sum_{a >= b} (a! Tb_a) (h_{a-b} / (a-b)!), the
-  // pair coefficient C(a,b) = a!/(b!(a-b)!) folded into per-row scales
-  std::vector<int> a3_orec;   // [*][4]: ib, pstart, pcount, 0
+  // adjoint, v5: Sb_b b! = sum_{a >= b} (a! Tb_a) (h_{a-b} / (a-b)!), the
+  // pair coefficient C(a,b) = a!/(b!(a-b)!) folded into per-row scales; the
+  // work lists are aj_list and aj_orec
   std::vector<int> a3_pair;   // [*][2]: byte offsets of the Tb and h rows
-  std::vector<uint32_t> a4_pair;  // [*]: Tb row | h row << 16
   std::vector<double> fact;   // a! per slot
   // adjoint
   std::vector<int> aj_list;   // [workers][2]

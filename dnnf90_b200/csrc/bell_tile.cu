@@ -533,18 +533,10 @@ __global__ void __launch_bounds__(TWA * 32, 1) k_bell_adj10(Adj10Args a) {
 }  // namespace
 
 // ------------------------------------------------------------ host side
-void TileDev::release() {
-  for (void *p : {(void *)flist, (void *)funit, (void *)frec, (void *)alist, (void *)aunit,
-                  (void *)arec, (void *)aflist, (void *)afin, (void *)perm, (void *)rowslot,
-                  (void *)fact, (void *)ifact})
-    if (p) cudaFree(p);
-  *this = TileDev();
-}
-
-int upload_tile_plan(const TableSet &t, TileDev &d) {
-  d.release();
+void upload_tile_plan(const TableSet &t, TileDev &d, PlanBlock &b) {
+  d = TileDev();
   TilePlan P = build_tile_plan(t, TWF, TWA);
-  if (!P.ok) return RC_OK;
+  if (!P.ok) return;
   std::vector<float> fact(P.na), ifact(P.na);
   for (int r = 0; r < P.na; ++r) {
     const int ia = P.rowslot[r];
@@ -554,16 +546,18 @@ int upload_tile_plan(const TableSet &t, TileDev &d) {
     fact[r] = (float)f;
     ifact[r] = (float)(1.0 / f);
   }
-  int rc;
-  if ((rc = put_vec(&d.flist, P.flist)) || (rc = put_vec(&d.funit, P.funit)) ||
-      (rc = put_vec(&d.frec, P.frec)) || (rc = put_vec(&d.alist, P.alist)) ||
-      (rc = put_vec(&d.aunit, P.aunit)) || (rc = put_vec(&d.arec, P.arec)) ||
-      (rc = put_vec(&d.aflist, P.aflist)) || (rc = put_vec(&d.afin, P.afin)) ||
-      (rc = put_vec(&d.perm, P.perm)) || (rc = put_vec(&d.rowslot, P.rowslot)) ||
-      (rc = put_vec(&d.fact, fact)) || (rc = put_vec(&d.ifact, ifact))) {
-    d.release();
-    return rc;
-  }
+  b.add(&d.flist, P.flist);
+  b.add(&d.funit, P.funit);
+  b.add(&d.frec, P.frec);
+  b.add(&d.alist, P.alist);
+  b.add(&d.aunit, P.aunit);
+  b.add(&d.arec, P.arec);
+  b.add(&d.aflist, P.aflist);
+  b.add(&d.afin, P.afin);
+  b.add(&d.perm, P.perm);
+  b.add(&d.rowslot, P.rowslot);
+  b.add(&d.fact, fact);
+  b.add(&d.ifact, ifact);
   d.td = P.td;
   d.k = P.k;
   d.na = P.na;
@@ -624,7 +618,6 @@ int upload_tile_plan(const TableSet &t, TileDev &d) {
   o += na * 4;
   d.a_smem = o;
   d.ok = true;
-  return RC_OK;
 }
 
 bool tile_fwd_applies(const TileDev &d, int n) {

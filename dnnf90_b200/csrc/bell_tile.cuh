@@ -67,20 +67,6 @@ int grid_for(const void *k, int threads, size_t smem, long items) {
   return (int)std::max(1L, std::min(g, items));
 }
 
-template <typename T>
-int put_vec(T **d, const std::vector<T> &h) {
-  if (h.empty()) return RC_OK;
-  if (cudaMalloc(d, h.size() * sizeof(T)) != cudaSuccess) {
-    set_error("device allocation failed (tile plan)");
-    return RC_NOMEM;
-  }
-  if (cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice) != cudaSuccess) {
-    set_error("copy to the device failed (tile plan)");
-    return RC_DEVICE;
-  }
-  return RC_OK;
-}
-
 #define CKT(x)                                                         \
   do {                                                                 \
     cudaError_t e_ = (x);                                              \

@@ -504,18 +504,10 @@ __global__ void __launch_bounds__(TWA * 32, 1) k_bell_adj64(Adj64Args a) {
 }  // namespace
 
 // ------------------------------------------------------------ host side
-void Tile64Dev::release() {
-  for (void *p : {(void *)flist, (void *)funit, (void *)frec, (void *)alist, (void *)aunit,
-                  (void *)arec, (void *)aflist, (void *)afin, (void *)perm, (void *)rowslot,
-                  (void *)fact, (void *)ifact})
-    if (p) cudaFree(p);
-  *this = Tile64Dev();
-}
-
-int upload_tile64_plan(const TableSet &t, Tile64Dev &d) {
-  d.release();
+void upload_tile64_plan(const TableSet &t, Tile64Dev &d, PlanBlock &b) {
+  d = Tile64Dev();
   const TilePlan P = build_tile_plan(t, TWF, TWA);
-  if (!P.ok) return RC_OK;
+  if (!P.ok) return;
   const int na = P.na, K = P.k, lim = 227 * 1024;
   // what the adjoint's tables take beside its rows, scratch and zeros (an
   // upper bound, checked below)
@@ -531,16 +523,19 @@ int upload_tile64_plan(const TableSet &t, Tile64Dev &d) {
     fact[r] = f;
     ifact[r] = 1.0 / f;
   }
-  int rc;
-  if ((rc = put_vec(&d.flist, P.flist)) || (rc = put_vec(&d.funit, P.funit)) ||
-      (rc = put_vec(&d.frec, P.frec)) || (rc = put_vec(&d.perm, P.perm)) ||
-      (rc = put_vec(&d.rowslot, P.rowslot)) || (rc = put_vec(&d.fact, fact)) ||
-      (rc = put_vec(&d.ifact, ifact)) ||
-      (A.ok && ((rc = put_vec(&d.alist, A.list)) || (rc = put_vec(&d.aunit, A.unit)) ||
-                (rc = put_vec(&d.arec, A.rec)) || (rc = put_vec(&d.aflist, A.flist)) ||
-                (rc = put_vec(&d.afin, A.fin))))) {
-    d.release();
-    return rc;
+  b.add(&d.flist, P.flist);
+  b.add(&d.funit, P.funit);
+  b.add(&d.frec, P.frec);
+  b.add(&d.perm, P.perm);
+  b.add(&d.rowslot, P.rowslot);
+  b.add(&d.fact, fact);
+  b.add(&d.ifact, ifact);
+  if (A.ok) {
+    b.add(&d.alist, A.list);
+    b.add(&d.aunit, A.unit);
+    b.add(&d.arec, A.rec);
+    b.add(&d.aflist, A.flist);
+    b.add(&d.afin, A.fin);
   }
   d.td = P.td;
   d.k = K;
@@ -588,7 +583,6 @@ int upload_tile64_plan(const TableSet &t, Tile64Dev &d) {
     d.a_smem = o;
     d.a_ok = d.a_smem <= lim;
   }
-  return RC_OK;
 }
 
 bool tile64_fwd_applies(const Tile64Dev &d, int n) { return d.f_ok && n % 2 == 0; }

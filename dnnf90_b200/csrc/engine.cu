@@ -224,11 +224,7 @@ static int dput(T **p, const T *h, size_t n) {
 }
 
 void DevTables::release() {
-  void *ps[] = {deg, alpha, ind_e1, seg, fq_pk, fq_c64, fq_c32, pseg, pair_pk,
-                pair_c64, pair_c32, tpc, l2par, l2up};
-  for (void *p : ps)
-    if (p) cudaFree(p);
-  bp.release();
+  if (base) cudaFree(base);
   *this = DevTables();
 }
 
@@ -282,24 +278,25 @@ int upload_tables(const TableSet &t, DevTables &d) {
     pair_pk[i] = (uint32_t)t.pair_ia[i] | ((uint32_t)t.pair_id[i] << 16);
     pair32[i] = (float)t.pair_binom[i];
   }
-  std::vector<int> ie1(t.ind_e1);
   d.nfq = (int)t.fq_ib.size();
   d.npair = (int)t.pair_ia.size();
-  if ((rc = dput(&d.deg, t.deg.data(), t.deg.size()))) return rc;
-  if ((rc = dput(&d.alpha, t.alpha.data(), t.alpha.size()))) return rc;
-  if ((rc = dput(&d.ind_e1, ie1.data(), ie1.size()))) return rc;
-  if ((rc = dput(&d.seg, seg.data(), seg.size()))) return rc;
-  if ((rc = dput(&d.fq_pk, fq_pk.data(), fq_pk.size()))) return rc;
-  if ((rc = dput(&d.fq_c64, t.fq_c.data(), t.fq_c.size()))) return rc;
-  if ((rc = dput(&d.fq_c32, fq32.data(), fq32.size()))) return rc;
-  if ((rc = dput(&d.pseg, pseg.data(), pseg.size()))) return rc;
-  if ((rc = dput(&d.pair_pk, pair_pk.data(), pair_pk.size()))) return rc;
-  if ((rc = dput(&d.pair_c64, t.pair_binom.data(), t.pair_binom.size()))) return rc;
-  if ((rc = dput(&d.pair_c32, pair32.data(), pair32.size()))) return rc;
-  if ((rc = dput(&d.tpc, t.tpc.data(), t.tpc.size()))) return rc;
+  PlanBlock blk;
+  blk.add(&d.deg, t.deg);
+  blk.add(&d.alpha, t.alpha);
+  blk.add(&d.ind_e1, t.ind_e1);
+  blk.add(&d.seg, seg);
+  blk.add(&d.fq_pk, fq_pk);
+  blk.add(&d.fq_c64, t.fq_c);
+  blk.add(&d.fq_c32, fq32);
+  blk.add(&d.pseg, pseg);
+  blk.add(&d.pair_pk, pair_pk);
+  blk.add(&d.pair_c64, t.pair_binom);
+  blk.add(&d.pair_c32, pair32);
+  blk.add(&d.tpc, t.tpc);
   {
     // parent / child slots along unit steps (downward closure keeps a - e_i)
     const int d0 = t.d0;
+    const SlotIndex at(t);
     std::vector<int> par(na, 0), up((size_t)na * d0, -1);
     std::vector<int> b(d0);
     for (int ia = 1; ia < na; ++ia) {
@@ -308,7 +305,7 @@ int upload_tables(const TableSet &t, DevTables &d) {
       while (i0 < d0 && al[i0] == 0) ++i0;
       for (int i = 0; i < d0; ++i) b[i] = al[i];
       b[i0] -= 1;
-      const int ps = t.find(b.data());
+      const int ps = at.find(b.data());
       if (ps < 0) {
         set_error("table program: the carried set is not downward closed");
         return RC_BAD_ARG;
@@ -319,7 +316,7 @@ int upload_tables(const TableSet &t, DevTables &d) {
       for (int i = 0; i < d0; ++i) {
         for (int c = 0; c < d0; ++c) b[c] = t.alpha[(size_t)ia * d0 + c];
         b[i] += 1;
-        const int u = t.find(b.data());
+        const int u = at.find(b.data());
         if (u >= 0) up[(size_t)ia * d0 + i] = u | (b[i] << 16);
       }
     d.graded = true;
@@ -328,10 +325,11 @@ int upload_tables(const TableSet &t, DevTables &d) {
     d.dstart.assign(k + 2, na);
     for (int ia = na - 1; ia >= 0; --ia) d.dstart[t.deg[ia]] = ia;
     for (int p = k; p >= 0; --p) d.dstart[p] = std::min(d.dstart[p], d.dstart[p + 1]);
-    if ((rc = dput(&d.l2par, par.data(), par.size()))) return rc;
-    if ((rc = dput(&d.l2up, up.data(), up.size()))) return rc;
+    blk.add(&d.l2par, par);
+    blk.add(&d.l2up, up);
   }
-  if ((rc = upload_bell_plan(t, d.bp))) return rc;
+  if ((rc = upload_bell_plan(t, d.bp, blk))) return rc;
+  CK(blk.upload(&d.base));
   return RC_OK;
 }
 

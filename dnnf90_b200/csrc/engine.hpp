@@ -67,8 +67,9 @@ struct SeedRuleHost {
 constexpr int SYS_MAXRES = 8;   // residuals of a system rule
 constexpr int SYS_MAXFAC = 4;   // factors of one term
 
-// device copy of one table set
+// device copy of one table set, in one allocation
 struct DevTables {
+  void *base = nullptr;
   int d0 = 0, k = 0, na = 0, nslot = 0, nfq = 0, npair = 0;
   int *deg = nullptr;        // [na]
   int *alpha = nullptr;      // [na][d0]

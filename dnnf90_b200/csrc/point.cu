@@ -631,12 +631,17 @@ int point_blocks(size_t smem) {
 
 }  // namespace
 
-int upload_point(const TableSet &t, PointDev &d) {
+bool point_set(const TableSet &t) {
   // the slots' exponents are packed four bits each
-  if (t.d0 > 8 || t.k < 1 || t.k > 14 || t.na > 512) return RC_OK;
-  const ColProg p = build_col_prog(t);
+  if (t.d0 > 8 || t.k < 1 || t.k > 14 || t.na > 512) return false;
   for (int a = 1; a < t.na; ++a)
-    if (t.deg[a] < t.deg[a - 1]) return RC_OK;
+    if (t.deg[a] < t.deg[a - 1]) return false;
+  return true;
+}
+
+void upload_point(const TableSet &t, const ColProg &p, PointDev &d, PlanBlock &b) {
+  d = PointDev();
+  const SlotIndex at(t);
   std::vector<uint32_t> ex(t.na, 0);
   for (int a = 0; a < t.na; ++a)
     for (int i = 0; i < t.d0; ++i) ex[a] |= (uint32_t)t.alpha[(size_t)a * t.d0 + i] << (4 * i);
@@ -645,35 +650,15 @@ int upload_point(const TableSet &t, PointDev &d) {
   for (int a = 0; a < t.na; ++a)
     for (int i = 0; i < t.d0; ++i) {
       al.assign(t.alpha.begin() + (size_t)a * t.d0, t.alpha.begin() + (size_t)(a + 1) * t.d0);
-      if (al[i]-- > 0) dn[(size_t)a * t.d0 + i] = (short)t.find(al.data());
+      if (al[i]-- > 0) dn[(size_t)a * t.d0 + i] = (short)at.find(al.data());
     }
-  // one block of memory: headers, records, exponents, neighbours
-  std::vector<unsigned char> all;
-  auto add = [&](const void *src, size_t bytes) {
-    const size_t at = all.size();
-    all.insert(all.end(), (const unsigned char *)src, (const unsigned char *)src + bytes);
-    return at;
-  };
-  const size_t fh = add(p.fhdr.data(), (size_t)t.na * 8), ah = add(p.ahdr.data(), (size_t)t.na * 8);
-  const size_t fr = add(p.frec.data(), p.frec.size() * 4);  // both of even length
-  const size_t ar = add(p.arec.data(), p.arec.size() * 4);
-  const size_t xo = add(ex.data(), (size_t)t.na * 4), no = add(dn.data(), dn.size() * 2);
-  CKP(cudaMalloc(&d.base, all.size()));
-  CKP(cudaMemcpy(d.base, all.data(), all.size(), cudaMemcpyHostToDevice));
-  char *q = (char *)d.base;
-  d.fhdr = (int2 *)(q + fh);
-  d.ahdr = (int2 *)(q + ah);
-  d.frec = (uint32_t *)(q + fr);
-  d.arec = (uint32_t *)(q + ar);
-  d.ex = (uint32_t *)(q + xo);
-  d.dn = (short *)(q + no);
+  b.add((int **)&d.fhdr, p.fhdr);
+  b.add((int **)&d.ahdr, p.ahdr);
+  b.add(&d.frec, p.frec);
+  b.add(&d.arec, p.arec);
+  b.add(&d.ex, ex);
+  b.add(&d.dn, dn);
   d.ok = true;
-  return RC_OK;
-}
-
-void PointDev::release() {
-  if (base) cudaFree(base);
-  *this = PointDev{};
 }
 
 // The rule: the plain path, a network whose planes fit shared memory, and up

@@ -4,6 +4,7 @@
 
 #include <cstdint>
 
+#include "bell_col.hpp"
 #include "tables.hpp"
 
 namespace dnnf90 {
@@ -16,13 +17,12 @@ struct BatchArgs;
 // device copy of the pair lists (ColProg) and of the slots' exponents
 struct PointDev {
   bool ok = false;
-  void *base = nullptr;
   int2 *fhdr = nullptr, *ahdr = nullptr;
   uint32_t *frec = nullptr, *arec = nullptr, *ex = nullptr;
   short *dn = nullptr;
-  void release();
 };
-int upload_point(const TableSet &t, PointDev &d);
+bool point_set(const TableSet &t);  // the sets it takes
+void upload_point(const TableSet &t, const ColProg &p, PointDev &d, PlanBlock &b);
 
 // whether one launch serves the batch, and the launch: the same results as
 // run_batch, with no plane in device memory

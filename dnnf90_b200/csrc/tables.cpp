@@ -46,6 +46,27 @@ int TableSet::find(const int *a) const {
   return -1;
 }
 
+SlotIndex::SlotIndex(const TableSet &t) : t_(t) {
+  if (t.d0 > 16 || t.k > 15) return;
+  at_.reserve(2 * (size_t)t.na);
+  for (int ia = 0; ia < t.na; ++ia) {
+    uint64_t key = 0;
+    for (int i = 0; i < t.d0; ++i) key |= (uint64_t)t.alpha[(size_t)ia * t.d0 + i] << (4 * i);
+    at_[key] = ia;
+  }
+}
+
+int SlotIndex::find(const int *a) const {
+  if (at_.empty()) return t_.find(a);
+  uint64_t key = 0;
+  for (int i = 0; i < t_.d0; ++i) {
+    if (a[i] < 0 || a[i] > 15) return -1;
+    key |= (uint64_t)a[i] << (4 * i);
+  }
+  const auto f = at_.find(key);
+  return f == at_.end() ? -1 : f->second;
+}
+
 std::string build_tables(int d0, int k, int nseed, const int *seeds,
                          TableSet &t) {
   // argument contract of table_args_ok (lib/c_api_module.f90:72-84)

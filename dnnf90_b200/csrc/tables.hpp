@@ -14,6 +14,7 @@
 #pragma once
 #include <cstdint>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 namespace dnnf90 {
@@ -43,6 +44,18 @@ struct TableSet {
   int fq_at(int ia, int q) const { return fq_start[ia * (k + 1) + q]; }
   int fq_len(int ia, int q) const { return fq_num[ia * (k + 1) + q]; }
   int find(const int *a) const;  // slot of multi-index a, or -1
+};
+
+// Slots of a set by multi-index, for the builders that ask for many: a
+// multi-index of at most 16 components up to 15 is one 64-bit key.
+class SlotIndex {
+ public:
+  explicit SlotIndex(const TableSet &t);
+  int find(const int *a) const;  // slot of multi-index a, or -1
+
+ private:
+  const TableSet &t_;
+  std::unordered_map<uint64_t, int> at_;
 };
 
 // Builds a table set; returns an empty string on success or the reason the
