@@ -51,7 +51,8 @@ struct Tile64Dev {
 
 struct DevBellPlan {
   bool ready = false;
-  uint64_t id = 0;              // distinct per upload (autotuner key)
+  uint64_t id = 0;              // distinct per upload
+  uint64_t set = 0;             // the same for equal sets and activations (autotuner key)
   int workers = 0, k = 0, na = 0, nslot = 0;
   int *fw_list = nullptr, *fw_arec = nullptr, *fw_grec = nullptr;
   double *fw_gc64 = nullptr;
