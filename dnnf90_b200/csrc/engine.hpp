@@ -259,7 +259,8 @@ struct KfDev {
   int nitem = 0;
   int4 *gitems = nullptr, *grt = nullptr;
   double *gU = nullptr, *gY = nullptr, *gJ[2] = {nullptr, nullptr};
-  double *grpart = nullptr, *gcpart = nullptr, *gdots = nullptr;
+  double *grpart = nullptr, *gcpart = nullptr;
+  double2 *gdots = nullptr;
   void *grp = nullptr;
   double *wprior = nullptr;  // [nw] iterated EKF: the prior weights
   bool prior = false;        // set by an IEKF begin

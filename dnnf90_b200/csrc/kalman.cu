@@ -550,8 +550,19 @@ __global__ void __launch_bounds__(256) k_kf_seq(const int4 *__restrict__ tiles, 
 // (s_i the gate's scale), because each update is P <- (P - p p^T / denom) /
 // lambda + q I: a <- a / lambda, c <- c / lambda + q, b_i <- b_i / lambda and
 // b_k = 1 / (lambda denom).  Every p_i is therefore a combination of the Y_l
-// and j_l, l <= i, whose coefficients, denominators and gates follow from the
-// 8 x 8 products j_l . Y_k and j_l . j_k alone.  Per group three launches:
+// and j_l, l <= i.  Its coefficients, the denominators and the gates come from
+// running the same update on 8 x 8 matrices: G = (j_l . P_k j_m) and the
+// coefficients of P_k j_m in the Y_l and in the j_l.  Rows that resemble each
+// other make G's update a difference of nearly equal numbers, whose rounding
+// the single updates share out over the whole covariance, so the products
+// j_l . Y_m, these matrices and the combinations of the Y_l are double-double.
+// (300 weights, 24 rows of correlation 0.9999, p0 = 1e4, weights against 80-bit
+// arithmetic: single updates 3.2e-13 to 6.6e-13, groups in doubles 3.1e-12 to
+// 7.8e-12, so 2.6e-13 to 4.1e-13; correlation 0.9, p0 = 10: 4.0e-16 to 4.5e-16,
+// 3.0e-16 to 4.9e-16, 1.5e-16 to 1.9e-16.  Here, 1217 weights, the error against
+// the single updates': weights 0.35 without correlation, 0.5 at 0.99, 2.1 at
+// 0.9999 (10.6 in doubles), covariance 0.5, 1.8 (4.2) and 1.5 (11.3).)  Per group
+// three launches:
 //   k_kf_greduce  sums the partial products into Y, forms the 8 x 8
 //                 products, and its last CTA runs the recursion over k
 //   k_kf_gvec     U_i = sqrt(b_i) p_i, w += sum_k p_k xi_k / denom_k, and the
@@ -567,11 +578,54 @@ constexpr int GM = 8;            // observations per group
 constexpr int GW = 8;            // warps of k_kf_gtiles: tile rows of a row block
 constexpr int GVS = 12;          // row stride of the staged column vectors (doubles)
 
+// double-double: h + l, |l| at most half an ulp of h
+struct Dd {
+  double h, l;
+};
+__device__ __forceinline__ Dd dd_norm(double h, double l) {
+  const double s = h + l;
+  return {s, l - (s - h)};
+}
+__device__ __forceinline__ double two_sum_err(double a, double b, double s) {
+  const double t = s - a;
+  return (a - (s - t)) + (b - t);
+}
+__device__ __forceinline__ Dd dd_add(Dd a, Dd b) {
+  const double s = a.h + b.h;
+  return dd_norm(s, two_sum_err(a.h, b.h, s) + (a.l + b.l));
+}
+__device__ __forceinline__ Dd dd_sub(Dd a, Dd b) { return dd_add(a, {-b.h, -b.l}); }
+__device__ __forceinline__ Dd dd_mul(Dd a, Dd b) {
+  const double p = __dmul_rn(a.h, b.h);  // not fused with the sum that follows
+  return dd_norm(p, fma(a.h, b.l, fma(a.l, b.h, fma(a.h, b.h, -p))));
+}
+__device__ __forceinline__ Dd dd_div(Dd a, Dd b) {
+  const double q = a.h / b.h, p = __dmul_rn(q, b.h);
+  const double r = ((a.h - p) - fma(q, b.h, -p)) + fma(-q, b.l, a.l);
+  return dd_norm(q, r / b.h);
+}
+__device__ __forceinline__ Dd dd_sqrt(Dd a) {  // a >= 0
+  if (!(a.h > 0.0)) return {0.0, 0.0};
+  const double s = sqrt(a.h);
+  return dd_norm(s, (fma(-s, s, a.h) + a.l) / (2.0 * s));
+}
+// a running sum: h the sum in doubles, l what it has rounded off
+__device__ __forceinline__ void dd_acc(Dd &a, double h, double l) {
+  const double s = a.h + h;
+  a.l += two_sum_err(a.h, h, s) + l;
+  a.h = s;
+}
+// a running sum plus x y
+__device__ __forceinline__ void dd_fma(Dd &a, Dd x, double y) {
+  const double p = __dmul_rn(x.h, y);
+  dd_acc(a, p, fma(x.l, y, fma(x.h, y, -p)));
+}
+
 struct KfGroup {
   int m;                         // observations to apply (0: none)
   double a, c;
-  double ua[GM][GM], ub[GM][GM]; // U_i = sum_l ua[i][l] Y_l + ub[i][l] j_l
-  double wa[GM], wb[GM];         // w += sum_l wa[l] Y_l + wb[l] j_l
+  Dd ua[GM][GM], ub[GM][GM];     // U_i = sum_l ua[i][l] Y_l + ub[i][l] j_l
+  Dd wa[GM], wb[GM];             // w += sum_l wa[l] Y_l + wb[l] j_l
 };
 
 __device__ __forceinline__ void kf_dmma(double (&d)[2], double a, double b) {
@@ -603,7 +657,7 @@ __device__ __forceinline__ int kf_chunk(int row, int c2) {
 // tiles and vectors stream in by cp.async meanwhile.  Row products stay in
 // registers along the item, column products are summed over the eight warps,
 // so the partial sums are a tenth of the covariance's traffic.
-// Bound: HBM; at nw = 17025 one pass takes 450 us for 2.32 GB (5.1 TB/s), 69 us
+// Bound: HBM; at nw = 17025 one pass takes 450 us for 2.32 GB (5.1 TB/s), 73 us
 // per observation with the two small launches, against 569 for single updates.
 template <int MODE>
 __global__ void __launch_bounds__(GW * 32, 1)
@@ -753,11 +807,12 @@ __global__ void __launch_bounds__(GRT)
     k_kf_greduce(int nw, const int4 *__restrict__ grt,
                  const double *__restrict__ rpart, const double *__restrict__ cpart,
                  const double *__restrict__ J, double *__restrict__ Y, KfRowArgs ra, int k0, int m,
-                 int kbase, double *__restrict__ dots, unsigned *__restrict__ ctr,
+                 int kbase, double2 *__restrict__ dots, unsigned *__restrict__ ctr,
                  KfGroup *__restrict__ grp, KfState *__restrict__ st) {
   __shared__ double ys[KT * GM], js[KT * GM], half[KT * GM];
-  __shared__ double tot[4][2 * GM * GM];
-  __shared__ double al[GM][GM], be[GM][GM], bb[GM], dd[GM], wc[GM];
+  __shared__ Dd tot[4][2 * GM * GM];
+  __shared__ Dd mat[3][GM][GM];        // G and the coefficients of P_k j_m in Y_l, in j_l
+  __shared__ Dd al[GM][GM], be[GM][GM], bb[GM], wc[GM];
   __shared__ bool s_last;
   const int t = threadIdx.x;
   if (st->status) {  // an earlier group failed: nothing is applied from there on
@@ -791,10 +846,13 @@ __global__ void __launch_bounds__(GRT)
   if (t < 2 * GM * GM) {  // j_l . Y_k, then j_l . j_k
     const int l = (t >> 3) & 7, k = t & 7;
     const double *b = t < GM * GM ? ys : js;
-    double v = 0.0;
+    Dd v = {0.0, 0.0};
 #pragma unroll 8
-    for (int r = 0; r < KT; ++r) v = fma(js[r * GM + l], b[r * GM + k], v);
-    dots[(size_t)blockIdx.x * 2 * GM * GM + t] = v;
+    for (int r = 0; r < KT; ++r) {
+      const double x = js[r * GM + l], y = b[r * GM + k], p = __dmul_rn(x, y);
+      dd_acc(v, p, fma(x, y, -p));
+    }
+    dots[(size_t)blockIdx.x * 2 * GM * GM + t] = make_double2(v.h, v.l);
   }
   __threadfence();
   __syncthreads();
@@ -804,89 +862,103 @@ __global__ void __launch_bounds__(GRT)
   __threadfence();
   {
     const int e = t & 127, h = t >> 7;
-    double v = 0.0;
+    Dd v = {0.0, 0.0};
 #pragma unroll 16
-    for (int b = h; b < (int)gridDim.x; b += 4) v += __ldcg(dots + (size_t)b * 2 * GM * GM + e);
+    for (int b = h; b < (int)gridDim.x; b += 4) {
+      const double2 d = __ldcg(dots + (size_t)b * 2 * GM * GM + e);
+      dd_acc(v, d.x, d.y);
+    }
     tot[h][e] = v;
   }
   __syncthreads();
-  if (t < 128) tot[0][t] += tot[1][t] + (tot[2][t] + tot[3][t]);
+  if (t < 128) {
+    Dd v = tot[0][t];
+    for (int h = 1; h < 4; ++h) dd_acc(v, tot[h][t].h, tot[h][t].l);
+    // an overflowed product keeps its infinity
+    tot[0][t] = fabs(v.h) <= 1.7976931348623157e308 ? dd_norm(v.h, v.l) : Dd{v.h, 0.0};
+  }
   __syncthreads();
-  if (t >= 32) return;
-  // one warp: lane l the coefficients of Y_l and j_l
-  const double *g = tot[0], *nn = tot[0] + GM * GM;
-  const int l = t & 7;
-  const double q = st->q, gate = st->gate, lam0 = st->lam0;
-  double lam = st->lam, a = 1.0, c = 0.0;
+  // the recursion: thread t < 192 holds entry (l, c) of one of the matrices
+  const int which = t >> 6, l = (t >> 3) & 7, c8 = t & 7;
+  const bool on = which < 3;
+  if (on)
+    mat[which][l][c8] =
+        which == 0 ? tot[0][l * GM + c8] : Dd{which == 1 && l == c8 ? 1.0 : 0.0, 0.0};
+  const double q = st->q > 0.0 ? st->q : 0.0, gate = st->gate, lam0 = st->lam0;
+  double lam = st->lam;
+  Dd a = {1.0, 0.0}, c = {0.0, 0.0}, b = {0.0, 0.0};  // b: of observation t, for t < 8
   int k = 0, ng = 0, fail = 0;
   double lamk = lam, denomk = 0.0, sgk = 1.0, xik = 0.0;
+  __syncthreads();
   for (; k < m; ++k) {
-    if (t < GM) {  // lane i: d_ik = p_i . j_k
-      double d = 0.0;
-      if (t < k)
-        for (int x = 0; x <= t; ++x)
-          d = fma(al[t][x], g[x * GM + k], fma(be[t][x], nn[x * GM + k], d));
-      dd[t] = d;
-    }
-    __syncwarp();
-    double jpj = fma(a, g[k * GM + k], c * nn[k * GM + k]);
-    double av = l == k ? a : 0.0, bv = l == k ? c : 0.0;
-    for (int i = 0; i < k; ++i) {
-      const double bd = bb[i] * dd[i];
-      jpj = fma(-bd, dd[i], jpj);
-      av = fma(-bd, al[i][l], av);
-      bv = fma(-bd, be[i][l], bv);
-    }
-    double denom = lam + jpj;
-    if (!(denom > 0.0)) {
+    const Dd lm = {lam, 0.0}, jpj = mat[0][k][k];
+    double den = lam + jpj.h;
+    if (!(den > 0.0)) {
       fail = kbase + k0 + k + 1;
       break;
     }
     double xi = row_scale(ra, k0 + k) * ra.xi[k0 + k], sg = 1.0;
-    if (gate > 0.0 && xi * xi > gate * gate * denom) {
-      const double s2 = gate * gate * lam / (xi * xi - gate * gate * jpj);
-      sg = sqrt(s2);
+    Dd s2 = {1.0, 0.0};
+    if (gate > 0.0 && xi * xi > gate * gate * den) {
+      s2.h = gate * gate * lam / (xi * xi - gate * gate * jpj.h);
+      sg = sqrt(s2.h);
       xi = sg * xi;
-      denom = lam + s2 * jpj;
+      s2 = dd_mul({sg, 0.0}, {sg, 0.0});
       ++ng;
     }
-    __syncwarp();
-    if (t < GM) {
-      al[k][l] = sg * av;
-      be[k][l] = sg * bv;
-      if (t < k) bb[t] /= lam;
-      if (t == k) {
-        bb[k] = 1.0 / (lam * denom);
-        wc[k] = xi / denom;
+    // P_{k+1} j = (P_k j - p_k (s2 j_k . P_k j) / denom) / lambda + q j
+    const bool inf = !(den <= 1.7976931348623157e308);
+    const Dd dd = inf ? Dd{den, 0.0} : dd_add(lm, dd_mul(s2, jpj));
+    den = dd.h;
+    Dd v = {0.0, 0.0}, pa = v, pb = v;
+    if (on) {
+      v = mat[which][l][c8];
+      if (!inf)
+        v = dd_sub(v, dd_mul(mat[which][l][k], dd_div(dd_mul(s2, mat[0][k][c8]), dd)));
+      v = dd_div(v, lm);
+      if (q > 0.0) {
+        if (which == 0) v = dd_add(v, dd_mul({q, 0.0}, tot[0][GM * GM + l * GM + c8]));
+        else if (which == 2 && l == c8) v = dd_add(v, {q, 0.0});
       }
     }
-    a /= lam;
-    c = c / lam + (q > 0.0 ? q : 0.0);
+    if (t < GM) {
+      pa = dd_mul({sg, 0.0}, mat[1][t][k]);
+      pb = dd_mul({sg, 0.0}, mat[2][t][k]);
+      b = t == k ? (inf ? Dd{0.0, 0.0} : dd_div({1.0, 0.0}, dd_mul(lm, dd))) : dd_div(b, lm);
+      al[k][t] = pa;
+      be[k][t] = pb;
+      if (t == k) wc[k] = inf ? Dd{0.0, 0.0} : dd_div({xi, 0.0}, dd);
+    }
+    a = dd_div(a, lm);
+    c = dd_add(dd_div(c, lm), {q, 0.0});
     lamk = lam;
-    denomk = denom;
+    denomk = den;
     sgk = sg;
     xik = xi;
     lam = __dadd_rn(__dmul_rn(lam0, lam), 1.0) - lam0;
-    __syncwarp();
+    __syncthreads();  // every entry of step k is read
+    if (on) mat[which][l][c8] = v;
+    __syncthreads();
   }
+  if (t < GM) bb[t] = dd_sqrt(b);
+  __syncthreads();
   if (t < GM) {
-    double wa = 0.0, wb = 0.0;
+    Dd wa = {0.0, 0.0}, wb = wa;
     for (int i = 0; i < k; ++i) {
-      const double s = sqrt(bb[i]);
-      grp->ua[i][l] = s * al[i][l];
-      grp->ub[i][l] = s * be[i][l];
-      wa = fma(wc[i], al[i][l], wa);
-      wb = fma(wc[i], be[i][l], wb);
+      grp->ua[i][t] = dd_mul(bb[i], al[i][t]);
+      grp->ub[i][t] = dd_mul(bb[i], be[i][t]);
+      wa = dd_add(wa, dd_mul(wc[i], al[i][t]));
+      wb = dd_add(wb, dd_mul(wc[i], be[i][t]));
     }
-    for (int i = k; i < GM; ++i) grp->ua[i][l] = grp->ub[i][l] = 0.0;
-    grp->wa[l] = wa;
-    grp->wb[l] = wb;
+    for (int i = k; i < GM; ++i) grp->ua[i][t] = grp->ub[i][t] = {0.0, 0.0};
+    grp->wa[t] = wa;
+    grp->wb[t] = wb;
   }
   if (t == 0) {
     *ctr = 0;
     grp->m = k;
-    grp->a = a;
-    grp->c = c;
+    grp->a = a.h;
+    grp->c = c.h;
     st->lam = lam;
     st->ngated += ng;
     if (k > 0) {
@@ -915,7 +987,7 @@ __global__ void __launch_bounds__(128)
   }
   if (R >= nw) return;
   if (grp) {
-    double y[GM], j[GM], dw = 0.0;
+    double y[GM], j[GM];
 #pragma unroll
     for (int l = 0; l < GM; l += 2) {
       const double2 a = *(const double2 *)(Y + (size_t)R * GM + l);
@@ -926,17 +998,28 @@ __global__ void __launch_bounds__(128)
       j[l] = l < g.m ? b.x : 0.0;
       j[l + 1] = l + 1 < g.m ? b.y : 0.0;
     }
+    // sums of nearly opposite terms where the rows resemble each other
+    const bool cj = g.c != 0.0;  // without process noise the j_l take no part
+    Dd dw = {0.0, 0.0};
 #pragma unroll
-    for (int l = 0; l < GM; ++l) dw = fma(g.wa[l], y[l], fma(g.wb[l], j[l], dw));
-    w[R] += dw;
+    for (int l = 0; l < GM; ++l) {
+      dd_fma(dw, g.wa[l], y[l]);
+      if (cj) dd_fma(dw, g.wb[l], j[l]);
+    }
+    w[R] += dw.h + dw.l;
 #pragma unroll
     for (int i = 0; i < GM; i += 2) {
-      double u[2] = {0.0, 0.0};
+      double u[2];
 #pragma unroll
-      for (int h = 0; h < 2; ++h)
+      for (int h = 0; h < 2; ++h) {
+        Dd v = {0.0, 0.0};
 #pragma unroll
-        for (int l = 0; l <= i + h; ++l)
-          u[h] = fma(g.ua[i + h][l], y[l], fma(g.ub[i + h][l], j[l], u[h]));
+        for (int l = 0; l <= i + h; ++l) {
+          dd_fma(v, g.ua[i + h][l], y[l]);
+          if (cj) dd_fma(v, g.ub[i + h][l], j[l]);
+        }
+        u[h] = v.h + v.l;
+      }
       *(double2 *)(U + (size_t)R * GM + i) = make_double2(u[0], u[1]);
     }
   }
@@ -984,8 +1067,8 @@ void KfDev::release() {
 // but each has products j_l . P j_k of its own, so that the recursion would
 // run per block.
 // Measured per observation, 64 (3) to a call, against the faster of the
-// single-update paths: nw = 1217 5.5 (21) us against 14.3 (25.5), 4481 9.4 (31)
-// against 48 (64), 17025 69 (220) against 569 (645).
+// single-update paths: nw = 1217 6.6 (25) us against 14.1 (27), 4545 10.7 (36)
+// against 50 (63), 17025 73 (233) against 566 (568).
 constexpr int KF_GROUP_TILES = 512, KF_GROUP_OBS = 3;
 constexpr size_t GT_SMEM =
     (size_t)(2 * GW * KTE + 2 * 2 * KT * GVS + GW * KT * GM) * sizeof(double);
@@ -1024,7 +1107,7 @@ static int group_create(KfDev &d) {
   const size_t oi = take(items.size() * sizeof(int4)), og = take(grt.size() * sizeof(int4));
   const size_t oU = take(vb), oY = take(vb), oJ0 = take(vb), oJ1 = take(vb);
   const size_t orp = take((size_t)rp * KT * GM * 8), ocp = take((size_t)cp * KT * GM * 8);
-  const size_t od = take((size_t)d.nred * 2 * GM * GM * 8), ogr = take(sizeof(KfGroup));
+  const size_t od = take((size_t)d.nred * 2 * GM * GM * 16), ogr = take(sizeof(KfGroup));
   if (cudaMalloc(&d.gbuf, cur) != cudaSuccess) {
     cudaGetLastError();  // the two-launch path needs none of it
     d.gbuf = nullptr;
@@ -1042,7 +1125,7 @@ static int group_create(KfDev &d) {
   d.gJ[1] = (double *)(p + oJ1);
   d.grpart = (double *)(p + orp);
   d.gcpart = (double *)(p + ocp);
-  d.gdots = (double *)(p + od);
+  d.gdots = (double2 *)(p + od);
   d.grp = p + ogr;
   return RC_OK;
 }
