@@ -330,11 +330,14 @@ struct AdjL {
     for (int k = 0; k < cnt; ++k) {
       const uint2 rr = rec[i + k];
       const uint32_t r = half ? rr.y : rr.x;
-      const double *hp = (r & TILE_NULL) ? zero : hb + (r & (TILE_NULL - 1)) * NPB;
+      // a missing record is zeros times zeros: Tb may be infinite
+      const bool null = r & TILE_NULL;
+      const double *hp = null ? zero : hb + (r & (TILE_NULL - 1)) * NPB;
+      const double *tp = null ? zero : tbb + ((r >> 14) & 0x3fffu) * NPB;
       double hv[NT];
 #pragma unroll
       for (int e = 0; e < NT; ++e) hv[e] = hp[e * NPB];
-      AdjRows<TD, 0, NT>::run(tbb + ((r >> 14) & 0x3fffu) * NPB, hv, acc);
+      AdjRows<TD, 0, NT>::run(tp, hv, acc);
     }
     AdjL<TD, L - 1>::run(tbb, hb, zero, rec, half, i + cnt, cw, lo, acc);
   }

@@ -86,7 +86,7 @@ TilePlan build_tile_plan(const TableSet &t, int fwarps, int awarps);
 // every tile of a degree has the same record sides), or, for the odd tile of
 // a degree, the even and the odd records of each side, whose sums the halves
 // exchange at the end.  A missing odd record is its neighbour with a factor
-// tile of zeros (TILE_NULL).
+// tile, and a Tb tile, of zeros (TILE_NULL).
 constexpr uint32_t TILE_NULL = 1u << 13;
 struct TileAdj64 {
   bool ok = false;
