@@ -331,6 +331,39 @@ __device__ __forceinline__ void l2_reduce(const L2aArgs &a, double *red, const d
   }
 }
 
+// One point's dW_2 sums over the slots a0 .. a1 - 1, one product at a time and
+// none for a slot without a_i, added to r.
+template <typename R, typename MT, int D0>
+__device__ __forceinline__ void l2a_plain(const L2aArgs &a, const MT *fact, const MT *Ml,
+                                          const int *off, int j, long pt, int a0, int a1,
+                                          double (&r)[D0 + 1]) {
+  const R *Tb = (const R *)a.Tb + (size_t)pt * a.na * a.n + j;
+  const R *sg = (const R *)a.sig + (size_t)pt * (a.k + 2) * a.n + j;
+  double v = 0.0;
+#pragma unroll 1
+  for (int p = 0; p <= a.k; ++p)
+#pragma unroll 1
+    for (int q = max(a.ds[p], a0); q < min(a.ds[p + 1], a1); ++q) {
+      const double x = (double)Tb[(size_t)q * a.n] * (double)fact[q];
+      v += (double)sg[(size_t)(p + 1) * a.n] * (x * (double)Ml[q * a.nt]);
+#pragma unroll
+      for (int i = 0; i < D0; ++i) {
+        const int o = off[q * D0 + i];
+        if (o != a.na * a.nt) r[1 + i] += (double)sg[(size_t)p * a.n] * (x * (double)Ml[o]);
+      }
+    }
+  r[0] += v;
+#pragma unroll
+  for (int i = 0; i < D0; ++i) r[1 + i] = fma(v, __ldg(a.X + (size_t)pt * D0 + i), r[1 + i]);
+}
+template <int N>
+__device__ __forceinline__ bool any_odd(const double (&v)[N]) {  // not finite
+  bool odd = false;
+#pragma unroll
+  for (int o = 0; o < N; ++o) odd |= !(fabs(v[o]) <= 1.7976931348623157e308);
+  return odd;
+}
+
 // Sb^0 = sum_a Tb^a h^a and Sb^{e_i} = sum_a a_i Tb^a h^{a - e_i} with
 // h^g = s^(|g|+1) W^g.  With M_a = W^a / a! and x_a = a! Tb^a both read
 // x_a M_a and x_a M_{a - e_i}, and s depends on the degree alone, so each
@@ -341,8 +374,8 @@ __device__ __forceinline__ void l2_reduce(const L2aArgs &a, double *red, const d
 // further points) and PT points at a time per thread: the tile's M rows sit
 // in shared memory and one read of a row serves PT points, and the slots go
 // in groups of G whose values are loaded a group ahead, so the kernel streams
-// Tb (32768 points x 128 at K = 7, D0 = 4 in FP32: 5.5 GB in 1.30 ms, 4.2
-// TB/s; in FP64, 16384 points, 5.5 GB in 1.03).
+// Tb (32768 points x 128 at K = 7, D0 = 4 in FP32: 5.5 GB in 1.35 ms, 4.1
+// TB/s; in FP64, 16384 points, 5.5 GB in 1.16).
 // Precision: the degrees, the points and the blocks are added in FP64.  On
 // the split path a degree is summed in FP32 runs of at most a.chain groups
 // (BT = float), or in FP64 throughout (BT = MT = double) where a run would be
@@ -353,6 +386,11 @@ __device__ __forceinline__ void l2_reduce(const L2aArgs &a, double *red, const d
 // points; row mode writes each point's sums, a warp's own (L2_ROWS) or, when
 // there are few points, those of a block's eight warps, which share the
 // slots of the same points (L2_ROWS8).
+// A slot without a_i multiplies a row of zeros for e_i.  Where a value of Tb is
+// not finite, neither are the sums, and the thread forms them again without
+// those products, which are NaN (l2a_plain; behind the loop and from a fresh
+// thread index, so that the loop keeps its registers: in the loop it cost a
+// third of its speed).
 enum L2Mode { L2_GRAD, L2_ROWS, L2_ROWS8 };
 template <typename R, typename BT, typename MT, int D0, int PT, L2Mode MODE>
 __global__ void __launch_bounds__(L2T, 2) k_adj_l2a(L2aArgs a) {
@@ -405,6 +443,7 @@ __global__ void __launch_bounds__(L2T, 2) k_adj_l2a(L2aArgs a) {
   const long nwarp = MODE == L2_ROWS8 ? (long)gridDim.x : (long)gridDim.x * NWP;
   const long w0 = MODE == L2_ROWS8 ? (long)blockIdx.x : (long)blockIdx.x * NWP + warp;
   const int step = a.ppw;
+  bool odd = false;  // a row that is not finite
   for (long w = w0; w * step * PT < a.npts; w += nwarp) {
     if (MODE != L2_ROWS8 && !act) continue;  // with shared slots every thread meets the barriers
     const R *Tb[PT], *sg[PT];
@@ -497,6 +536,7 @@ __global__ void __launch_bounds__(L2T, 2) k_adj_l2a(L2aArgs a) {
       s[0] += v0[k];
 #pragma unroll
       for (int i = 0; i < D0; ++i) s[1 + i] = fma(v0[k], __ldg(x + i), s[1 + i]);
+      if (MODE != L2_GRAD) odd |= any_odd(s);
       if (MODE == L2_ROWS) {
         double *row = a.rows + (size_t)pt * a.nw + a.woff + (size_t)j * (D0 + 1);
 #pragma unroll
@@ -523,6 +563,44 @@ __global__ void __launch_bounds__(L2T, 2) k_adj_l2a(L2aArgs a) {
         a.rows[(size_t)pt * a.nw + a.woff + (size_t)j * (D0 + 1) + o] = v;
       }
     }
+  }
+  if (MODE == L2_GRAD) odd = any_odd(acc[0]);
+  if (MODE == L2_ROWS8) odd = __syncthreads_or(odd);
+  if (odd) {
+    int tid;
+    asm volatile("mov.u32 %0, %%tid.x;" : "=r"(tid));
+    const int ln = tid & 31, wp = tid >> 5, jl2 = ln % a.nt, sub2 = ln / a.nt;
+    const int j2 = blockIdx.y * a.nt + jl2;
+    double r[D0 + 1];
+#pragma unroll
+    for (int o = 0; o <= D0; ++o) r[o] = 0.0;
+    const bool mine = sub2 < a.ppw && j2 < a.n && (MODE != L2_ROWS8 || wp == 0);
+    const long first = MODE == L2_ROWS8 ? (long)blockIdx.x : (long)blockIdx.x * NWP + wp;
+    const long nw = MODE == L2_ROWS8 ? (long)gridDim.x : (long)gridDim.x * NWP;
+    const int b0 = MODE == L2_GRAD ? (int)((long)a.na * blockIdx.z / a.zsplit) : 0;
+    const int b1 = MODE == L2_GRAD ? (int)((long)a.na * (blockIdx.z + 1) / a.zsplit) : a.na;
+#pragma unroll 1
+    for (long w = first; mine && w * a.ppw * PT < a.npts; w += nw)
+#pragma unroll 1
+      for (int k = 0; k < PT; ++k) {
+        const long pt = (w * PT + k) * a.ppw + sub2;
+        if (pt >= a.npts) break;
+        l2a_plain<R, MT, D0>(a, fact, M + jl2, off, j2, pt, b0, b1, r);
+        if (MODE == L2_GRAD) continue;
+        double *row = a.rows + (size_t)pt * a.nw + a.woff + (size_t)j2 * (D0 + 1);
+        double old[D0 + 1];
+#pragma unroll
+        for (int o = 0; o <= D0; ++o) old[o] = row[o];
+        const bool again = any_odd(old);
+#pragma unroll
+        for (int o = 0; o <= D0; ++o) {
+          if (again) row[o] = r[o];
+          r[o] = 0.0;
+        }
+      }
+    if (MODE == L2_GRAD)
+#pragma unroll
+      for (int o = 0; o <= D0; ++o) acc[0][o] = r[o];
   }
   if (MODE == L2_GRAD && a.g) l2_reduce<D0, L2T>(a, (double *)sm2, acc[0], act, j0);
 }
@@ -766,19 +844,19 @@ int l2a_k(L2aArgs a, cudaStream_t st) {
     return RC_OK;
   }
   // Runs of FP32 sums: |A| / 32 slots in whole groups of four; below that a
-  // gradient's sums are FP64 (65536 points x 128, 35 slots: 0.46 ms, 0.41 in
+  // gradient's sums are FP64 (65536 points x 128, 35 slots: 0.48 ms, 0.41 in
   // FP32).  k_adj_l2s added the parts of a row in FP32 too, so a row keeps its
   // runs of one group.
   const int run = (a.na + 31) / 32 / 4;
   if constexpr (sizeof(R) == 4) {
     a.chain = std::max(1, run);
     if (a.rows) return l2a_rows<R, float, D0>(a, st);
-    if (run >= 1) return l2a_launch<R, float, float, D0, D0 <= 5 ? 4 : 3, L2_GRAD>(a, st);
+    if (run >= 1) return l2a_launch<R, float, float, D0, D0 <= 4 ? 4 : 3, L2_GRAD>(a, st);
   }
   a.chain = a.na;
   if constexpr (sizeof(R) == 8)
     if (a.rows) return l2a_rows<R, double, D0>(a, st);
-  return l2a_launch<R, double, double, D0, 3, L2_GRAD>(a, st);
+  return l2a_launch<R, double, double, D0, sizeof(R) == 8 && D0 >= 4 ? 2 : 3, L2_GRAD>(a, st);
 }
 
 template <typename R>
