@@ -156,8 +156,18 @@ cudaError_t DevScratch::take(size_t bytes, cudaStream_t st) {
   return e;
 }
 void DevScratch::release() {
-  if (p_) cudaFreeAsync(p_, st_);
+  if (!p_) return;
+  cudaFreeAsync(p_, st_);
   p_ = nullptr;
+  // beyond what the pool may keep: the memory is the caller's again when the
+  // call returns, as after cudaFree
+  cudaMemPool_t pool = scratch_pool(false);
+  unsigned long long held = 0;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if (pool && cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held) == cudaSuccess &&
+      held > POOL_KEEP && cudaStreamIsCapturing(st_, &cs) == cudaSuccess &&
+      cs == cudaStreamCaptureStatusNone && cudaStreamSynchronize(st_) == cudaSuccess)
+    cudaMemPoolTrimTo(pool, POOL_KEEP);
 }
 void scratch_trim() {
   cudaMemPool_t pool = scratch_pool(false);

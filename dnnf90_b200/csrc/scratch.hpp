@@ -3,9 +3,9 @@
 // A call that needs device memory only while it runs takes it from one pool
 // per device, private to the library (cudaMallocAsync), instead of
 // cudaMalloc / cudaFree, which wait for the whole device and map fresh pages
-// on every call (0.75 ms for a 7 MB operand).  The pool is bounded: at each
-// synchronisation CUDA returns what it holds beyond POOL_KEEP bytes, and
-// scratch_trim (called when a network is freed) returns the rest.  The
+// on every call (0.75 ms for a 7 MB operand).  The pool is bounded: a call ends
+// with what it holds beyond POOL_KEEP bytes given back, and scratch_trim
+// (called when a network is freed) returns the rest.  The
 // allocations are ordered on the caller's stream, so calls of several
 // threads and streams share the pool safely.
 #pragma once
