@@ -254,9 +254,8 @@ struct KfDev {
   KfState *st = nullptr;
   KfBar *bar = nullptr;
   int seq_grid = 0;          // CTAs of the one-launch sequence (0: no cooperative launch)
-  // grouped updates (null gbuf: none yet; gfull: no memory for them)
+  // grouped updates (null gbuf: the filter is small): one allocation
   void *gbuf = nullptr;
-  bool gfull = false;
   int nitem = 0;
   int4 *gitems = nullptr, *grt = nullptr;
   double *gU = nullptr, *gY = nullptr, *gJ[2] = {nullptr, nullptr};

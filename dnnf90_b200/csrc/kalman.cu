@@ -43,7 +43,6 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
-#include <cstring>
 #include <string>
 #include <vector>
 
@@ -1074,14 +1073,8 @@ constexpr int KF_GROUP_TILES = 512, KF_GROUP_OBS = 3;
 constexpr size_t GT_SMEM =
     (size_t)(2 * GW * KTE + 2 * 2 * KT * GVS + GW * KT * GM) * sizeof(double);
 
-// Buffers and work items of the grouped updates, one allocation, made by the
-// first call that groups (a filter that is only handed single observations
-// has none) and in place before what s runs next, also when s is capturing:
-// the allocation and the tables are not part of the graph.  Without the memory
-// the updates stay single.
-static bool group_ready(KfDev &d, cudaStream_t s) {
-  if (d.gbuf) return true;
-  if (!d.dense || d.ntile < KF_GROUP_TILES || d.gfull) return false;
+// buffers and work items of the grouped updates: one allocation
+static int group_create(KfDev &d) {
   std::vector<int4> items, grt;
   const int tb = (d.nw + KT - 1) / KT;
   long steps = 0;
@@ -1115,37 +1108,14 @@ static bool group_ready(KfDev &d, cudaStream_t s) {
   const size_t oU = take(vb), oY = take(vb), oJ0 = take(vb), oJ1 = take(vb);
   const size_t orp = take((size_t)rp * KT * GM * 8), ocp = take((size_t)cp * KT * GM * 8);
   const size_t od = take((size_t)d.nred * 2 * GM * GM * 16), ogr = take(sizeof(KfGroup));
-  std::vector<unsigned char> tab(og + grt.size() * sizeof(int4));
-  std::memcpy(tab.data() + oi, items.data(), items.size() * sizeof(int4));
-  std::memcpy(tab.data() + og, grt.data(), grt.size() * sizeof(int4));
-  void *buf = nullptr;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  cudaError_t e = cudaStreamIsCapturing(s, &cs);
-  if (e == cudaSuccess && cs == cudaStreamCaptureStatusNone) {
-    e = cudaMalloc(&buf, cur);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(buf, tab.data(), tab.size(), cudaMemcpyHostToDevice, s);
-  } else if (e == cudaSuccess) {
-    cudaStream_t own = nullptr;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    e = cudaThreadExchangeStreamCaptureMode(&mode);
-    if (e == cudaSuccess) {
-      e = cudaMalloc(&buf, cur);
-      if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(buf, tab.data(), tab.size(), cudaMemcpyHostToDevice, own);
-      if (e == cudaSuccess) e = cudaStreamSynchronize(own);
-      if (own) cudaStreamDestroy(own);
-      cudaThreadExchangeStreamCaptureMode(&mode);
-    }
+  if (cudaMalloc(&d.gbuf, cur) != cudaSuccess) {
+    cudaGetLastError();  // the two-launch path needs none of it
+    d.gbuf = nullptr;
+    return RC_OK;
   }
-  if (e != cudaSuccess && buf) cudaFree(buf);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    d.gfull = true;
-    return false;
-  }
-  d.gbuf = buf;
-  char *p = (char *)buf;
+  char *p = (char *)d.gbuf;
+  CKK(cudaMemcpy(p + oi, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
+  CKK(cudaMemcpy(p + og, grt.data(), grt.size() * sizeof(int4), cudaMemcpyHostToDevice));
   d.nitem = (int)items.size() / 2;
   d.gitems = (int4 *)(p + oi);
   d.grt = (int4 *)(p + og);
@@ -1157,7 +1127,7 @@ static bool group_ready(KfDev &d, cudaStream_t s) {
   d.gcpart = (double *)(p + ocp);
   d.gdots = (double2 *)(p + od);
   d.grp = p + ogr;
-  return true;
+  return RC_OK;
 }
 
 template <int MODE>
@@ -1245,6 +1215,10 @@ int kf_create(KfDev &d, const std::vector<int> &bsz, const std::vector<int> &bof
     d.seq_grid = coop && per_sm > 0 ? std::min(grid_sms() * per_sm, std::max(d.ntile, d.nred))
                                     : 0;
   }
+  if (d.dense && d.ntile >= KF_GROUP_TILES) {
+    const int rc = group_create(d);
+    if (rc) return rc;
+  }
   CKK(cudaMemcpy(d.tiles, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice));
   CKK(cudaMemcpy(d.rtl, rtl.data(), rtl.size() * sizeof(int4), cudaMemcpyHostToDevice));
   CKK(cudaMemset(d.ctr, 0, sizeof(unsigned)));
@@ -1268,7 +1242,7 @@ int kf_run(KfDev &d, int nobs, const double *rows, size_t ld, const double *xi,
   int path = g_kf_path.load();
   // a call of several observations on a larger filter: every call of a
   // sequence comes here, so each forms its own first products
-  if (path < 0 && nobs >= KF_GROUP_OBS && group_ready(d, s)) {
+  if (path < 0 && d.gbuf && nobs >= KF_GROUP_OBS) {
     if (kbase == 0) CKK(cudaMemsetAsync(&d.st->status, 0, sizeof(int), s));
     return run_groups(d, nobs, ra, w, s, kbase);
   }

@@ -83,59 +83,3 @@ def test_rows_whose_square_overflows(path):
     path(-1)
     wg, Pg = _run(*args)
     assert np.all(np.isfinite(wg)) and rel_err(wg, w1) < 1e-11 and rel_err(Pg, P1) < 1e-11
-
-
-def test_a_filter_of_single_observations_has_no_group_buffers():
-    """The groups' buffers (some 60 MB at 17025 weights) come with the first
-    call that groups, which may be one in a capture."""
-    import torch
-    dims = [2, 128, 128, 1]
-    ts = api.TableSet(2, 1)
-    nw = 128 * 3 + 128 * 129 + 129
-    rng = np.random.default_rng(0)
-    net = api.Net(ts, dims, weights=rng.normal(size=nw) * 0.1)
-    rows = torch.tensor(rng.normal(size=(9, nw)) * 0.05, device="cuda")
-    xi = torch.tensor(rng.normal(size=9), device="cuda")
-    w0 = torch.tensor(rng.normal(size=nw), device="cuda")
-    api.Kalman(net, 0.5, 0.98, 0.99).free()          # whatever a first filter loads
-
-    def used():
-        torch.cuda.synchronize()
-        free, total = torch.cuda.mem_get_info()
-        return total - free
-
-    def update(kf, nobs, w):
-        api.call("dnnf90_kf_update_rows_dev", kf.kid, nobs, rows.data_ptr(), xi.data_ptr(), None,
-                 w.data_ptr(), torch.cuda.current_stream().cuda_stream)
-
-    tb = (nw + 31) // 32
-    cov = tb * (tb + 1) // 2 * 32 * 32 * 8 + tb * tb * 32 * 8  # the tiles and their partial sums
-    base = used()
-    kf = api.Kalman(net, 0.5, 0.98, 0.99)
-    w = w0.clone()
-    update(kf, 1, w)
-    update(kf, 2, w)
-    assert used() - base <= cov + (24 << 20)
-    before = used()
-    update(kf, 3, w)
-    assert used() - before >= 30 << 20
-    kf.free()
-    # a capture before the first grouped call, and the same calls outside one
-    out = []
-    for captured in (True, False):
-        kf = api.Kalman(net, 0.5, 0.98, 0.99)
-        w = w0.clone()
-        if captured:
-            torch.cuda.synchronize()
-            graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(graph):
-                update(kf, 9, w)
-            graph.replay()
-            torch.cuda.synchronize()
-        else:
-            update(kf, 9, w)
-        update(kf, 9, w)
-        out.append(w.cpu().numpy())
-        kf.free()
-    assert np.array_equal(out[0], out[1])
-    net.free(); ts.free()
