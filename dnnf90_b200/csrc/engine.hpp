@@ -241,6 +241,7 @@ struct KfBar {
 
 // covariance in packed 32 x 32 tiles of each block's upper triangle
 struct KfDev {
+  void *base = nullptr;      // one allocation
   int nw = 0, ntile = 0, nred = 0;
   bool dense = false;        // a single block (the global filter)
   double *P = nullptr;       // [ntile][32][32]
@@ -254,8 +255,7 @@ struct KfDev {
   KfState *st = nullptr;
   KfBar *bar = nullptr;
   int seq_grid = 0;          // CTAs of the one-launch sequence (0: no cooperative launch)
-  // grouped updates (null gbuf: the filter is small): one allocation
-  void *gbuf = nullptr;
+  bool grouped = false;      // grouped updates: the buffers below
   int nitem = 0;
   int4 *gitems = nullptr, *grt = nullptr;
   double *gU = nullptr, *gY = nullptr, *gJ[2] = {nullptr, nullptr};

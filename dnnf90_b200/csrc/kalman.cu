@@ -43,10 +43,12 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <cstring>
 #include <string>
 #include <vector>
 
 #include "engine.hpp"
+#include "scratch.hpp"
 
 namespace dnnf90 {
 
@@ -1045,20 +1047,20 @@ __global__ void k_kf_init_tiles(const int4 *__restrict__ tiles, double *__restri
 }
 
 void KfDev::release() {
-  cudaFree(P);
-  cudaFree(tiles);
-  cudaFree(rtl);
-  cudaFree(part);
-  cudaFree(pj);
-  cudaFree(dotp);
-  cudaFree(ctr);
-  cudaFree(st);
-  cudaFree(bar);
+  cudaFree(base);
   cudaFree(stage);
-  cudaFree(wprior);
-  cudaFree(gbuf);
   *this = KfDev();
 }
+
+// Places of a filter's arrays in its one allocation
+struct KfLayout {
+  size_t cur = 0;
+  size_t take(size_t bytes) {
+    const size_t at = cur;
+    cur = (cur + bytes + 255) / 256 * 256;
+    return at;
+  }
+};
 
 // Dense filters of at least this many tiles group the observations of a call
 // (of at least KF_GROUP_OBS); smaller ones keep the one-launch sequence, whose
@@ -1073,17 +1075,15 @@ constexpr int KF_GROUP_TILES = 512, KF_GROUP_OBS = 3;
 constexpr size_t GT_SMEM =
     (size_t)(2 * GW * KTE + 2 * 2 * KT * GVS + GW * KT * GM) * sizeof(double);
 
-// buffers and work items of the grouped updates: one allocation
-static int group_create(KfDev &d) {
-  std::vector<int4> items, grt;
-  const int tb = (d.nw + KT - 1) / KT;
+// Work items of the grouped updates, the partial tiles they write (rows, columns)
+static void group_items(int tb, std::vector<int4> &items, std::vector<int4> &grt, int &rp, int &cp) {
   long steps = 0;
   for (int I0 = 0; I0 < tb; I0 += GW) steps += tb - I0;
   // column tiles per item: about 12, so that its start-up is small beside
   // it, and a whole number of waves of one CTA per SM
   const long waves = std::max(1L, (steps + 6L * grid_sms()) / (12L * grid_sms()));
   const int seg = (int)std::max(2L, (steps + waves * grid_sms() - 1) / (waves * grid_sms()));
-  int cp = 0, rp = 0;
+  cp = rp = 0;
   for (int I0 = 0; I0 < tb; I0 += GW) {
     const int rblock = rp, ns = (tb - I0 + seg - 1) / seg;
     for (int s = 0; s < ns; ++s) {
@@ -1093,41 +1093,8 @@ static int group_create(KfDev &d) {
       rp += GW;
       cp += nJ;
     }
-    for (int K = I0; K < std::min(tb, I0 + GW); ++K) {
-      grt.push_back(make_int4(rblock + K - I0, ns, 0, 0));
-    }
+    for (int K = I0; K < std::min(tb, I0 + GW); ++K) grt.push_back(make_int4(rblock + K - I0, ns, 0, 0));
   }
-  size_t cur = 0;
-  auto take = [&](size_t bytes) {
-    const size_t at = cur;
-    cur = (cur + bytes + 255) / 256 * 256;
-    return at;
-  };
-  const size_t vb = (size_t)d.nw * GM * sizeof(double);
-  const size_t oi = take(items.size() * sizeof(int4)), og = take(grt.size() * sizeof(int4));
-  const size_t oU = take(vb), oY = take(vb), oJ0 = take(vb), oJ1 = take(vb);
-  const size_t orp = take((size_t)rp * KT * GM * 8), ocp = take((size_t)cp * KT * GM * 8);
-  const size_t od = take((size_t)d.nred * 2 * GM * GM * 16), ogr = take(sizeof(KfGroup));
-  if (cudaMalloc(&d.gbuf, cur) != cudaSuccess) {
-    cudaGetLastError();  // the two-launch path needs none of it
-    d.gbuf = nullptr;
-    return RC_OK;
-  }
-  char *p = (char *)d.gbuf;
-  CKK(cudaMemcpy(p + oi, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  CKK(cudaMemcpy(p + og, grt.data(), grt.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  d.nitem = (int)items.size() / 2;
-  d.gitems = (int4 *)(p + oi);
-  d.grt = (int4 *)(p + og);
-  d.gU = (double *)(p + oU);
-  d.gY = (double *)(p + oY);
-  d.gJ[0] = (double *)(p + oJ0);
-  d.gJ[1] = (double *)(p + oJ1);
-  d.grpart = (double *)(p + orp);
-  d.gcpart = (double *)(p + ocp);
-  d.gdots = (double2 *)(p + od);
-  d.grp = p + ogr;
-  return RC_OK;
 }
 
 template <int MODE>
@@ -1195,39 +1162,76 @@ int kf_create(KfDev &d, const std::vector<int> &bsz, const std::vector<int> &bof
   d.dense = bsz.size() == 1;
   d.ntile = (int)tl.size();
   d.nred = (int)rtl.size();
-  CKK(cudaMalloc(&d.P, (size_t)d.ntile * KTE * sizeof(double)));
-  CKK(cudaMalloc(&d.tiles, tl.size() * sizeof(int4)));
-  CKK(cudaMalloc(&d.rtl, rtl.size() * sizeof(int4)));
-  CKK(cudaMalloc(&d.part, pslots * sizeof(double)));
-  CKK(cudaMalloc(&d.pj, nw * sizeof(double)));
-  CKK(cudaMalloc(&d.dotp, 2 * d.nred * sizeof(double)));
-  CKK(cudaMalloc(&d.wprior, nw * sizeof(double)));
-  CKK(cudaMalloc(&d.ctr, sizeof(unsigned)));
-  CKK(cudaMalloc(&d.st, sizeof(KfState)));
-  CKK(cudaMalloc(&d.bar, sizeof(KfBar)));
-  CKK(cudaMemset(d.bar, 0, sizeof(KfBar)));
+  // one allocation: the tables first, in the order of the host block that fills
+  // them with one copy, the covariance last but for the groups' buffers, which
+  // a filter does without where there is no memory for them
+  const bool grouped = d.dense && d.ntile >= KF_GROUP_TILES;
+  std::vector<int4> items, grt;
+  int rp = 0, cp = 0;
+  if (grouped) group_items((nw + KT - 1) / KT, items, grt, rp, cp);
+  KfLayout L;
+  const size_t ost = L.take(sizeof(KfState)), obar = L.take(sizeof(KfBar)),
+               octr = L.take(sizeof(unsigned)), otl = L.take(tl.size() * sizeof(int4)),
+               ort = L.take(rtl.size() * sizeof(int4)), oit = L.take(items.size() * sizeof(int4)),
+               ogt = L.take(grt.size() * sizeof(int4)), head = L.cur;
+  const size_t opart = L.take(pslots * sizeof(double)), opj = L.take(nw * sizeof(double)),
+               odp = L.take(2 * d.nred * sizeof(double)), owp = L.take(nw * sizeof(double)),
+               oP = L.take((size_t)d.ntile * KTE * sizeof(double)), single = L.cur;
+  const size_t vb = (size_t)nw * GM * sizeof(double);
+  const size_t oU = L.take(vb), oY = L.take(vb), oJ0 = L.take(vb), oJ1 = L.take(vb),
+               orp = L.take((size_t)rp * KT * GM * 8), ocp = L.take((size_t)cp * KT * GM * 8),
+               ods = L.take((size_t)d.nred * 2 * GM * GM * 16), ogr = L.take(sizeof(KfGroup));
+  bool room = false;
+  if (grouped) {
+    room = cudaMalloc(&d.base, L.cur) == cudaSuccess;
+    if (!room) cudaGetLastError();
+  }
+  if (!room) CKK(cudaMalloc(&d.base, single));
+  char *p = (char *)d.base;
+  d.st = (KfState *)(p + ost);
+  d.bar = (KfBar *)(p + obar);
+  d.ctr = (unsigned *)(p + octr);
+  d.tiles = (int4 *)(p + otl);
+  d.rtl = (int4 *)(p + ort);
+  d.part = (double *)(p + opart);
+  d.pj = (double *)(p + opj);
+  d.dotp = (double *)(p + odp);
+  d.wprior = (double *)(p + owp);
+  d.P = (double *)(p + oP);
+  if (room) {
+    d.grouped = true;
+    d.nitem = (int)items.size() / 2;
+    d.gitems = (int4 *)(p + oit);
+    d.grt = (int4 *)(p + ogt);
+    d.gU = (double *)(p + oU);
+    d.gY = (double *)(p + oY);
+    d.gJ[0] = (double *)(p + oJ0);
+    d.gJ[1] = (double *)(p + oJ1);
+    d.grpart = (double *)(p + orp);
+    d.gcpart = (double *)(p + ocp);
+    d.gdots = (double2 *)(p + ods);
+    d.grp = p + ogr;
+  }
   {
-    int coop = 0, dev = 0, per_sm = 0;
+    int coop = 0, dev = 0;
     CKK(cudaGetDevice(&dev));
     CKK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
-    CKK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &per_sm, d.dense ? k_kf_seq<true> : k_kf_seq<false>, 256, 0));
-    d.seq_grid = coop && per_sm > 0 ? std::min(grid_sms() * per_sm, std::max(d.ntile, d.nred))
-                                    : 0;
+    const int per_sm = blocks_per_sm(d.dense ? (const void *)k_kf_seq<true>
+                                             : (const void *)k_kf_seq<false>, 256, 0);
+    d.seq_grid = coop ? std::min(grid_sms() * per_sm, std::max(d.ntile, d.nred)) : 0;
   }
-  if (d.dense && d.ntile >= KF_GROUP_TILES) {
-    const int rc = group_create(d);
-    if (rc) return rc;
-  }
-  CKK(cudaMemcpy(d.tiles, tl.data(), tl.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  CKK(cudaMemcpy(d.rtl, rtl.data(), rtl.size() * sizeof(int4), cudaMemcpyHostToDevice));
-  CKK(cudaMemset(d.ctr, 0, sizeof(unsigned)));
+  std::vector<unsigned char> tab(head, 0);  // the barrier and the counter at zero
   KfState s{};
   s.lam = lam_ini;
   s.lam0 = lam0;
   s.q = q;
   s.gate = gate;
-  CKK(cudaMemcpy(d.st, &s, sizeof(s), cudaMemcpyHostToDevice));
+  std::memcpy(tab.data() + ost, &s, sizeof s);
+  std::memcpy(tab.data() + otl, tl.data(), tl.size() * sizeof(int4));
+  std::memcpy(tab.data() + ort, rtl.data(), rtl.size() * sizeof(int4));
+  if (!items.empty()) std::memcpy(tab.data() + oit, items.data(), items.size() * sizeof(int4));
+  if (!grt.empty()) std::memcpy(tab.data() + ogt, grt.data(), grt.size() * sizeof(int4));
+  CKK(cudaMemcpy(d.base, tab.data(), head, cudaMemcpyHostToDevice));
   LAUNCH("k_kf_init_tiles", 0, k_kf_init_tiles<<<d.ntile, 256>>>(d.tiles, d.P, p0));
   CKK(cudaGetLastError());
   CKK(cudaDeviceSynchronize());
@@ -1242,13 +1246,13 @@ int kf_run(KfDev &d, int nobs, const double *rows, size_t ld, const double *xi,
   int path = g_kf_path.load();
   // a call of several observations on a larger filter: every call of a
   // sequence comes here, so each forms its own first products
-  if (path < 0 && d.gbuf && nobs >= KF_GROUP_OBS) {
+  if (path < 0 && d.grouped && nobs >= KF_GROUP_OBS) {
     if (kbase == 0) CKK(cudaMemsetAsync(&d.st->status, 0, sizeof(int), s));
     return run_groups(d, nobs, ra, w, s, kbase);
   }
   // one or two observations of a grouping filter: the call before, grouped,
   // formed no products for this one
-  if (path < 0 && d.gbuf) {
+  if (path < 0 && d.grouped) {
     first = true;
     has_next = false;
   }

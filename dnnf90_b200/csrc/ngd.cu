@@ -7,9 +7,9 @@
 // once damped, so the factorization is the natural device form).
 //
 // The metric build is a GEMM: in the split path J is carried as three bf16
-// terms and the six cross products are accumulated in FP32 per 64-row slab
-// (tensor cores), the slabs summed in FP64; in the plain path it is an FP64
-// CUDA-core GEMM.
+// terms and the six cross products are accumulated in FP32 over runs of at most
+// 512 rows on the tensor cores, the runs summed in FP64; in the plain path it
+// runs on the FP64 tensor cores.
 #include <cuda_runtime.h>
 
 #include <algorithm>
