@@ -70,6 +70,34 @@ def test_kept_planes_save_the_forward(kept):
     assert n_kept == n_again < n_recomputed
 
 
+@pytest.mark.parametrize("between", ["batch", "queue", "rows"])
+def test_host_calls_between(kept, between):
+    """The host entries that write the same work space's planes, through the
+    layered kernels (a pinned variant: the one-launch step touches no plane),
+    the batch and the rows at the kept points themselves."""
+    X = kept.x.cpu().numpy()
+    g = kept.net.grad()
+    j = api.SeedRule(api.SEED_JROW, [(1.0, 1, False)])
+    api.tune_force(0, 2)
+    try:
+        kept.forward()
+        n_kept = kept.backward()[1]
+        if between == "batch":
+            g.rule_batch(X, kept.rule)
+        elif between == "queue":
+            for p in range(3):
+                g.point(kept.y[p].cpu().numpy(), np.ones(kept.net.na))
+            g.read()
+        else:
+            api.jacobian_rows(kept.net, X[:40], j)
+        got, n = kept.backward()
+    finally:
+        api.tune_force(0, -1)
+    kept.check(got)
+    assert n > n_kept            # recomputed
+    j.free(); g.free()
+
+
 def test_committee_replay_between(kept):
     import torch
     loss = torch.zeros(1, dtype=torch.float64, device="cuda")
