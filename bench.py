@@ -299,8 +299,8 @@ def committee_members(nnet=64):
 
 
 def autotuner_summary(api, pinned=None):
-    """The Bell kernels' autotuner choices, keyed on (kernel, D0, K, |A|,
-    width, precision): the ZK7 shapes by name, the others (the committee's
+    """The Bell kernels' autotuner choices, keyed on (table set, kernel, D0, K,
+    |A|, width, precision): the ZK7 shapes by name, the others (the committee's
     members) as counts per (kernel, precision, variant).  Launches under
     --pin-variants are not tuned (pinned names the pin)."""
     zk7, other = [], collections.Counter()
@@ -312,7 +312,7 @@ def autotuner_summary(api, pinned=None):
             zk7.append(f"{kern} {prec}: {name}")
         else:
             other[f"{kern} {prec} {name}"] += 1
-    out = {"key": "(kernel, D0, K, |A|, width, precision)", "shapes": len(rows),
+    out = {"key": "(table set, kernel, D0, K, |A|, width, precision)", "shapes": len(rows),
            "zk7": sorted(set(zk7)), "others": dict(sorted(other.items()))}
     if pinned:
         out["pinned"] = pinned
